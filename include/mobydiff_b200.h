@@ -91,14 +91,17 @@ typedef struct {
     int max_iter;      /* red-black: iteration cap when tol > 0               */
     int check_every;   /* red-black: iterations between residual checks       */
     int precision;     /* MDX_PREC_*                                          */
-    int sor_variant;   /* red-black kernels (bit-identical results): 0 auto -- the
-                          first projection times each variant on one residual-check
+    int sor_variant;   /* red-black kernels (bit-identical results): 0 auto -- where the
+                          whole state fits the SMs (about 1 M cells in FP64, 4 M in
+                          FP32), one launch per run of sweeps with the state on chip;
+                          else the first projection times each variant on one residual-check
                           block of its own iterations and keeps the fastest; 1 one
                           launch per colour; 2 fused red+black pass, 32x8 tiles;
                           3 fused pass, 32x16 tiles; 4 one launch per colour on
                           colour-split copies of u, v, w, p made once per projection;
                           5 the same with two cells per thread and 16-byte accesses
-                          (2-5: periodic x and z, IBM factors 1 or z-invariant).
+                          (2-5: periodic x and z, IBM factors 1 or z-invariant);
+                          6 the on-chip run, or auto where it does not fit.
                           FP32 sweeps of the mixed precision: 1 one launch per colour,
                           one cell per thread; 2 or 3 the fused red+black pass (one
                           launch per iteration) in the fastest of four tile shapes; 4 or
@@ -107,7 +110,7 @@ typedef struct {
                           first iterations (all give the same bits).  In the potential
                           form (inner_form 0 or 2): 1-15 pin one shape of its sweep
                           kernels, 0 the fastest of those the grid allows (all give the
-                          same bits) */
+                          same bits), 16 the on-chip run */
     int sor_kz;        /* z planes per block of the fused pass (0: default 16) */
     int check_mode;    /* red-black, tol > 0: 0 (default) residual checks at multiples of check_every,
                           up to 8 blocks apart while the residual falls at a steady rate that

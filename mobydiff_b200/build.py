@@ -31,6 +31,7 @@ CUDA_SOURCES = {
     "k_fft.cu": ["-fmad=false"],
     "k_sor.cu": ["-fmad=false"],
     "k_sor_mixed.cu": [],   # FP32 sweeps inside FP64 defect correction: FMA allowed
+    "k_sor_resident.cu": ["-fmad=false"],
     "k_warm.cu": ["-fmad=false"],
     "k_unet.cu": [],        # BF16 network with FP32 accumulation: FMA allowed
     "k_ensemble.cu": ["-fmad=false"],

@@ -3,6 +3,7 @@
 // reference-facing time-step calls, the CUDA-graph replay of whole RK3
 // steps, and per-kernel-class event timing.
 #include "mdx_internal.cuh"
+#include "mdx_resident.cuh"
 
 #include <cmath>
 #include <cstring>
@@ -251,6 +252,7 @@ int mdx_destroy_pressure_solver(mdx_ctx_t* ctx) {
     ctx->split_tab = nullptr;
     ctx->split_norms = false;
     mdx_mixed_free(ctx);
+    mdx_res_free(ctx);
     mdx_warm_free(ctx);
     ctx->solver = false;
     return MDX_OK;
@@ -384,7 +386,7 @@ int mdx_update_host(mdx_ctx_t* ctx, double* un, double* vn, double* wn, double* 
             MDX_CUDA(ctx, cudaMemcpyAsync(dst[t], ctx->f[ids[t]], sizeof(double) * ctx->d.npad, cudaMemcpyDeviceToHost,
                                           ctx->stream));
     MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return MDX_OK;
+    return mdx_res_check(ctx);
 }
 
 int mdx_update_device(mdx_ctx_t* ctx, const double* un, const double* vn, const double* wn, const double* pn) {

@@ -17,6 +17,7 @@
 // opposite directions, so each starts on the planes the previous one left
 // in the 126 MB L2.
 #include "mdx_cell.cuh"
+#include "mdx_resident.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -764,6 +765,12 @@ static int sor_iterate(mdx_ctx_t* ctx, const mdx_sor_params& p, int variant) {
     return sor_iteration(ctx, p);
 }
 
+static int sor_iterations(mdx_ctx_t* ctx, const mdx_sor_params& p, int variant, int n) {
+    if (variant == MDX_SORV_RESIDENT) return n > 0 ? mdx_res_face64_run(ctx, p, n) : MDX_OK;
+    for (int it = 0; it < n; ++it) MDX_TRY(sor_iterate(ctx, p, variant));
+    return MDX_OK;
+}
+
 // The IBM factors of this projection's dt_gamma.
 static int mu_tables(mdx_ctx_t* ctx, double dg) {
     const mdx_dims& d = ctx->d;
@@ -827,9 +834,12 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     // the next untried candidate for each residual-check block
     const bool fok = fused_ok(ctx);
     int want = ctx->opts.sor_variant;
-    if (want < MDX_SORV_AUTO || want >= MDX_SORV_NUM) want = MDX_SORV_AUTO;
+    if (want < MDX_SORV_AUTO || want > MDX_SORV_RESIDENT) want = MDX_SORV_AUTO;
+    // where the state fits the SMs the on-chip run is taken without tuning:
+    // it was the fastest on every such grid measured
+    if ((want == MDX_SORV_AUTO || want == MDX_SORV_RESIDENT))
+        want = mdx_res_face64_ok(ctx) ? MDX_SORV_RESIDENT : MDX_SORV_AUTO;
     if (want != MDX_SORV_SWEEPS && !fok) want = MDX_SORV_SWEEPS;
-    if (want == MDX_SORV_AUTO || want == MDX_SORV_FUSED8 || want == MDX_SORV_FUSED16) MDX_TRY(fused_prepare(ctx));
     const bool splitv = want == MDX_SORV_AUTO || want == MDX_SORV_SPLITV;
     if (want == MDX_SORV_AUTO || want == MDX_SORV_SPLIT || splitv) MDX_TRY(split_alloc(ctx));
     const mdx_sor_params p = sor_params(ctx, dg);
@@ -837,7 +847,12 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     // where u, v, w, p live while the sweeps run: the colour-split copies for
     // MDX_SORV_SPLIT blocks, the reference arrays for the others
     bool in_split = false;
+    bool fused_ready = false;
     auto layout_for = [&](int v) -> int {
+        if ((v == MDX_SORV_FUSED8 || v == MDX_SORV_FUSED16) && !fused_ready) {
+            MDX_TRY(fused_prepare(ctx));
+            fused_ready = true;
+        }
         if ((v == MDX_SORV_SPLIT || v == MDX_SORV_SPLITV) != in_split) {
             in_split = !in_split;
             MDX_TRY(split_copy(ctx, in_split));
@@ -862,8 +877,8 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
         MDX_TRY(layout_for(v));
         mdx_event_pair run{};
         mdx_sweep_run_begin(ctx, &run);
-        for (int it = 0; it < o.n_iter; ++it) MDX_TRY(sor_iterate(ctx, p, v));
-        mdx_sweep_run_end(ctx, &run);
+        MDX_TRY(sor_iterations(ctx, p, v, o.n_iter));
+        mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT ? 2LL * o.n_iter : -1);
         MDX_TRY(layout_for(MDX_SORV_SWEEPS));
         s.variant = v;
         s.iterations = o.n_iter;
@@ -891,14 +906,15 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
                 if (timing_block) MDX_CUDA(ctx, cudaEventRecord(ctx->tune_ev[0], ctx->stream));
                 mdx_event_pair run{};
                 mdx_sweep_run_begin(ctx, &run);
-                for (int q = 0; q < m; ++q) MDX_TRY(sor_iterate(ctx, p, v));
-                mdx_sweep_run_end(ctx, &run);
+                MDX_TRY(sor_iterations(ctx, p, v, m));
+                mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT ? 2LL * m : -1);
                 if (timing_block) MDX_CUDA(ctx, cudaEventRecord(ctx->tune_ev[1], ctx->stream));
                 it += m;
                 s.variant = v;
                 double** uvw = in_split ? ctx->split_f : nullptr;
                 MDX_TRY(mdx_k_div_norms(ctx, uvw ? uvw[0] : f[MDX_UN], uvw ? uvw[1] : f[MDX_VN],
                                         uvw ? uvw[2] : f[MDX_WN], &r, &linf));
+                MDX_TRY(mdx_res_check(ctx));
                 if (timing_block) {   // the norms synchronised the stream; time per iteration
                     float ms = 0.f;
                     if (cudaEventElapsedTime(&ms, ctx->tune_ev[0], ctx->tune_ev[1]) == cudaSuccess)

@@ -22,6 +22,8 @@
 // homogeneous ones (the wall faces v(1), v(ny+1) stay 0); IBM factors 1 or
 // z-invariant.  Other boundary sets run the FP64 path.
 #include "mdx_cell32.cuh"
+#include "mdx_pot.cuh"
+#include "mdx_resident.cuh"
 
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
@@ -554,31 +556,6 @@ __global__ void k_mixed_apply(mdx_dims d, double* __restrict__ u, double* __rest
 // of the cells it updates, so no neighbour read tests for a wrap.  Corners
 // are never read.  tests/pot32_model.py restates the sweep thread by thread.
 // ---------------------------------------------------------------------------
-struct pot_geom {
-    int nx, ny, nz;
-    int hq;   // row length of one half (positions)
-    int rz;   // one plane of one half: hq (ny+2)
-    int H;    // one half, a multiple of 64 elements
-};
-
-__host__ __device__ __forceinline__ int pot_row(const pot_geom& L, int h, int j, int k) {
-    return h * L.H + (k * (L.ny + 2) + j) * L.hq;
-}
-__host__ __device__ __forceinline__ int pot_idx(const pot_geom& L, int i, int j, int k) {
-    return pot_row(L, (i + j + k) & 1, j, k) + 3 + (i + 1) / 2;
-}
-
-pot_geom pot_make(const mdx_dims& d) {
-    pot_geom L;
-    L.nx = d.nx;
-    L.ny = d.ny;
-    L.nz = d.nz;
-    L.hq = ((d.nx / 2 + 5) + 3) & ~3;
-    L.rz = L.hq * (d.ny + 2);
-    L.H = (int)((((long long)L.rz * (d.nz + 2)) + 63) & ~63LL);
-    return L;
-}
-
 // Column table: per (i, j) {a_x of the low x face, a_y of the low y face (0
 // at a wall), a_z, fac = -omega/denom}; column nx+1 repeats column 1's a_x,
 // row ny+1 holds the top faces' a_y (0 at walls, row 1's when y is
@@ -1439,6 +1416,10 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
     else if (pot)
         for (int c = 0; c < POT_SHAPES; ++c)
             if (pot_shape_ok(ctx, c)) pcands[npc++] = c;
+    // where the state fits the SMs the on-chip runs are taken without tuning:
+    // they were the fastest on every such grid measured
+    const bool on_chip = pot ? (o.sor_variant < 1 || o.sor_variant > POT_SHAPES) && mdx_res_pot_ok(ctx)
+                             : (o.sor_variant < 1 || o.sor_variant > MDX_SORV_SPLITV) && mdx_res_face32_ok(ctx);
     if (pot && npc > 1 && !ctx->tune_ev[0]) {
         MDX_CUDA(ctx, cudaEventCreate(&ctx->tune_ev[0]));
         MDX_CUDA(ctx, cudaEventCreate(&ctx->tune_ev[1]));
@@ -1480,6 +1461,14 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
         return MDX_OK;
     };
     auto sweeps = [&](int iters) -> int {
+        if (on_chip) {
+            mdx_event_pair run{};
+            mdx_sweep_run_begin(ctx, &run);
+            MDX_TRY(pot ? mdx_res_pot_run(ctx, L, iters) : mdx_res_face32_run(ctx, P, iters));
+            mdx_sweep_run_end(ctx, &run, 2LL * iters);
+            used_kind = pot ? 7 : 1;
+            return MDX_OK;
+        }
         if (pot) return pot_sweeps(iters);
         mdx_event_pair run{};
         int cand = cands[0];
@@ -1551,6 +1540,7 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
                 MDX_TRY(sweeps(m));
                 it += m;
                 MDX_TRY(corr_residual(&e));
+                MDX_TRY(mdx_res_check(ctx));
                 if (!std::isfinite(e)) break;
                 if (e <= inner_target) break;
                 // FP32 stagnation: less than 0.1 % per check_every iterations for 20 x check_every

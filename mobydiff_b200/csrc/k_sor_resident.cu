@@ -1,0 +1,780 @@
+// k_sor_resident.cu -- red-black sweeps with the whole state on chip.
+//
+// One cooperative launch makes a run of iterations (the sweeps between two
+// residual checks).  The grid is cut into one box of rows per SM: by rows in
+// y times bz planes in z, each row whole in x.  A thread owns a fixed
+// (i, j) column window and marches its planes; what only it touches stays in
+// its registers for the whole run, what its block shares lies in shared
+// memory, and only the values on the faces between boxes travel: each as a
+// 16-byte word, its halves a payload and a sequence number each, written
+// straight into the neighbouring block's inbox in global memory (L2) and
+// polled there: there is no separate flag, no fence and no grid barrier, and
+// a block waits for its own neighbours only.  Inboxes alternate by sweep: a
+// block can only write sweep h's words after its neighbours' words of sweep
+// h-1 arrived, which they sent after reading sweep h-2's.
+//
+// What bounds it: for small grids the chain of a sweep -- compute, one L2
+// write, one L2 poll, one block barrier; 1.4 us a colour sweep on 64x32x32,
+// of which 0.4 are the compute.  For grids that fill the SMs the compute and
+// the face words: 2.7 + 2.1 us on 256x128x128 (47 KB of words each way per SM
+// and sweep).  Measured per colour sweep, against the fastest of the other
+// kernels on the same grid: potential form 256x128x128 4.7 us (6.9, one
+// cooperative launch with grid barriers), 116x70x62 1.9 (6.1, a launch per
+// sweep); FP32 faces 118x70x62 2.0 (6.2); FP64 faces 128x64x64 2.8 (6.2).
+//
+// Every wait is bounded: a block that gives up sets the host's error word and
+// returns, and so do its neighbours.  Co-residency comes from the
+// cooperative launch (one block per SM, at most as many blocks as SMs).
+//
+// Per-cell arithmetic: pot_e / sweep32_update (mdx_cell32.cuh) and
+// sor_cell_fac (mdx_cell.cuh), as in the other kernels, so the same bits.
+#include "mdx_cell.cuh"
+#include "mdx_cell32.cuh"
+#include "mdx_pot.cuh"
+#include "mdx_resident.cuh"
+
+#include <type_traits>
+
+namespace {
+
+struct res_box {          // this block's part of the grid
+    int j0, nj, k0, nk;   // first row and number of rows, first plane and number of planes
+    int ylo, yhi, zlo, zhi;   // neighbouring blocks (-1: a wall)
+    int wlo, whi;             // where this block's words start in ylo's y-hi and yhi's y-lo section
+};
+
+__device__ __forceinline__ int cut(int n, int b, int nb) { return (int)(((long long)n * b) / nb); }
+
+template <int PY>
+__device__ __forceinline__ res_box make_box(int ny, int nz, int nyb, int tpr) {
+    res_box b;
+    const int nzb = (int)gridDim.x / nyb;
+    const int yb = (int)blockIdx.x % nyb, zb = (int)blockIdx.x / nyb;
+    b.j0 = 1 + cut(ny, yb, nyb);
+    b.nj = cut(ny, yb + 1, nyb) - cut(ny, yb, nyb);
+    b.k0 = 1 + cut(nz, zb, nzb);
+    b.nk = cut(nz, zb + 1, nzb) - cut(nz, zb, nzb);
+    b.ylo = yb > 0 ? (int)blockIdx.x - 1 : (PY ? (int)blockIdx.x + nyb - 1 : -1);
+    b.yhi = yb + 1 < nyb ? (int)blockIdx.x + 1 : (PY ? (int)blockIdx.x - nyb + 1 : -1);
+    b.zlo = zb > 0 ? (int)blockIdx.x - nyb : (int)blockIdx.x + (nzb - 1) * nyb;
+    b.zhi = zb + 1 < nzb ? (int)blockIdx.x + nyb : (int)blockIdx.x - (nzb - 1) * nyb;
+    auto rows = [&](int y) { return cut(ny, y + 1, nyb) - cut(ny, y, nyb); };
+    const int lo = yb > 0 ? yb - 1 : nyb - 1, hi = yb + 1 < nyb ? yb + 1 : 0;
+    b.wlo = (2 * rows(lo) + (PY || lo > 0 ? b.nk : 0)) * tpr;
+    b.whi = 2 * rows(hi) * tpr;
+    return b;
+}
+
+// The value, unknown to the compiler: what is computed from it inside the
+// iteration loop is computed there again instead of being kept in registers
+// across it (they hold the state).
+__device__ __forceinline__ int here(int x) {
+    asm volatile("" : "+r"(x));
+    return x;
+}
+
+// Two 8-byte halves, each a 32-bit payload and the sequence number: a 64-bit
+// access is atomic, so a half whose number matches holds its payload.  (One
+// number for the whole 16 bytes was tried as a 128-bit access; words of the
+// FP32 faces then came back with the payload of an earlier sweep.)
+struct __align__(16) word { unsigned a, sa, b, sb; };
+
+__device__ __forceinline__ void st_word(word* p, unsigned a, unsigned b, unsigned s) {
+    asm volatile("{ .reg .b64 lo, hi; mov.b64 lo, {%1, %3}; mov.b64 hi, {%2, %3};"
+                 " st.relaxed.gpu.global.v2.b64 [%0], {lo, hi}; }" ::"l"(p), "r"(a), "r"(b), "r"(s)
+                 : "memory");
+}
+__device__ __forceinline__ word ld_word(const word* p) {
+    word w;
+    asm volatile("{ .reg .b64 lo, hi; ld.relaxed.gpu.global.v2.b64 {lo, hi}, [%4];"
+                 " mov.b64 {%0, %1}, lo; mov.b64 {%2, %3}, hi; }"
+                 : "=r"(w.a), "=r"(w.sa), "=r"(w.b), "=r"(w.sb)
+                 : "l"(p)
+                 : "memory");
+    return w;
+}
+// Polls about as long as a second; false when the word did not come.
+constexpr int POLLS = 1 << 20;
+__device__ __forceinline__ bool wait_word(const word* p, unsigned seq, word& w) {
+    for (int n = 0; w.sa != seq || w.sb != seq; ++n) {
+        if (n == POLLS) return false;
+        w = ld_word(p);
+    }
+    return true;
+}
+
+// Inbox of a block: two parities of [z-lo rows | z-hi rows | y-lo planes |
+// y-hi planes], a row or plane of tpr words each, a wall's section empty; the
+// stride is that of the largest box.  The halo words a thread of the block
+// receives are those at its index, T apart.
+struct res_geom {
+    int nyb, by, bz;   // blocks along y; rows and planes of the largest box
+    int tpr;           // words per row
+    __host__ __device__ int words() const { return 2 * (by + bz) * tpr; }
+};
+__device__ __forceinline__ word* inbox(word* box, const res_geom& R, int block, int parity) {
+    return box + ((long long)block * 2 + parity) * R.words();
+}
+
+// ---------------------------------------------------------------------------
+// Potential form (k_sor_mixed.cu): Phi of both colours of the box with a
+// one-row halo in shared memory, r~ and the columns' coefficients in
+// registers.  A thread owns positions q, q+1 of both colours (four cells) of
+// its row in each of its planes.  In plane m its swept cells have odd i when
+// the thread's parity t0 + m is odd (for the first colour; the other way
+// round for the second), so the two coefficient sets are loaded in the order
+// the planes alternate and no select is needed for them.
+//
+// The two cells of a window go through the packed FP32 instructions (each
+// half rounded as the scalar one; c - x is fma(x, -1, c), one rounding), and
+// planes are taken two at a time so that the second plane's loads are in
+// flight while the first is computed.
+// ---------------------------------------------------------------------------
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float lo2(f2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi2(f2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, 0xbf800000bf800000ull, a); }
+__device__ __forceinline__ f2 ld2s(const float* p) { return *reinterpret_cast<const f2*>(p); }
+__device__ __forceinline__ void st2s(float* p, f2 v) { *reinterpret_cast<f2*>(p) = v; }
+
+template <int PY, int KZ>
+__global__ void __launch_bounds__(512, 1)
+k_pot_resident(pot_geom L, res_geom R, int iters, float* __restrict__ phi, const float* __restrict__ r,
+               const float4* __restrict__ tab, word* __restrict__ box, unsigned seq, int* __restrict__ err) {
+    constexpr int NB = 4, PG = KZ > 8 ? 1 : 2;   // words in flight, planes taken together (registers)
+    extern __shared__ __align__(16) float S[];
+    const int half = L.nx / 2, tpr = half / 2, ncol = L.nx + 2;
+    const res_box b = make_box<PY>(L.ny, L.nz, R.nyb, tpr);
+    const int tid = threadIdx.x, T = blockDim.x;
+    const int RZ = (b.nj + 2) * half, SC = RZ * (b.nk + 2);   // one plane, one colour
+    // the last group's second plane may lie one past the halo: read, not used
+    int* const DT = reinterpret_cast<int*>(S + 2 * SC + RZ);  // where each received word goes
+    const int nzw = b.nj * tpr, nyw = b.nk * tpr, nylo = b.ylo >= 0 ? nyw : 0;
+    const int nw = 2 * nzw + nylo + (b.yhi >= 0 ? nyw : 0);
+    // Phi with its halo (the copies of wrapped rows and planes are in global memory)
+    for (int t = tid; t < 2 * (b.nk + 2) * (b.nj + 2) * tpr; t += T) {
+        const int qi = t % tpr, row = t / tpr;
+        const int jj = row % (b.nj + 2), rk = row / (b.nj + 2);
+        const int kk = rk % (b.nk + 2), c = rk / (b.nk + 2);
+        const float2 v = __ldcg(reinterpret_cast<const float2*>(phi + pot_row(L, c, b.j0 - 1 + jj, b.k0 - 1 + kk) + 4) + qi);
+        *reinterpret_cast<float2*>(S + c * SC + kk * RZ + jj * half + 2 * qi) = v;
+    }
+    for (int t = tid; t < nw; t += T) {
+        if (t < 2 * nzw) {
+            const int hi = t >= nzw ? 1 : 0;
+            DT[t] = hi * (b.nk + 1) * RZ + half + 2 * (t - hi * nzw);
+        } else {
+            const int y = t - 2 * nzw, hi = y >= nylo ? 1 : 0, x = y - hi * nylo, m = x / tpr;
+            DT[t] = (m + 1) * RZ + hi * (b.nj + 1) * half + 2 * (x - m * tpr);
+        }
+    }
+    const int jj = tid / tpr, qi = tid - jj * tpr, q = 2 * qi;
+    const bool act = jj < b.nj;
+    const int j = b.j0 + jj;
+    const int o0 = RZ + (jj + 1) * half + q;           // own window of plane 0 of the box
+    const bool par = ((1 + j + b.k0) & 1) != 0;        // first colour, plane 0: swept cells have odd i
+    const int xl = (q == 0 ? half - 1 : -1);           // offset of the x neighbour outside the window, swept
+    const int xr = (q + 2 == half ? 2 - half : 2);     // cells with odd i / even i (x periodic)
+    const int xo[2] = {par ? xl : xr, par ? xr : xl};
+    f2 rr[KZ][2], axl[2], axr[2], ayl[2], ayr[2], az[2], fc[2];
+    if (act) {
+        const float4* t0 = tab + j * ncol + 2 * q + 1;
+        const float4* t1 = t0 + ncol;
+        float4 c[5];
+        float up[4];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) c[m] = __ldg(t0 + m);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) up[m] = __ldg(&t1[m].y);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {   // set s: the cells swept in planes of parity s
+            const bool odd = (s == 0) == par;
+            const float4 a0 = odd ? c[0] : c[1], a1 = odd ? c[2] : c[3], n0 = odd ? c[1] : c[2], n1 = odd ? c[3] : c[4];
+            axl[s] = pack2(a0.x, a1.x);
+            axr[s] = pack2(n0.x, n1.x);
+            ayl[s] = pack2(a0.y, a1.y);
+            ayr[s] = odd ? pack2(up[0], up[2]) : pack2(up[1], up[3]);
+            az[s] = pack2(a0.z, a1.z);
+            fc[s] = pack2(a0.w, a1.w);
+        }
+#pragma unroll
+        for (int m = 0; m < KZ; ++m)
+            if (m < b.nk)
+#pragma unroll
+                for (int c2 = 0; c2 < 2; ++c2)
+                    rr[m][c2] = __ldg(reinterpret_cast<const f2*>(r + pot_row(L, c2, j, b.k0 + m) + 4 + q));
+    }
+    const bool slo = act && jj == 0 && b.ylo >= 0, shi = act && jj == b.nj - 1 && b.yhi >= 0;
+    __syncthreads();
+
+    // one cell pair: swept cells c, other colour's x window z0 and the value
+    // xs beside it, rows ym, yp, planes zm, zp
+    auto cells = [&](int s, f2 rc, f2 c, f2 z0, float xs, f2 ym, f2 yp, f2 zm, f2 zp) -> f2 {
+        const bool odd = (s == 0) == par;
+        const f2 zl = pack2(xs, lo2(z0)), zr = pack2(hi2(z0), xs);
+        f2 e = fma2(axl[s], sub2(c, odd ? zl : z0), rc);   // pot_e
+        e = fma2(axr[s], sub2(c, odd ? z0 : zr), e);
+        e = fma2(ayl[s], sub2(c, ym), e);
+        e = fma2(ayr[s], sub2(c, yp), e);
+        e = fma2(az[s], add2(sub2(c, zm), sub2(c, zp)), e);
+        return fma2(fc[s], e, c);
+    };
+    auto sweep = [&](auto csc, unsigned sq) -> bool {
+        constexpr int CS = decltype(csc)::value;
+        float* W = S + CS * SC;
+        const int ph = (int)(sq & 1u), at = here(tid);
+        if (act) {
+            const float* o = S + (1 - CS) * SC + here(o0);   // the other colour, not written by this sweep
+            float* w = W + here(o0);
+            // this thread's values on the box's surface go to the neighbours
+            // as they are made, so most have arrived when they are waited for
+            auto out = [&](word* p, f2 v) { st_word(p, (unsigned)v, (unsigned)(v >> 32), sq); };
+            word* const yl = inbox(box, R, b.ylo, ph) + b.wlo;
+            word* const yu = inbox(box, R, b.yhi, ph) + b.whi;
+            word* py = (slo ? yl : yu) + here(qi);
+            auto out_y = [&](word* p, f2 v) {
+                out(p, v);
+                if (b.nj == 1 && slo && shi) out(p + (yu - yl), v);
+            };
+            f2 zm = ld2s(o - RZ), z0 = ld2s(o), vt = 0;
+#pragma unroll
+            for (int m = 0; m < KZ; m += PG) {
+                if (m >= b.nk) break;
+                constexpr int s0 = 1 - CS, s1 = CS;        // coefficient sets of even and odd planes' swept cells
+                if constexpr (PG == 2) {
+                    const f2 z1 = ld2s(o + RZ), z2 = ld2s(o + 2 * RZ);
+                    const f2 ym0 = ld2s(o - half), yp0 = ld2s(o + half), c0 = ld2s(w);
+                    const float xs0 = o[xo[s0]];
+                    const f2 ym1 = ld2s(o + RZ - half), yp1 = ld2s(o + RZ + half), c1 = ld2s(w + RZ);
+                    const float xs1 = (o + RZ)[xo[s1]];
+                    const f2 v0 = cells(s0, rr[m][CS], c0, z0, xs0, ym0, yp0, zm, z1);
+                    const f2 v1 = cells(s1, rr[m + 1][CS], c1, z1, xs1, ym1, yp1, z0, z2);
+                    const bool two = m + 1 < b.nk;
+                    st2s(w, v0);
+                    if (two) st2s(w + RZ, v1);
+                    if (m == 0) out(inbox(box, R, b.zlo, ph) + nzw + at, v0);
+                    vt = two ? v1 : v0;
+                    if (slo || shi) {
+                        out_y(py, v0);
+                        if (two) out_y(py + tpr, v1);
+                        py += 2 * tpr;
+                    }
+                    zm = z1;
+                    z0 = z2;
+                    o += 2 * RZ;
+                    w += 2 * RZ;
+                } else {
+                    const f2 z1 = ld2s(o + RZ), ym = ld2s(o - half), yp = ld2s(o + half), c = ld2s(w);
+                    const float xs = o[xo[(m & 1) ? s1 : s0]];
+                    vt = cells((m & 1) ? s1 : s0, rr[m][CS], c, z0, xs, ym, yp, zm, z1);
+                    st2s(w, vt);
+                    if (m == 0) out(inbox(box, R, b.zlo, ph) + nzw + at, vt);
+                    if (slo || shi) {
+                        out_y(py, vt);
+                        py += tpr;
+                    }
+                    zm = z0;
+                    z0 = z1;
+                    o += RZ;
+                    w += RZ;
+                }
+            }
+            out(inbox(box, R, b.zhi, ph) + at, vt);
+        }
+        // the neighbours' values into the halo, NB words in flight per thread
+        const word* in = inbox(box, R, blockIdx.x, ph);
+        bool ok = true;
+        for (int t = at; t < nw; t += NB * T) {
+            word v[NB];
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+                if (t + u * T < nw) v[u] = ld_word(in + t + u * T);
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+                if (t + u * T < nw) {
+                    ok = wait_word(in + t + u * T, sq, v[u]) && ok;
+                    st2s(W + DT[t + u * T], (f2)v[u].a | (f2)v[u].b << 32);
+                }
+        }
+        return __syncthreads_or(!ok) == 0;
+    };
+    for (int it = 0; it < iters; ++it) {
+        // first colour i+j+k odd, as the face form
+        if (!sweep(std::integral_constant<int, 1>(), seq + 2 * it + 1) ||
+            !sweep(std::integral_constant<int, 0>(), seq + 2 * it + 2)) {
+            if (tid == 0) *err = 1;
+            return;
+        }
+    }
+    // back to global memory with the copies of wrapped cells, rows and planes
+    if (!act) return;
+    for (int m = 0; m < b.nk; ++m)
+        for (int c = 0; c < 2; ++c) {
+            const int k = b.k0 + m;
+            const float2 v = *reinterpret_cast<const float2*>(S + c * SC + o0 + m * RZ);
+            float* g = phi + pot_row(L, c, j, k) + 4 + q;
+            auto put = [&](int off) { *reinterpret_cast<float2*>(g + off) = v; };
+            put(0);
+            const bool odd = ((c + j + k) & 1) != 0;
+            if (odd && q == 0) g[half] = v.x;               // cell nx+1 = cell 1
+            if (!odd && q + 2 == half) g[-q - 1] = v.y;     // cell 0 = cell nx
+            if (k == L.nz) put(-L.nz * L.rz);
+            if (k == 1) put(L.nz * L.rz);
+            if (PY && j == L.ny) put(-L.ny * L.hq);
+            if (PY && j == 1) put(L.ny * L.hq);
+        }
+}
+
+// ---------------------------------------------------------------------------
+// Face form: u, v, w, p of the box (FP64), or the corrections du, dv, dw, dp
+// and r~ (FP32).  A thread owns the cell pairs (2 qi + 1, 2 qi + 2) of its
+// row in each of its planes.  In registers: p (and r~) of both cells, the x
+// face between them and the w faces of its columns, the box's top faces
+// included; in shared memory: the x faces between pairs and the y faces.  A
+// face lies between a cell of each colour, so a sweep touches it from one
+// side only: no two threads of a sweep meet.  The y and z faces on the box's
+// surface are held by both blocks; the one whose cell was swept sends it.
+//
+// F[m] / G[m] name the cell of plane m swept by the first / second colour;
+// the column that is F in plane m is G in plane m + 1.  Their side s (0: odd
+// i) alternates with the plane, so the factors are loaded in that order.
+// ---------------------------------------------------------------------------
+enum { MU_NONE = 0, MU_PLANES = 1 };   // IBM factors all 1, or one (i, j) plane per component
+
+template <typename T> struct face_col { T mu_u, mu_ux, mu_v, mu_vy, mu_w, fac; };
+
+template <int PY, int MU>
+struct faces64 {
+    typedef double T;
+    static constexpr bool HAS_R = false;
+    mdx_dims d;
+    mdx_bc_dev bc;
+    mdx_sor_params p;
+    double *u, *v, *w, *q;
+    const double* mu;
+    __device__ __forceinline__ long long at(int i, int j, int k) const { return pidx(d, i, j, k); }
+    __device__ __forceinline__ T res(int, int, int) const { return 0.0; }
+    __device__ __forceinline__ void column(face_col<T>& c, int i, int j) const {
+        c.mu_u = c.mu_ux = c.mu_v = c.mu_vy = c.mu_w = 1.0;
+        if (MU == MU_PLANES) {
+            const long long np = (long long)d.nxp * d.nyp;
+            const int ip = i == d.nx ? 1 : i + 1, jp = (PY && j == d.ny) ? 1 : j + 1;
+            c.mu_u = __ldg(mu + i + (long long)d.nxp * j);
+            c.mu_ux = __ldg(mu + ip + (long long)d.nxp * j);
+            c.mu_v = __ldg(mu + np + i + (long long)d.nxp * j);
+            c.mu_vy = __ldg(mu + np + i + (long long)d.nxp * jp);
+            c.mu_w = __ldg(mu + 2 * np + i + (long long)d.nxp * j);
+        }
+        c.fac = sor_factor(c.mu_u, c.mu_ux, c.mu_v, c.mu_vy, c.mu_w, c.mu_w, p);
+    }
+    // inner: a row that touches no wall
+    __device__ __forceinline__ void cell(const face_col<T>& c, T, T& u_i, T& u_ip, T& v_j, T& v_jp, T& w_k, T& w_kp,
+                                         T& pc, int j, bool inner) const {
+        const T one = 1.0;
+        const T mu_u = MU ? c.mu_u : one, mu_ux = MU ? c.mu_ux : one, mu_v = MU ? c.mu_v : one,
+                mu_vy = MU ? c.mu_vy : one, mu_w = MU ? c.mu_w : one;
+        if (inner)
+            sor_cell_fac<1, 1, 1>(u_i, u_ip, v_j, v_jp, w_k, w_kp, pc, mu_u, mu_ux, mu_v, mu_vy, mu_w, mu_w, c.fac, p,
+                                  bc, 1, j, 1, d.nx, d.ny, d.nz);
+        else
+            sor_cell_fac<1, PY, 1>(u_i, u_ip, v_j, v_jp, w_k, w_kp, pc, mu_u, mu_ux, mu_v, mu_vy, mu_w, mu_w, c.fac, p,
+                                   bc, 1, j, 1, d.nx, d.ny, d.nz);
+    }
+};
+
+template <int PY>
+struct faces32 {
+    typedef float T;
+    static constexpr bool HAS_R = true;
+    mdx_dims d;
+    mixed_params P;
+    float *u, *v, *w, *q;
+    const float *r, *mu, *fac;
+    __device__ __forceinline__ long long at(int i, int j, int k) const { return cidx(d, i, j, k); }
+    __device__ __forceinline__ T res(int i, int j, int k) const { return __ldg(r + cidx(d, i, j, k)); }
+    __device__ __forceinline__ void column(face_col<T>& c, int i, int j) const {
+        const int np = split_plane_elems(d);
+        const int ip = i == d.nx ? 1 : i + 1, jp = (PY && j == d.ny) ? 1 : j + 1;
+        c.mu_u = __ldg(mu + pidx2(d, i, j));
+        c.mu_ux = __ldg(mu + pidx2(d, ip, j));
+        c.mu_v = __ldg(mu + np + pidx2(d, i, j));
+        c.mu_vy = __ldg(mu + np + pidx2(d, i, jp));
+        c.mu_w = __ldg(mu + 2 * np + pidx2(d, i, j));
+        c.fac = __ldg(fac + pidx2(d, i, j));
+    }
+    __device__ __forceinline__ void cell(const face_col<T>& c, T rc, T& u_i, T& u_ip, T& v_j, T& v_jp, T& w_k, T& w_kp,
+                                         T& pc, int j, bool) const {
+        sweep32_update(P, rc, u_i, u_ip, v_j, v_jp, w_k, w_kp, pc, c.mu_u, c.mu_ux, c.mu_v, c.mu_vy, c.mu_w, c.fac,
+                       PY || j > 1, PY || j < d.ny);
+    }
+};
+
+__device__ __forceinline__ void send(word* p, double v, unsigned sq) {
+    st_word(p, (unsigned)__double2loint(v), (unsigned)__double2hiint(v), sq);
+}
+__device__ __forceinline__ void send(word* p, float v, unsigned sq) { st_word(p, __float_as_uint(v), 0u, sq); }
+__device__ __forceinline__ void value(const word& w, double& v) { v = __hiloint2double((int)w.b, (int)w.a); }
+__device__ __forceinline__ void value(const word& w, float& v) { v = __uint_as_float(w.a); }
+
+template <class A, int PY, int KZ, int NT>
+__global__ void __launch_bounds__(NT, 1)
+k_face_resident(const __grid_constant__ A a, res_geom R, int iters, word* __restrict__ box, unsigned seq,
+                int* __restrict__ err) {
+    typedef typename A::T T;
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    const int tpr = a.d.nx / 2, tid = threadIdx.x, NTH = blockDim.x;
+    const res_box b = make_box<PY>(a.d.ny, a.d.nz, R.nyb, tpr);
+    T* const V = reinterpret_cast<T*>(sm_raw);               // [nk][nj + 1][side][tpr]
+    T* const U = V + b.nk * (b.nj + 1) * 2 * tpr;            // [nk][nj][tpr]
+    const int VZ = (b.nj + 1) * 2 * tpr, UZ = b.nj * tpr;    // one plane
+    const int jj = tid / tpr, qi = tid - jj * tpr;
+    const bool act = jj < b.nj;
+    const int j = b.j0 + jj, sb = (j + b.k0) & 1;            // side of F[0]
+    const int qn = qi + 1 == tpr ? 0 : qi + 1;
+    const bool slo = act && jj == 0 && b.ylo >= 0, shi = act && jj == b.nj - 1 && b.yhi >= 0;
+    T pF[KZ], pG[KZ], um[KZ], wF[KZ + 1], wG[KZ + 1], rF[KZ], rG[KZ];
+    face_col<T> col[2];                                      // the columns on side sb and on the other
+    if (act) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) a.column(col[s], 2 * qi + 1 + (sb ^ s), j);
+#pragma unroll
+        for (int m = 0; m <= KZ; ++m)
+            if (m <= b.nk) {   // the top faces wrap to plane 1
+                const int k = b.k0 + m > a.d.nz ? 1 : b.k0 + m;
+                wF[m] = a.w[a.at(2 * qi + 1 + (sb ^ (m & 1)), j, k)];
+                wG[m] = a.w[a.at(2 * qi + 2 - (sb ^ (m & 1)), j, k)];
+            }
+#pragma unroll
+        for (int m = 0; m < KZ; ++m)
+            if (m < b.nk) {
+                const int k = b.k0 + m;
+                const int iF = 2 * qi + 1 + (sb ^ (m & 1)), iG = 2 * qi + 2 - (sb ^ (m & 1));
+                pF[m] = a.q[a.at(iF, j, k)];
+                pG[m] = a.q[a.at(iG, j, k)];
+                if (A::HAS_R) {
+                    rF[m] = a.res(iF, j, k);
+                    rG[m] = a.res(iG, j, k);
+                }
+                um[m] = a.u[a.at(2 * qi + 2, j, k)];
+                U[m * UZ + tid] = a.u[a.at(2 * qi + 1, j, k)];
+                for (int s = 0; s < 2; ++s) {
+                    V[m * VZ + (jj * 2 + s) * tpr + qi] = a.v[a.at(2 * qi + 1 + s, j, k)];
+                    if (jj == b.nj - 1)
+                        V[m * VZ + ((jj + 1) * 2 + s) * tpr + qi] =
+                            a.v[a.at(2 * qi + 1 + s, (PY && j == a.d.ny) ? 1 : j + 1, k)];
+                }
+            }
+    }
+    // where the received y faces go: the offset of their side 0 and, in the
+    // low bit, their side in the first colour's sweeps
+    int* const DT = reinterpret_cast<int*>(U + b.nk * UZ);
+    const int nzw = b.nj * tpr, nyw = b.nk * tpr, nylo = b.ylo >= 0 ? nyw : 0, nw = nylo + (b.yhi >= 0 ? nyw : 0);
+    for (int t = tid; t < nw; t += NTH) {
+        const int hi = t >= nylo ? 1 : 0, x = t - hi * nylo, m = x / tpr;
+        const int row = hi ? b.j0 + b.nj : b.j0 - 1;   // the neighbour's row
+        DT[t] = 2 * (m * VZ + hi * b.nj * 2 * tpr + x - m * tpr) + ((row + b.k0 + m) & 1);
+    }
+    const bool inner = PY || (j > 1 && j < a.d.ny);
+    __syncthreads();
+
+    // one colour sweep: X is swept, Y the other colour's cells
+    auto sweep = [&](auto parc, unsigned sq, T(&pX)[KZ], T(&wX)[KZ + 1], T(&wY)[KZ + 1], const T(&rX)[KZ]) -> bool {
+        constexpr int PAR = decltype(parc)::value;
+        const int ph = (int)(sq & 1u), at = here(tid);
+        const word* const in = inbox(box, R, blockIdx.x, ph);
+        bool ok = true;
+        word zl{}, zh{};
+        if (act) {
+            // sides of the even and odd planes' swept cells, as offsets
+            const int se = sb ^ PAR, so = se ^ 1;
+            T* const v0 = V + here(jj * 2 * tpr + qi);
+            T* const u0 = U + here(jj * tpr);
+            T *ve = v0 + (se ? tpr : 0), *vo = v0 + VZ + (so ? tpr : 0);
+            T *ue = u0 + (se ? qn : qi), *uo = u0 + UZ + (so ? qn : qi);
+            T top = wY[1];
+            word* const yl = inbox(box, R, b.ylo, ph) + b.wlo;
+            word* const yu = inbox(box, R, b.yhi, ph) + b.whi;
+            word* py = (slo ? yl : yu) + here(qi);
+            auto cell = [&](int m, int s, T* u, T* v) {   // and its values on the box's surface to the neighbours
+                T x = *u, vj = v[0], vjp = v[2 * tpr];
+                T ui = s ? um[m] : x, uip = s ? x : um[m];
+                a.cell(col[(m + PAR) & 1], rX[m], ui, uip, vj, vjp, wX[m], wY[m + 1], pX[m], j, inner);
+                um[m] = s ? ui : uip;
+                *u = s ? uip : ui;
+                v[0] = vj;
+                v[2 * tpr] = vjp;
+                top = wY[m + 1];
+                if (slo || shi) {
+                    send(py, slo ? vj : vjp, sq);
+                    if (b.nj == 1 && slo && shi) send(py + (yu - yl), vjp, sq);
+                    py += tpr;
+                }
+            };
+#pragma unroll
+            for (int m = 0; m < KZ; m += 2) {
+                if (m >= b.nk) break;
+                cell(m, se, ue, ve);
+                if (m == 0) send(inbox(box, R, b.zlo, ph) + nzw + at, wX[0], sq);
+                if (m + 1 >= b.nk) break;
+                cell(m + 1, so, uo, vo);
+                ve += 2 * VZ;
+                vo += 2 * VZ;
+                ue += 2 * UZ;
+                uo += 2 * UZ;
+            }
+            send(inbox(box, R, b.zhi, ph) + at, top, sq);
+            zl = ld_word(in + at);
+            zh = ld_word(in + nzw + at);
+        }
+        // the y faces the neighbours' cells moved
+        for (int t = at; t < nw; t += 2 * NTH) {
+            word w[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (t + e * NTH < nw) w[e] = ld_word(in + 2 * nzw + t + e * NTH);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (t + e * NTH < nw) {
+                    ok = wait_word(in + 2 * nzw + t + e * NTH, sq, w[e]) && ok;
+                    const int dst = DT[t + e * NTH];
+                    value(w[e], V[(dst >> 1) + ((dst ^ PAR) & 1 ? tpr : 0)]);
+                }
+        }
+        // the z faces: those of the columns this block did not sweep there
+        if (act) {
+            ok = wait_word(in + at, sq, zl) && ok;
+            ok = wait_word(in + nzw + at, sq, zh) && ok;
+            value(zl, wY[0]);
+            T v;
+            value(zh, v);
+#pragma unroll
+            for (int m = 1; m <= KZ; ++m) wX[m] = m == b.nk ? v : wX[m];   // selected: the index stays a constant
+        }
+        return __syncthreads_or(!ok) == 0;
+    };
+    for (int it = 0; it < iters; ++it) {
+        if (!sweep(std::integral_constant<int, 0>(), seq + 2 * it + 1, pF, wF, wG, rF) ||
+            !sweep(std::integral_constant<int, 1>(), seq + 2 * it + 2, pG, wG, wF, rG)) {
+            if (tid == 0) *err = 1;
+            return;
+        }
+    }
+    if (!act) return;
+#pragma unroll
+    for (int m = 0; m < KZ; ++m) {
+        if (m >= b.nk) break;
+        const int k = b.k0 + m;
+        const int iF = 2 * qi + 1 + (sb ^ (m & 1)), iG = 2 * qi + 2 - (sb ^ (m & 1));
+        a.w[a.at(iF, j, k)] = wF[m];
+        a.w[a.at(iG, j, k)] = wG[m];
+        a.q[a.at(iF, j, k)] = pF[m];
+        a.q[a.at(iG, j, k)] = pG[m];
+        a.u[a.at(2 * qi + 2, j, k)] = um[m];
+        a.u[a.at(2 * qi + 1, j, k)] = U[m * UZ + tid];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            a.v[a.at(2 * qi + 1 + s, j, k)] = V[m * VZ + (jj * 2 + s) * tpr + qi];
+            if (!PY && j == a.d.ny) a.v[a.at(2 * qi + 1 + s, j + 1, k)] = V[m * VZ + ((jj + 1) * 2 + s) * tpr + qi];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Host side: the cut of the grid, the inboxes, the launches.
+// ---------------------------------------------------------------------------
+struct res_shape { int kz, threads; };   // planes a thread can hold; threads its registers leave
+struct res_plan {
+    res_geom R{};
+    int blocks = 0, threads = 0, shape = -1;
+    size_t smem = 0;
+};
+
+// The cut with the shortest sweep: per plane a warp issues about `issue`
+// cycles of the SM's time and no less than 100 in sequence, and a face word
+// costs about a cycle.  ny rows and nz planes are spread over at most one
+// block per SM; a box has at most the shape's planes and threads.
+template <class SM>
+bool make_plan(const mdx_ctx_t* ctx, int tpr, const res_shape* shapes, int nshapes, int issue, SM&& smem, res_plan* out) {
+    const mdx_dims& d = ctx->d;
+    int sms = 0, most = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    double best = 0.0;
+    out->shape = -1;
+    if (tpr < 1 || tpr > 128) return false;
+    for (int s = 0; s < nshapes; ++s)
+        for (int by0 = 1; by0 <= d.ny && by0 * tpr <= shapes[s].threads; ++by0) {
+            const int nyb = (d.ny + by0 - 1) / by0, by = (d.ny + nyb - 1) / nyb;
+            const int nzb = std::min(d.nz, sms / nyb);
+            if (nzb < 1) continue;
+            const int bz = (d.nz + nzb - 1) / nzb;
+            const size_t bytes = smem(by, bz);
+            if (bz > shapes[s].kz || bytes > (size_t)most) continue;
+            const int warps = (by * tpr + 31) / 32;
+            const double cost = (double)bz * std::max(issue * warps, 100) + (double)(by + bz) * tpr + 0.01 * s;
+            if (out->shape >= 0 && cost >= best) continue;
+            best = cost;
+            out->R = res_geom{nyb, by, bz, tpr};
+            out->blocks = nyb * nzb;
+            out->threads = (by * tpr + 31) & ~31;
+            out->shape = s;
+            out->smem = bytes;
+        }
+    return out->shape >= 0;
+}
+
+bool capturing(const mdx_ctx_t* ctx) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return cap != cudaStreamCaptureStatusNone;
+}
+
+// The kernels' error word: in the pinned block of the reductions' results.
+int* err_word(const mdx_ctx_t* ctx) { return reinterpret_cast<int*>(ctx->red_host + 3); }
+
+// Inboxes for the plan and `iters` iterations' sequence numbers.
+int res_prepare(mdx_ctx_t* ctx, const res_plan& P, int iters) {
+    MDX_TRY(mdx_reduce_init(ctx));
+    MDX_TRY(mdx_res_check(ctx));
+    const size_t bytes = sizeof(word) * 2 * (size_t)P.blocks * P.R.words();
+    if (ctx->rs_bytes < bytes) {
+        cudaFree(ctx->rs_box);
+        ctx->rs_box = nullptr;
+        ctx->rs_bytes = 0;
+        MDX_CUDA(ctx, cudaMalloc(&ctx->rs_box, bytes));
+        ctx->rs_bytes = bytes;
+        ctx->rs_seq = 0;
+    }
+    if (ctx->rs_seq == 0 || ctx->rs_seq > 0xffffffffu - 2u * (unsigned)iters - 2u) {
+        MDX_CUDA(ctx, cudaMemsetAsync(ctx->rs_box, 0, ctx->rs_bytes, ctx->stream));
+        ctx->rs_seq = 2;
+    }
+    return MDX_OK;
+}
+
+template <class F, class... Args>
+int res_launch(mdx_ctx_t* ctx, const char* what, F fn, const res_plan& P, int iters, Args... args) {
+    MDX_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+    void* av[] = {&args...};
+    mdx_event_pair p{};
+    mdx_timer_begin(ctx, MDX_T_SOR_SWEEP, &p);
+    MDX_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)fn, dim3(P.blocks), dim3(P.threads), av, P.smem, ctx->stream));
+    mdx_timer_end(ctx, &p);
+    ctx->rs_seq += 2u * (unsigned)iters;
+    return mdx_check_launch(ctx, what);
+}
+
+const res_shape pot_shapes[] = {{4, 512}, {8, 512}, {16, 512}};
+const res_shape face64_shapes[] = {{4, 384}, {8, 320}, {16, 256}};
+const res_shape face32_shapes[] = {{4, 512}, {8, 512}, {16, 384}};
+
+bool pot_plan(const mdx_ctx_t* ctx, res_plan* P) {
+    const int half = ctx->d.nx / 2;
+    return make_plan(ctx, half / 2, pot_shapes, 3, 10,
+                     [&](int by, int bz) { return sizeof(float) * ((size_t)(by + 2) * (2 * bz + 5) * half + (size_t)(by + bz) * half); }, P);
+}
+template <typename T>
+bool face_plan(const mdx_ctx_t* ctx, const res_shape* shapes, int issue, res_plan* P) {
+    const int tpr = ctx->d.nx / 2;
+    return make_plan(ctx, tpr, shapes, 3, issue,
+                     [&](int by, int bz) { return sizeof(T) * (size_t)(bz + 1) * tpr * (2 * (by + 1) + by) + sizeof(int) * 2 * (size_t)bz * tpr; }, P);
+}
+
+template <int PY>
+int pot_run(mdx_ctx_t* ctx, const pot_geom& L, int iters) {
+    res_plan P;
+    if (!pot_plan(ctx, &P)) return mdx_fail(ctx, MDX_ERR_ARG, "resident sweeps: the grid does not fit the SMs");
+    MDX_TRY(res_prepare(ctx, P, iters));
+    auto fn = P.shape == 0 ? k_pot_resident<PY, 4> : P.shape == 1 ? k_pot_resident<PY, 8> : k_pot_resident<PY, 16>;
+    return res_launch(ctx, "pot resident", fn, P, iters, L, P.R, iters, ctx->pt_phi, (const float*)ctx->pt_r,
+                      (const float4*)ctx->pt_tab, (word*)ctx->rs_box, ctx->rs_seq, err_word(ctx));
+}
+
+template <class A, int PY, int N4, int N8, int N16>
+int face_run(mdx_ctx_t* ctx, const A& a, const res_plan& P, int iters) {
+    MDX_TRY(res_prepare(ctx, P, iters));
+    auto fn = P.shape == 0 ? k_face_resident<A, PY, 4, N4>
+                           : P.shape == 1 ? k_face_resident<A, PY, 8, N8> : k_face_resident<A, PY, 16, N16>;
+    return res_launch(ctx, "face resident", fn, P, iters, a, P.R, iters, (word*)ctx->rs_box, ctx->rs_seq, err_word(ctx));
+}
+
+template <int PY, int MU>
+int face64_run(mdx_ctx_t* ctx, const mdx_sor_params& p, const res_plan& P, int iters) {
+    double** f = ctx->f;
+    const faces64<PY, MU> a{ctx->d, ctx->bcd, p, f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN], ctx->mu};
+    return face_run<faces64<PY, MU>, PY, 384, 320, 256>(ctx, a, P, iters);
+}
+template <int PY>
+int face32_run(mdx_ctx_t* ctx, const mixed_params& q, const res_plan& P, int iters) {
+    const faces32<PY> a{ctx->d, q, ctx->mx_du, ctx->mx_dv, ctx->mx_dw, ctx->mx_dp, ctx->mx_r, ctx->mx_mu, ctx->mx_fac};
+    return face_run<faces32<PY>, PY, 512, 512, 384>(ctx, a, P, iters);
+}
+
+}  // namespace
+
+bool mdx_res_pot_ok(mdx_ctx_t* ctx) {
+    res_plan P;
+    return pot_plan(ctx, &P) && !capturing(ctx);
+}
+bool mdx_res_face32_ok(mdx_ctx_t* ctx) {
+    res_plan P;
+    return face_plan<float>(ctx, face32_shapes, 12, &P) && !capturing(ctx);
+}
+bool mdx_res_face64_ok(mdx_ctx_t* ctx) {
+    res_plan P;
+    return ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL &&
+           face_plan<double>(ctx, face64_shapes, 18, &P) && !capturing(ctx);
+}
+
+int mdx_res_pot_run(mdx_ctx_t* ctx, const pot_geom& L, int iters) {
+    return ctx->bc.is_periodic[1] ? pot_run<1>(ctx, L, iters) : pot_run<0>(ctx, L, iters);
+}
+int mdx_res_face32_run(mdx_ctx_t* ctx, const mixed_params& q, int iters) {
+    res_plan P;
+    if (!face_plan<float>(ctx, face32_shapes, 12, &P))
+        return mdx_fail(ctx, MDX_ERR_ARG, "resident sweeps: the grid does not fit the SMs");
+    return ctx->bc.is_periodic[1] ? face32_run<1>(ctx, q, P, iters) : face32_run<0>(ctx, q, P, iters);
+}
+int mdx_res_face64_run(mdx_ctx_t* ctx, const mdx_sor_params& p, int iters) {
+    res_plan P;
+    if (!face_plan<double>(ctx, face64_shapes, 18, &P))
+        return mdx_fail(ctx, MDX_ERR_ARG, "resident sweeps: the grid does not fit the SMs");
+    if (ctx->mu_mode == MU_ONE)
+        return ctx->bc.is_periodic[1] ? face64_run<1, MU_NONE>(ctx, p, P, iters) : face64_run<0, MU_NONE>(ctx, p, P, iters);
+    return ctx->bc.is_periodic[1] ? face64_run<1, MU_PLANES>(ctx, p, P, iters) : face64_run<0, MU_PLANES>(ctx, p, P, iters);
+}
+
+int mdx_res_check(mdx_ctx_t* ctx) {
+    if (!ctx->red_host || *(volatile int*)err_word(ctx) == 0) return MDX_OK;
+    *err_word(ctx) = 0;
+    ctx->rs_seq = 0;   // the inboxes are cleared before the next run
+    return mdx_fail(ctx, MDX_ERR_TIMEOUT, "resident red-black sweeps: a block gave up waiting for its neighbour");
+}
+
+void mdx_res_free(mdx_ctx_t* ctx) {
+    cudaFree(ctx->rs_box);
+    ctx->rs_box = nullptr;
+    ctx->rs_bytes = 0;
+    ctx->rs_seq = 0;
+}

@@ -361,7 +361,8 @@ int mdx_reduce_init(mdx_ctx_t* ctx) {
     ctx->red_blocks = sms * 4;
     MDX_CUDA(ctx, cudaMalloc(&ctx->red_part, sizeof(double) * 3 * ctx->red_blocks));
     MDX_CUDA(ctx, cudaMalloc(&ctx->red_out, sizeof(double) * 3));
-    MDX_CUDA(ctx, cudaMallocHost(&ctx->red_host, sizeof(double) * 3));
+    MDX_CUDA(ctx, cudaMallocHost(&ctx->red_host, sizeof(double) * 4));
+    ctx->red_host[3] = 0.0;
     MDX_CUDA(ctx, cudaEventCreate(&ctx->tune_ev[0]));
     MDX_CUDA(ctx, cudaEventCreate(&ctx->tune_ev[1]));
     return MDX_OK;

@@ -65,7 +65,8 @@ __host__ __device__ inline int split_plane_elems(const mdx_dims& d) { return 2 *
 // Red-black kernel variants (opts.sor_variant; k_sor.cu, k_sor_mixed.cu).
 enum {
     MDX_SORV_AUTO = 0, MDX_SORV_SWEEPS = 1, MDX_SORV_FUSED8 = 2, MDX_SORV_FUSED16 = 3, MDX_SORV_SPLIT = 4,
-    MDX_SORV_SPLITV = 5, MDX_SORV_NUM = 6
+    MDX_SORV_SPLITV = 5, MDX_SORV_NUM = 6,
+    MDX_SORV_RESIDENT = 6   // the whole state on chip (k_sor_resident.cu), where it fits
 };
 
 // A step scalar (dt times an RK coefficient) handed to a kernel either by
@@ -154,6 +155,11 @@ struct mdx_ctx {
     int pt_tuned = 0;                        // candidate + 1 chosen by the autotuner (0: not yet)
     unsigned pt_attr = 0;                    // staged sweeps: shared-memory attribute set, bit per kernel
     double pt_tune_ms[16] = {0.0};            // time per iteration per candidate
+    // on-chip red-black runs (k_sor_resident.cu): the blocks' inboxes, the last
+    // sequence number used (0: the inboxes are to be cleared)
+    void* rs_box = nullptr;
+    size_t rs_bytes = 0;
+    unsigned rs_seq = 0;
     // warm starts: increments of the last projection of each RK substage
     int guess_mode = 0;                      // MDX_GUESS_*
     bool record_increments = false;
@@ -199,7 +205,7 @@ struct mdx_ctx {
     double* red_part = nullptr;              // per-block partials (2 per block)
     int red_blocks = 0;
     double* red_out = nullptr;               // device result [2]
-    double* red_host = nullptr;              // pinned host result [2]
+    double* red_host = nullptr;              // pinned host result [3], then the on-chip runs' error word
 
     mdx_solve_stats_t last{};
 

@@ -1,0 +1,22 @@
+// mdx_resident.cuh -- host interface of the on-chip red-black runs
+// (k_sor_resident.cu).
+#pragma once
+
+#include "mdx_internal.cuh"
+#include "mdx_cell32.cuh"
+#include "mdx_pot.cuh"
+
+// Whether the grid's whole state fits the SMs in that form (and the stream is
+// not being captured: a replay would repeat the words' sequence numbers).
+bool mdx_res_pot_ok(mdx_ctx_t* ctx);
+bool mdx_res_face32_ok(mdx_ctx_t* ctx);
+bool mdx_res_face64_ok(mdx_ctx_t* ctx);
+// `iters` red-black iterations in one launch on, respectively, Phi, the FP32
+// corrections and the FP64 fields.
+int mdx_res_pot_run(mdx_ctx_t* ctx, const pot_geom& L, int iters);
+int mdx_res_face32_run(mdx_ctx_t* ctx, const mixed_params& P, int iters);
+struct mdx_sor_params;
+int mdx_res_face64_run(mdx_ctx_t* ctx, const mdx_sor_params& p, int iters);
+// After a synchronisation: MDX_ERR_TIMEOUT when a run gave up a wait.
+int mdx_res_check(mdx_ctx_t* ctx);
+void mdx_res_free(mdx_ctx_t* ctx);
