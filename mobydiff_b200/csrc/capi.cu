@@ -631,14 +631,14 @@ static int rk_step_eager(mdx_ctx_t* ctx, double dt, long long* iters, const doub
         const double da = dt * a[s], db = dt * b[s], dg = dt * c[s];
         if (dtp) {
             MDX_TRY(mdx_k_momentum(ctx, mdx_dscal(dtp, a[s]), mdx_dscal(dtp, b[s]), mdx_dscal(dtp, c[s])));
-            MDX_TRY(mdx_k_apply_bc(ctx));
+            MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_STAR));
             MDX_TRY(mdx_k_projection_fft(ctx, mdx_dscal(dtp, c[s])));
-            MDX_TRY(mdx_k_apply_bc(ctx));
+            MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_N));
             continue;
         }
         MDX_TRY(mdx_k_momentum(ctx, da, db, dg));
         if (ctx->opts.solver == MDX_SOLVER_FFT) {
-            MDX_TRY(mdx_k_apply_bc(ctx));
+            MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_STAR));
             MDX_TRY(mdx_k_projection_fft(ctx, dg));
             if (ctx->opts.precision == MDX_PREC_MIXED) {
                 if (iters) *iters += ctx->last.iterations;
@@ -646,7 +646,7 @@ static int rk_step_eager(mdx_ctx_t* ctx, double dt, long long* iters, const doub
                     return mdx_fail(ctx, ctx->last.status, "FFT defect correction ended with status %d",
                                     ctx->last.status);
             }
-            MDX_TRY(mdx_k_apply_bc(ctx));
+            MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_N));
         } else {
             mdx_solve_stats_t st{};
             MDX_TRY(mdx_k_projection_redblack(ctx, dg, &st));

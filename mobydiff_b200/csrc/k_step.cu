@@ -8,9 +8,11 @@
 // coefficients are zero is exact: 1/(1+dt_gamma*0) == 1.
 #include "mdx_cell.cuh"
 
+#include <type_traits>
+
 // ---------------------------------------------------------------------------
 // Predictor, src/modules/step.f90:76-204.  A block is a 32 x 8 (i, j) tile
-// that walks MOM_KZ planes along z; each thread carries the values its
+// that walks KZ planes along z; each thread carries the values its
 // stencil reuses from plane to plane in registers (u, v, w, p at the cell in
 // planes k-1..k+1, u(i+1) and v(j+1) of plane k-1, w(i-1) and w(j-1) of
 // plane k+1), so per cell it reads the five values of plane k+1 it will need
@@ -18,11 +20,10 @@
 // read 32 consecutive doubles of every array.  The arithmetic is
 // momentum_vals, the same as the ensemble kernel's.
 // ---------------------------------------------------------------------------
-constexpr int MOM_KZ = 8;
 
 // DTD: the three step scalars come from the device's dt (adaptive-dt graph);
 // otherwise their values are kernel parameters.
-template <bool IBM, bool DTD>
+template <bool IBM, bool DTD, int KZ>
 __global__ void __launch_bounds__(256, 4)
 k_momentum(mdx_dims d, mdx_step_params p, mdx_dscal da, mdx_dscal db, mdx_dscal dg,
            const double* __restrict__ un, const double* __restrict__ vn, const double* __restrict__ wn,
@@ -31,11 +32,11 @@ k_momentum(mdx_dims d, mdx_step_params p, mdx_dscal da, mdx_dscal db, mdx_dscal 
            const double* __restrict__ cu, const double* __restrict__ cv, const double* __restrict__ cw) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k0 = blockIdx.z * MOM_KZ + 1;
+    const int k0 = blockIdx.z * KZ + 1;
     if (i > d.nx || j > d.ny) return;
     const double dt_alpha = DTD ? da.get() : da.v, dt_beta = DTD ? db.get() : db.v,
                  dt_gamma = DTD ? dg.get() : dg.v;
-    const int k1 = min(k0 + MOM_KZ - 1, d.nz);
+    const int k1 = min(k0 + KZ - 1, d.nz);
     const long long SX = 1, SY = d.nxp, SZ = (long long)d.nxp * d.nyp;
     long long c = pidx(d, i, j, k0);
     long long q = qidx(d, i, j, k0);
@@ -91,92 +92,76 @@ mdx_step_params mdx_make_params(const mdx_ctx_t* ctx) {
 int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg) {
     const mdx_dims& d = ctx->d;
     dim3 block(32, 8, 1);
-    dim3 grid((d.nx + 31) / 32, (d.ny + 7) / 8, (d.nz + MOM_KZ - 1) / MOM_KZ);
+    // planes per block: 8 (the values carried from plane to plane), fewer while
+    // the blocks would not give every SM four (its resident blocks)
+    dim3 grid((d.nx + 31) / 32, (d.ny + 7) / 8);
+    int kz = 8;
+    while (kz > 1 && (long long)grid.x * grid.y * ((d.nz + kz - 1) / kz) < 4 * 148) kz = kz == 8 ? 2 : 1;
+    grid.z = (d.nz + kz - 1) / kz;
     mdx_step_params p = mdx_make_params(ctx);
     double** f = ctx->f;
     const bool dev = da.p || db.p || dg.p;
-    auto kfn = ctx->ibm_zero ? (dev ? k_momentum<false, true> : k_momentum<false, false>)
-                             : (dev ? k_momentum<true, true> : k_momentum<true, false>);
-    MDX_LAUNCH(ctx, MDX_T_MOMENTUM, "momentum", kfn, grid, block, 0, d, p, da, db, dg, f[MDX_UN], f[MDX_VN],
-               f[MDX_WN], f[MDX_PN], f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_OLDRHSU], f[MDX_OLDRHSV], f[MDX_OLDRHSW],
-               f[MDX_COEF_U], f[MDX_COEF_V], f[MDX_COEF_W]);
+    auto go = [&](auto kc) -> int {
+        constexpr int K = decltype(kc)::value;
+        auto kfn = ctx->ibm_zero ? (dev ? k_momentum<false, true, K> : k_momentum<false, false, K>)
+                                 : (dev ? k_momentum<true, true, K> : k_momentum<true, false, K>);
+        MDX_LAUNCH(ctx, MDX_T_MOMENTUM, "momentum", kfn, grid, block, 0, d, p, da, db, dg, f[MDX_UN], f[MDX_VN],
+                   f[MDX_WN], f[MDX_PN], f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_OLDRHSU], f[MDX_OLDRHSV],
+                   f[MDX_OLDRHSW], f[MDX_COEF_U], f[MDX_COEF_V], f[MDX_COEF_W]);
+        return MDX_OK;
+    };
+    if (kz == 8) MDX_TRY(go(std::integral_constant<int, 8>()));
+    else if (kz >= 2) MDX_TRY(go(std::integral_constant<int, 2>()));
+    else MDX_TRY(go(std::integral_constant<int, 1>()));
     return MDX_OK;
 }
 
 // ---------------------------------------------------------------------------
-// apply_bc of the FFT builds, src/modules/boundary.f90:23-170, as the
-// reference's three sequential phases (y walls, x periodic, z periodic).
-// Each phase writes only ghost planes (plus the v wall row) and reads
-// interior or already-final values, so threads within a phase never race.
+// apply_bc of the FFT builds, src/modules/boundary.f90:23-170: walls in y
+// (:48-67), then the periodic copies in x (:87-117) and z (:137-168) of u, v,
+// w and, for the n arrays, p.  The three sequential phases composed: a ghost
+// value is that of the interior cell its x and z wrap lead to, negated (u, w)
+// beyond a y wall; v is 0 on both wall rows and left alone in row 0, p in its
+// y ghost rows.  Every source is an interior value that no thread writes, so
+// one launch sets all of them (three ordered launches before, 6.7 + 9.8 + 9.4
+// us on 64x32x32).
 // ---------------------------------------------------------------------------
-struct mdx_six { double *un, *vn, *wn, *us, *vs, *ws, *pn; };
+struct mdx_bc_set { mdx_four a, b; };   // one or two sets of arrays (b.un null: one; pn null: no p)
 
-__global__ void k_bc_walls_y(mdx_dims d, mdx_six f) {   // boundary.f90:48-67
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i > d.nx + 1 || k > d.nz + 1) return;
-    const int ny = d.ny;
-    f.un[pidx(d, i, ny + 1, k)] = -f.un[pidx(d, i, ny, k)];
-    f.vn[pidx(d, i, ny + 1, k)] = 0.0;
-    f.wn[pidx(d, i, ny + 1, k)] = -f.wn[pidx(d, i, ny, k)];
-    f.un[pidx(d, i, 0, k)] = -f.un[pidx(d, i, 1, k)];
-    f.vn[pidx(d, i, 1, k)] = 0.0;
-    f.wn[pidx(d, i, 0, k)] = -f.wn[pidx(d, i, 1, k)];
-    f.us[pidx(d, i, ny + 1, k)] = -f.us[pidx(d, i, ny, k)];
-    f.vs[pidx(d, i, ny + 1, k)] = 0.0;
-    f.ws[pidx(d, i, ny + 1, k)] = -f.ws[pidx(d, i, ny, k)];
-    f.us[pidx(d, i, 0, k)] = -f.us[pidx(d, i, 1, k)];
-    f.vs[pidx(d, i, 1, k)] = 0.0;
-    f.ws[pidx(d, i, 0, k)] = -f.ws[pidx(d, i, 1, k)];
-}
-
-__global__ void k_bc_periodic_x(mdx_dims d, mdx_six f) {   // boundary.f90:87-117
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y * blockDim.y + threadIdx.y;
-    if (j > d.ny + 1 || k > d.nz + 1) return;
-    const int nx = d.nx;
-    f.un[pidx(d, 0, j, k)] = f.un[pidx(d, nx, j, k)];
-    f.wn[pidx(d, 0, j, k)] = f.wn[pidx(d, nx, j, k)];
-    f.un[pidx(d, nx + 1, j, k)] = f.un[pidx(d, 1, j, k)];
-    f.wn[pidx(d, nx + 1, j, k)] = f.wn[pidx(d, 1, j, k)];
-    f.us[pidx(d, 0, j, k)] = f.us[pidx(d, nx, j, k)];
-    f.ws[pidx(d, 0, j, k)] = f.ws[pidx(d, nx, j, k)];
-    f.us[pidx(d, nx + 1, j, k)] = f.us[pidx(d, 1, j, k)];
-    f.ws[pidx(d, nx + 1, j, k)] = f.ws[pidx(d, 1, j, k)];
-    if (j >= 1) {
-        f.vn[pidx(d, 0, j, k)] = f.vn[pidx(d, nx, j, k)];
-        f.vn[pidx(d, nx + 1, j, k)] = f.vn[pidx(d, 1, j, k)];
-        f.vs[pidx(d, 0, j, k)] = f.vs[pidx(d, nx, j, k)];
-        f.vs[pidx(d, nx + 1, j, k)] = f.vs[pidx(d, 1, j, k)];
-    }
-    if (j >= 1 && j <= d.ny) {
-        f.pn[pidx(d, 0, j, k)] = f.pn[pidx(d, nx, j, k)];
-        f.pn[pidx(d, nx + 1, j, k)] = f.pn[pidx(d, 1, j, k)];
-    }
-}
-
-__global__ void k_bc_periodic_z(mdx_dims d, mdx_six f) {   // boundary.f90:137-168
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i > d.nx + 1 || j > d.ny + 1) return;
-    const int nz = d.nz;
-    f.un[pidx(d, i, j, 0)] = f.un[pidx(d, i, j, nz)];
-    f.wn[pidx(d, i, j, 0)] = f.wn[pidx(d, i, j, nz)];
-    f.un[pidx(d, i, j, nz + 1)] = f.un[pidx(d, i, j, 1)];
-    f.wn[pidx(d, i, j, nz + 1)] = f.wn[pidx(d, i, j, 1)];
-    f.us[pidx(d, i, j, 0)] = f.us[pidx(d, i, j, nz)];
-    f.ws[pidx(d, i, j, 0)] = f.ws[pidx(d, i, j, nz)];
-    f.us[pidx(d, i, j, nz + 1)] = f.us[pidx(d, i, j, 1)];
-    f.ws[pidx(d, i, j, nz + 1)] = f.ws[pidx(d, i, j, 1)];
-    if (j >= 1) {
-        f.vn[pidx(d, i, j, 0)] = f.vn[pidx(d, i, j, nz)];
-        f.vn[pidx(d, i, j, nz + 1)] = f.vn[pidx(d, i, j, 1)];
-        f.vs[pidx(d, i, j, 0)] = f.vs[pidx(d, i, j, nz)];
-        f.vs[pidx(d, i, j, nz + 1)] = f.vs[pidx(d, i, j, 1)];
-    }
-    if (j >= 1 && j <= d.ny) {
-        f.pn[pidx(d, i, j, 0)] = f.pn[pidx(d, i, j, nz)];
-        f.pn[pidx(d, i, j, nz + 1)] = f.pn[pidx(d, i, j, 1)];
+__global__ void k_bc_fft(mdx_dims d, mdx_bc_set sets) {
+    const int face = blockIdx.z % 3;   // z planes, y rows, x columns
+    const mdx_four f = blockIdx.z < 3 ? sets.a : sets.b;
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
+    const int nx = d.nx, ny = d.ny, nz = d.nz;
+    auto put = [&](int i, int j, int k) {
+        const int si = i == 0 ? nx : i == nx + 1 ? 1 : i, sk = k == 0 ? nz : k == nz + 1 ? 1 : k;
+        const long long c = pidx(d, i, j, k);
+        if (j == 0 || j == ny + 1) {
+            const long long s = pidx(d, si, j == 0 ? 1 : ny, sk);
+            f.un[c] = -f.un[s];
+            f.wn[c] = -f.wn[s];
+            if (j == ny + 1) f.vn[c] = 0.0;
+        } else {
+            const long long s = pidx(d, si, j, sk);
+            f.un[c] = f.un[s];
+            f.wn[c] = f.wn[s];
+            f.vn[c] = j == 1 ? 0.0 : f.vn[s];
+            if (f.pn) f.pn[c] = f.pn[s];
+        }
+    };
+    if (face == 0) {
+        if (a > nx + 1 || b > ny + 1) return;
+        put(a, b, 0);
+        put(a, b, nz + 1);
+    } else if (face == 1) {
+        if (a > nx + 1 || b >= nz) return;
+        put(a, 0, b + 1);
+        put(a, ny + 1, b + 1);
+        f.vn[pidx(d, a, 1, b + 1)] = 0.0;
+    } else {
+        if (a >= ny || b >= nz) return;
+        put(0, a + 1, b + 1);
+        put(nx + 1, a + 1, b + 1);
     }
 }
 
@@ -184,7 +169,7 @@ __global__ void k_bcrb_y(mdx_dims d, mdx_bc_dev bc, double dy, mdx_four f);
 __global__ void k_bcrb_x(mdx_dims d, mdx_bc_dev bc, double dx, mdx_four f);
 __global__ void k_bcrb_z(mdx_dims d, mdx_bc_dev bc, double dz, mdx_four f);
 
-int mdx_k_apply_bc(mdx_ctx_t* ctx) {
+int mdx_k_apply_bc(mdx_ctx_t* ctx, int which) {
     const mdx_dims& d = ctx->d;
     double** a = ctx->f;
     if (ctx->fft_ext_x || ctx->fft_ext_z) {
@@ -193,8 +178,11 @@ int mdx_k_apply_bc(mdx_ctx_t* ctx) {
         // velocity give apply_bc's values) on u, v, w, p and on u*, v*, w*,
         // whose wall faces the right-hand side reads
         dim3 b(32, 8);
-        for (const mdx_four& f : {mdx_four{a[MDX_UN], a[MDX_VN], a[MDX_WN], a[MDX_PN]},
-                                  mdx_four{a[MDX_US], a[MDX_VS], a[MDX_WS], a[MDX_PN]}}) {
+        const mdx_four sets[2] = {mdx_four{a[MDX_UN], a[MDX_VN], a[MDX_WN], a[MDX_PN]},
+                                  mdx_four{a[MDX_US], a[MDX_VS], a[MDX_WS], a[MDX_PN]}};
+        for (int t = 0; t < 2; ++t) {
+            if (!(which & (1 << t))) continue;
+            const mdx_four& f = sets[t];
             MDX_LAUNCH(ctx, MDX_T_BC, "apply_bc y (walls)", k_bcrb_y, dim3((d.nx + 31) / 32, (d.nz + 7) / 8), b, 0, d,
                        ctx->bcd, ctx->g.dy, f);
             MDX_LAUNCH(ctx, MDX_T_BC, "apply_bc x (walls)", k_bcrb_x, dim3((d.ny + 31) / 32, (d.nz + 7) / 8), b, 0, d,
@@ -204,11 +192,10 @@ int mdx_k_apply_bc(mdx_ctx_t* ctx) {
         }
         return MDX_OK;
     }
-    mdx_six f{a[MDX_UN], a[MDX_VN], a[MDX_WN], a[MDX_US], a[MDX_VS], a[MDX_WS], a[MDX_PN]};
-    dim3 b(32, 8);
-    MDX_LAUNCH(ctx, MDX_T_BC, "apply_bc y", k_bc_walls_y, dim3((d.nxp + 31) / 32, (d.nzp + 7) / 8), b, 0, d, f);
-    MDX_LAUNCH(ctx, MDX_T_BC, "apply_bc x", k_bc_periodic_x, dim3((d.nyp + 31) / 32, (d.nzp + 7) / 8), b, 0, d, f);
-    MDX_LAUNCH(ctx, MDX_T_BC, "apply_bc z", k_bc_periodic_z, dim3((d.nxp + 31) / 32, (d.nyp + 7) / 8), b, 0, d, f);
+    const mdx_four n{a[MDX_UN], a[MDX_VN], a[MDX_WN], a[MDX_PN]}, s{a[MDX_US], a[MDX_VS], a[MDX_WS], nullptr};
+    const mdx_bc_set sets{(which & MDX_BC_N) ? n : s, which == MDX_BC_ALL ? s : mdx_four{}};
+    dim3 grid((std::max(d.nxp, d.ny) + 31) / 32, (std::max(d.nyp, d.nz) + 7) / 8, which == MDX_BC_ALL ? 6 : 3);
+    MDX_LAUNCH(ctx, MDX_T_BC, "apply_bc", k_bc_fft, grid, dim3(32, 8), 0, d, sets);
     return MDX_OK;
 }
 

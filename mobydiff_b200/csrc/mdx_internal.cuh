@@ -99,12 +99,15 @@ struct mdx_bc_dev {
 };
 __host__ __device__ inline int bci(int dir, int side, int var) { return (dir - 1) + 3 * (side + 2 * var); }
 
-// FFT plan for one length: radix list and twiddle table exp(-2 pi i t/n).
+// FFT plan for one length: radix list (twiddles exp(-2 pi i t/n) beside it).
 #define MDX_MAX_STAGES 16
 struct mdx_fft_plan {
     int n;
     int nstages;
     int radix[MDX_MAX_STAGES];
+    // floor(2^32 / d) + 1 for d = n/radix and d = the product of the radices
+    // before (0 for d = 1): t / d = umulhi(t, inv), exact for t d < 2^32
+    unsigned inv_nr[MDX_MAX_STAGES], inv_ns[MDX_MAX_STAGES];
 };
 
 struct mdx_event_pair { cudaEvent_t a, b; int cls; long long n; };   // n: launches inside the pair
@@ -303,7 +306,11 @@ int mdx_check_launch(mdx_ctx_t* ctx, const char* what);
 // ---- per-module entry points (internal) --------------------------------------
 mdx_step_params mdx_make_params(const mdx_ctx_t* ctx);
 int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg);
-int mdx_k_apply_bc(mdx_ctx_t* ctx);
+// apply_bc on the n arrays (un, vn, wn, pn), the * arrays or both.  Inside a
+// step the * arrays need it after the predictor and the n arrays after the
+// projection: the other set has not changed since it was last set.
+enum { MDX_BC_N = 1, MDX_BC_STAR = 2, MDX_BC_ALL = 3 };
+int mdx_k_apply_bc(mdx_ctx_t* ctx, int which = MDX_BC_ALL);
 int mdx_k_apply_bc_redblack(mdx_ctx_t* ctx);
 int mdx_fft_init(mdx_ctx_t* ctx);
 void mdx_fft_free(mdx_ctx_t* ctx);
