@@ -39,18 +39,22 @@
 void mdx_fft_make_plan(int n, mdx_fft_plan* p, bool* ok) {
     p->n = n;
     p->nstages = 0;
-    int m = n;
+    int m = n, Ns = 1;
     *ok = true;
-    for (int r : {4, 2, 3, 5, 7}) {
+    // odd radices first: the first stage's writes are r elements apart, free
+    // of bank conflicts when r is odd; then as few stages as possible
+    for (int r : {7, 5, 3, 8, 4, 2}) {
         while (m % r == 0) {
             if (p->nstages >= MDX_MAX_STAGES) { *ok = false; return; }
-            p->radix[p->nstages++] = r;
+            const int nr = n / r, s = p->nstages++;
+            p->radix[s] = r;
+            p->inv_nr[s] = nr > 1 ? (unsigned)((1ull << 32) / (unsigned)nr) + 1u : 0u;
+            p->inv_ns[s] = Ns > 1 ? (unsigned)((1ull << 32) / (unsigned)Ns) + 1u : 0u;
+            Ns *= r;
             m /= r;
         }
     }
     if (m != 1) *ok = false;
-    // one radix-2 stage is cheaper at the end than between radix-4 stages
-    // only in bank terms; keep the order 4..4,2,3,5,7.
 }
 
 void mdx_fft_twiddles(int n, std::vector<double2>& tw) {
@@ -101,61 +105,148 @@ __device__ __forceinline__ C2 twid(const C2* __restrict__ tw, int t) {
     return w;
 }
 
-// Radix-r DFT in registers.  For r = 3, 5, 7 the roots come from the table:
-// W_r^m = tw[m * (n/r) * tws].
-template <bool INV, typename C2>
-__device__ __forceinline__ void dft_r(C2* a, int r, const C2* __restrict__ tw, int root_step) {
-    if (r == 2) {
+// a / b for a divisor used again and again: q = a rb corrected by one fused
+// residual step, rb = 1/b rounded -- the correctly rounded quotient (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990) at three operations instead of a division.
+// Quotients that are zero, infinite, NaN or within 2^100 of the ends of the
+// range (where the residual may not be exact) stay a rb.
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q = a * rb;
+    const unsigned e = (unsigned)__double2hiint(q) & 0x7ff00000u;
+    const double r = __fma_rn(__fma_rn(-q, b, a), rb, q);
+    return e - 0x06400000u < 0x73500000u ? r : q;   // exponents 100 .. 1944
+}
+
+// cos and sin of 2 pi m / R for the odd radices, and sqrt(1/2)
+#define MDX_COS3 -0.5
+#define MDX_SIN3 0.86602540378443864676
+#define MDX_COS5_1 0.30901699437494742410
+#define MDX_COS5_2 -0.80901699437494742410
+#define MDX_SIN5_1 0.95105651629515357212
+#define MDX_SIN5_2 0.58778525229247312917
+#define MDX_COS7_1 0.62348980185873353053
+#define MDX_COS7_2 -0.22252093395631440429
+#define MDX_COS7_3 -0.90096886790241912624
+#define MDX_SIN7_1 0.78183148246802980871
+#define MDX_SIN7_2 0.97492791218182360702
+#define MDX_SIN7_3 0.43388373911755812048
+#define MDX_SQRT1_2 0.70710678118654752440
+
+// Radix-R DFT of a[] in registers.  Odd R: with s_m = a_m + a_{R-m} and
+// d_m = a_m - a_{R-m}, X_p = a_0 + sum cos(2 pi p m / R) s_m
+// -+ i sum sin(2 pi p m / R) d_m.
+template <bool INV, int R, typename C2>
+__device__ __forceinline__ void dft_r(C2 (&a)[R]) {
+    typedef typename cx<C2>::R RT;
+    if constexpr (R == 2) {
         const C2 x0 = a[0], x1 = a[1];
         a[0] = cadd(x0, x1);
         a[1] = csub(x0, x1);
-    } else if (r == 4) {
-        const C2 x0 = a[0], x1 = a[1], x2 = a[2], x3 = a[3];
-        const C2 s02 = cadd(x0, x2), d02 = csub(x0, x2);
-        const C2 s13 = cadd(x1, x3), d13 = csub(x1, x3);
+    } else if constexpr (R == 4) {
+        const C2 s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]);
+        const C2 s13 = cadd(a[1], a[3]), d13 = csub(a[1], a[3]);
         const C2 rd13 = INV ? cmul_pi(d13) : cmul_mi(d13);
         a[0] = cadd(s02, s13);
         a[1] = cadd(d02, rd13);
         a[2] = csub(s02, s13);
         a[3] = csub(d02, rd13);
-    } else {
-        C2 b[7];
-        for (int p = 0; p < r; ++p) {
-            C2 acc = a[0];
-            for (int q = 1; q < r; ++q) acc = cadd(acc, cmul(a[q], twid<INV>(tw, ((p * q) % r) * root_step)));
-            b[p] = acc;
+    } else if constexpr (R == 8) {
+        C2 e[4] = {a[0], a[2], a[4], a[6]}, o[4] = {a[1], a[3], a[5], a[7]};
+        dft_r<INV, 4>(e);
+        dft_r<INV, 4>(o);
+        const RT h = (RT)MDX_SQRT1_2;
+        // W_8 o1, W_8^2 o2, W_8^3 o3
+        o[1] = INV ? cx<C2>::mk(h * (o[1].x - o[1].y), h * (o[1].x + o[1].y))
+                   : cx<C2>::mk(h * (o[1].x + o[1].y), h * (o[1].y - o[1].x));
+        o[2] = INV ? cmul_pi(o[2]) : cmul_mi(o[2]);
+        o[3] = INV ? cx<C2>::mk(-h * (o[3].x + o[3].y), h * (o[3].x - o[3].y))
+                   : cx<C2>::mk(h * (o[3].y - o[3].x), -h * (o[3].x + o[3].y));
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            a[m] = cadd(e[m], o[m]);
+            a[m + 4] = csub(e[m], o[m]);
         }
-        for (int p = 0; p < r; ++p) a[p] = b[p];
+    } else {
+        constexpr int H = R / 2;
+        const RT c[3] = {(RT)(R == 3 ? MDX_COS3 : R == 5 ? MDX_COS5_1 : MDX_COS7_1),
+                         (RT)(R == 5 ? MDX_COS5_2 : MDX_COS7_2), (RT)MDX_COS7_3};
+        const RT sn[3] = {(RT)(R == 3 ? MDX_SIN3 : R == 5 ? MDX_SIN5_1 : MDX_SIN7_1),
+                          (RT)(R == 5 ? MDX_SIN5_2 : MDX_SIN7_2), (RT)MDX_SIN7_3};
+        C2 s[H], d[H];
+        C2 x0 = a[0];
+#pragma unroll
+        for (int m = 1; m <= H; ++m) {
+            s[m - 1] = cadd(a[m], a[R - m]);
+            d[m - 1] = csub(a[m], a[R - m]);
+            x0 = cadd(x0, s[m - 1]);
+        }
+        const C2 a0 = a[0];
+        a[0] = x0;
+#pragma unroll
+        for (int p = 1; p <= H; ++p) {
+            C2 u = a0, v = cx<C2>::mk(0, 0);
+#pragma unroll
+            for (int m = 1; m <= H; ++m) {
+                const int t = (p * m) % R, i = t <= H ? t : R - t;   // cos even, sin odd about R/2
+                const RT cc = c[i - 1], ss = t <= H ? sn[i - 1] : -sn[i - 1];
+                u = cx<C2>::mk(fma_r(cc, s[m - 1].x, u.x), fma_r(cc, s[m - 1].y, u.y));
+                v = cx<C2>::mk(fma_r(ss, d[m - 1].x, v.x), fma_r(ss, d[m - 1].y, v.y));
+            }
+            const C2 iv = INV ? cmul_pi(v) : cmul_mi(v);
+            a[p] = cadd(u, iv);
+            a[R - p] = csub(u, iv);
+        }
+    }
+}
+
+// One Stockham stage of radix R over `total` = nlines n/R butterflies.
+template <bool INV, int R, typename C2>
+__device__ __forceinline__ void smem_stage(const C2* A, C2* B, int n, int nlines, int ls, int Ns, unsigned inv_nr,
+                                           unsigned inv_ns, const C2* __restrict__ tw, int tws) {
+    const int nr = n / R, total = nlines * nr;
+    const int tstep = (n / (Ns * R)) * tws;
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        const int line = nr > 1 ? (int)__umulhi((unsigned)t, inv_nr) : t;
+        const int jb = t - line * nr;
+        const int g = Ns > 1 ? (int)__umulhi((unsigned)jb, inv_ns) : jb;
+        const int k = jb - g * Ns;
+        const C2* src = A + line * ls + jb;
+        C2 a[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) a[q] = src[q * nr];
+        if (Ns > 1) {
+#pragma unroll
+            for (int q = 1; q < R; ++q) a[q] = cmul_f(a[q], twid<INV>(tw, q * k * tstep));
+        }
+        dft_r<INV, R>(a);
+        C2* dst = B + line * ls + g * Ns * R + k;
+#pragma unroll
+        for (int p = 0; p < R; ++p) dst[p * Ns] = a[p];
     }
 }
 
 // In-place (ping-pong) Stockham FFT of `nlines` lines of length n held in
 // shared memory at A[line*ls + t]; all threads of the block participate.
 // `tw` is a table of exp(-2 pi i t / N) with N = n * tws.  Returns the
-// buffer holding the result (A or B).
+// buffer holding the result (A or B).  Each radix is its own code (constants
+// instead of roots from the table, indices without division); with the radix
+// a run-time number the four transforms of a 200 x 200 x 200 projection took
+// 850 us.
 template <bool INV, typename C2>
 __device__ C2* smem_fft(C2* A, C2* B, int n, int nlines, int ls, const mdx_fft_plan& pl, const C2* __restrict__ tw,
                         int tws) {
     int Ns = 1;
     for (int s = 0; s < pl.nstages; ++s) {
         const int r = pl.radix[s];
-        const int nr = n / r;
-        const int total = nlines * nr;
-        const int tstep = (n / (Ns * r)) * tws;
-        const int root_step = nr * tws;
-        for (int t = threadIdx.x; t < total; t += blockDim.x) {
-            const int line = t / nr;
-            const int jb = t - line * nr;
-            const int k = jb % Ns;
-            const C2* src = A + line * ls;
-            C2 a[7];
-            for (int q = 0; q < r; ++q) a[q] = src[jb + q * nr];
-            if (Ns > 1)
-                for (int q = 1; q < r; ++q) a[q] = cmul(a[q], twid<INV>(tw, q * k * tstep));
-            dft_r<INV>(a, r, tw, root_step);
-            C2* dst = B + line * ls;
-            const int base = (jb / Ns) * Ns * r + k;
-            for (int p = 0; p < r; ++p) dst[base + p * Ns] = a[p];
+        const unsigned i1 = pl.inv_nr[s], i2 = pl.inv_ns[s];
+        switch (r) {
+            case 8: smem_stage<INV, 8>(A, B, n, nlines, ls, Ns, i1, i2, tw, tws); break;
+            case 4: smem_stage<INV, 4>(A, B, n, nlines, ls, Ns, i1, i2, tw, tws); break;
+            case 2: smem_stage<INV, 2>(A, B, n, nlines, ls, Ns, i1, i2, tw, tws); break;
+            case 3: smem_stage<INV, 3>(A, B, n, nlines, ls, Ns, i1, i2, tw, tws); break;
+            case 5: smem_stage<INV, 5>(A, B, n, nlines, ls, Ns, i1, i2, tw, tws); break;
+            default: smem_stage<INV, 7>(A, B, n, nlines, ls, Ns, i1, i2, tw, tws); break;
         }
         __syncthreads();
         C2* t = A; A = B; B = t;
@@ -169,34 +260,56 @@ __device__ C2* smem_fft(C2* A, C2* B, int n, int nlines, int ls, const mdx_fft_p
 // along x of each (k, j) row.  Rows are numbered r = (k-1) + nz*(j-1), the
 // order of plane_hat(nxh, nz, ny).  R rows per block, M = nx/2.
 // ---------------------------------------------------------------------------
+// 1/dx, 1/dy, 1/dz beside dx, dy, dz for div_by.
+struct fft_h { double dx, dy, dz, rdx, rdy, rdz; };
+static fft_h make_h(double dx, double dy, double dz) { return fft_h{dx, dy, dz, 1.0 / dx, 1.0 / dy, 1.0 / dz}; }
+
+// div(u*)/dt_gamma of the cell at padded index c.
+__device__ __forceinline__ double div_rhs(const fft_h& h, double dg, double rdg, const double* __restrict__ us,
+                                          const double* __restrict__ vs, const double* __restrict__ ws, long long c,
+                                          int nxp, long long plane) {
+    return div_by(div_by(__ldg(us + c + 1) - __ldg(us + c), h.dx, h.rdx) +
+                      div_by(__ldg(vs + c + nxp) - __ldg(vs + c), h.dy, h.rdy) +
+                      div_by(__ldg(ws + c + plane) - __ldg(ws + c), h.dz, h.rdz), dg, rdg);
+}
+
+// t / n for 0 <= t < 2^20, rn = 1.0f / n.
+__device__ __forceinline__ int quot(int t, float rn) { return (int)(((float)t + 0.5f) * rn); }
+#define MDX_FFT_ROWS 128   // at most this many x rows per block
+// Dynamic shared memory the Stockham kernels may ask for (two lines of 4096
+// FP64 values are 131 KB): the same cap for every plan, so that no context
+// lowers another's.
+#define MDX_FFT_SMEM (200 * 1024)
+
 template <typename C2>
 __global__ void __launch_bounds__(256)
-k_div_fftx(mdx_dims d, int R, double dx, double dy, double dz, mdx_dscal dgs, const double* __restrict__ us,
+k_div_fftx(mdx_dims d, int R, fft_h h, mdx_dscal dgs, const double* __restrict__ us,
            const double* __restrict__ vs, const double* __restrict__ ws, C2* __restrict__ spec,
            mdx_fft_plan pl, const C2* __restrict__ twx) {
-    const double dt_gamma = dgs.get();
+    const double dt_gamma = dgs.get(), rdg = 1.0 / dt_gamma;
     typedef typename cx<C2>::R RT;
     extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ long long rowc[MDX_FFT_ROWS];   // padded index of (0, j, k) of each row, -1 past the last
     C2* sm = reinterpret_cast<C2*>(sm_raw);
     const int M = d.nx / 2;
     C2* A = sm;
     C2* B = sm + R * M;
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
+    const long long plane = (long long)d.nxp * d.nyp;
+    const float rM = 1.0f / (float)M, rN = 1.0f / (float)(M + 1);
+    for (int t = threadIdx.x; t < R; t += blockDim.x) {
+        const int row = row0 + t;
+        rowc[t] = row < nrows ? pidx(d, 0, row / d.nz + 1, row % d.nz + 1) : -1;
+    }
+    __syncthreads();
     for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
-        const int rl = t / M, n = t - rl * M;
-        const int row = row0 + rl;
+        const int rl = quot(t, rM), n = t - rl * M;
         C2 z = cx<C2>::mk(0, 0);
-        if (row < nrows) {
-            const int k = row % d.nz + 1, j = row / d.nz + 1;
-            double x[2];
-            for (int e = 0; e < 2; ++e) {
-                const int i = 2 * n + 1 + e;
-                const long long c = pidx(d, i, j, k);
-                x[e] = ((__ldg(us + c + 1) - __ldg(us + c)) / dx + (__ldg(vs + c + d.nxp) - __ldg(vs + c)) / dy +
-                        (__ldg(ws + c + (long long)d.nxp * d.nyp) - __ldg(ws + c)) / dz) / dt_gamma;
-            }
-            z = cx<C2>::mk((RT)x[0], (RT)x[1]);
+        if (rowc[rl] >= 0) {
+            const long long c = rowc[rl] + 2 * n + 1;
+            z = cx<C2>::mk((RT)div_rhs(h, dt_gamma, rdg, us, vs, ws, c, d.nxp, plane),
+                           (RT)div_rhs(h, dt_gamma, rdg, us, vs, ws, c + 1, d.nxp, plane));
         }
         A[rl * M + n] = z;
     }
@@ -205,16 +318,15 @@ k_div_fftx(mdx_dims d, int R, double dx, double dy, double dz, mdx_dscal dgs, co
     // split step: X_k = E_k + W^k O_k, E = (Z_k + conj Z_{M-k})/2, O = -i/2 (Z_k - conj Z_{M-k})
     const int nxh = M + 1;
     for (int t = threadIdx.x; t < R * nxh; t += blockDim.x) {
-        const int rl = t / nxh, kx = t - rl * nxh;
+        const int rl = quot(t, rN), kx = t - rl * nxh;
         const int row = row0 + rl;
         if (row >= nrows) continue;
         const C2 zk = Z[rl * M + (kx == M ? 0 : kx)];
         const C2 zc = cconj(Z[rl * M + (kx == 0 ? 0 : M - kx)]);
-        const RT h = (RT)0.5;
-        const C2 e = cx<C2>::mk(h * (zk.x + zc.x), h * (zk.y + zc.y));
-        const C2 o = cmul_mi(cx<C2>::mk(h * (zk.x - zc.x), h * (zk.y - zc.y)));
-        const C2 X = cadd(e, cmul(__ldg(twx + kx), o));
-        spec[(long long)row * nxh + kx] = X;
+        const RT hf = (RT)0.5;
+        const C2 e = cx<C2>::mk(hf * (zk.x + zc.x), hf * (zk.y + zc.y));
+        const C2 o = cmul_mi(cx<C2>::mk(hf * (zk.x - zc.x), hf * (zk.y - zc.y)));
+        spec[(long long)row * nxh + kx] = cadd(e, cmul_f(__ldg(twx + kx), o));
     }
 }
 
@@ -223,25 +335,25 @@ k_div_fftx(mdx_dims d, int R, double dx, double dy, double dz, mdx_dscal dgs, co
 // ---------------------------------------------------------------------------
 template <bool INV, typename C2>
 __global__ void __launch_bounds__(256)
-k_fftz(mdx_dims d, int TX, C2* __restrict__ spec, mdx_fft_plan pl, const C2* __restrict__ twz) {
+k_fftz(mdx_dims d, int lgTX, C2* __restrict__ spec, mdx_fft_plan pl, const C2* __restrict__ twz) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     C2* sm = reinterpret_cast<C2*>(sm_raw);
-    const int nz = d.nz, nxh = d.nxh, ls = nz + 1;
+    const int TX = 1 << lgTX, nz = d.nz, nxh = d.nxh, ls = nz | 1;   // odd line stride: columns in distinct banks
     C2* A = sm;
     C2* B = sm + TX * ls;
-    const int ntiles = (nxh + TX - 1) / TX;
+    const int ntiles = (nxh + TX - 1) >> lgTX;
     const int j = blockIdx.x / ntiles;
-    const int kx0 = (blockIdx.x - j * ntiles) * TX;
+    const int kx0 = (blockIdx.x - j * ntiles) << lgTX;
     C2* base = spec + (long long)j * nz * nxh;
     for (int t = threadIdx.x; t < TX * nz; t += blockDim.x) {
-        const int c = t % TX, kz = t / TX;
+        const int c = t & (TX - 1), kz = t >> lgTX;
         const int kx = kx0 + c;
         A[c * ls + kz] = (kx < nxh) ? base[(long long)kz * nxh + kx] : cx<C2>::mk(0, 0);
     }
     __syncthreads();
     C2* Z = smem_fft<INV>(A, B, nz, TX, ls, pl, twz, 1);
     for (int t = threadIdx.x; t < TX * nz; t += blockDim.x) {
-        const int c = t % TX, kz = t / TX;
+        const int c = t & (TX - 1), kz = t >> lgTX;
         const int kx = kx0 + c;
         if (kx < nxh) base[(long long)kz * nxh + kx] = Z[c * ls + kz];
     }
@@ -383,9 +495,10 @@ k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec
     C2* B = sm + R * M;
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
+    const float rM = 1.0f / (float)M;
     // Z'_k = (X_k + conj X_{M-k}) + i W^{-k} (X_k - conj X_{M-k}),  k < M
     for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
-        const int rl = t / M, k = t - rl * M;
+        const int rl = quot(t, rM), k = t - rl * M;
         const int row = row0 + rl;
         C2 z = cx<C2>::mk(0, 0);
         if (row < nrows) {
@@ -394,7 +507,7 @@ k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec
             if (k == 0) { xk.y = 0; xm.y = 0; }   // kx = 0 and kx = M bins are real
             const C2 xc = cconj(xm);
             const C2 e = cadd(xk, xc);
-            const C2 o = cmul(csub(xk, xc), cconj(__ldg(twx + k)));
+            const C2 o = cmul_f(csub(xk, xc), cconj(__ldg(twx + k)));
             z = cadd(e, cmul_pi(o));
         }
         A[rl * M + k] = z;
@@ -402,7 +515,7 @@ k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec
     __syncthreads();
     C2* Z = smem_fft<true>(A, B, M, R, M, pl, twx, 2);
     for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
-        const int rl = t / M, n = t - rl * M;
+        const int rl = quot(t, rM), n = t - rl * M;
         const int row = row0 + rl;
         if (row >= nrows) continue;
         const C2 z = Z[rl * M + n];
@@ -541,10 +654,10 @@ template <typename C2> __device__ __forceinline__ void cp_async_elem(C2* dst, co
 // build_fft_rhs + forward real FFT along x, one warp per (k, j) row; M = nx/2 = 32 P.
 template <int P, typename C2>
 __global__ void __launch_bounds__(256, P >= 16 ? 2 : 4)
-k_div_fftx_w(mdx_dims d, double dx, double dy, double dz, mdx_dscal dgs, const double* __restrict__ us,
+k_div_fftx_w(mdx_dims d, fft_h g, mdx_dscal dgs, const double* __restrict__ us,
              const double* __restrict__ vs, const double* __restrict__ ws, C2* __restrict__ spec,
              const C2* __restrict__ twx) {
-    const double dt_gamma = dgs.get();
+    const double dt_gamma = dgs.get(), rdg = 1.0 / dt_gamma;
     typedef typename cx<C2>::R RT;
     constexpr int M = 32 * P;
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -561,9 +674,7 @@ k_div_fftx_w(mdx_dims d, double dx, double dy, double dz, mdx_dscal dgs, const d
         double x[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const long long c = pidx(d, 2 * n + 1 + e, j, k);
-            x[e] = ((__ldg(us + c + 1) - __ldg(us + c)) / dx + (__ldg(vs + c + d.nxp) - __ldg(vs + c)) / dy +
-                    (__ldg(ws + c + plane) - __ldg(ws + c)) / dz) / dt_gamma;
+            x[e] = div_rhs(g, dt_gamma, rdg, us, vs, ws, pidx(d, 2 * n + 1 + e, j, k), d.nxp, plane);
         }
         v[m] = cx<C2>::mk((RT)x[0], (RT)x[1]);
     }
@@ -678,39 +789,61 @@ k_ifftx_w(mdx_dims d, typename cx<C2>::R scale, const C2* __restrict__ spec, typ
 // ---------------------------------------------------------------------------
 // apply_fft_pressure_correction, pressure_solver.f90:150-169.
 // ---------------------------------------------------------------------------
+// A thread takes KC planes of its (i, j) column, all their loads before the
+// first store: with one plane per thread and three divisions per cell the
+// pass ran at 4.4 TB/s on 512x256x256.
+constexpr int KC = 4;
 template <bool IBM>
 __global__ void __launch_bounds__(256)
-k_correct(mdx_dims d, double dx, double dy, double dz, mdx_dscal dgs, const double* __restrict__ phi,
+k_correct(mdx_dims d, fft_h h, mdx_dscal dgs, const double* __restrict__ phi,
           const double* __restrict__ us, const double* __restrict__ vs, const double* __restrict__ ws,
           double* __restrict__ un, double* __restrict__ vn, double* __restrict__ wn, double* __restrict__ pn,
           const double* __restrict__ cu, const double* __restrict__ cv, const double* __restrict__ cw) {
     const double dt_gamma = dgs.get();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > d.nx || j > d.ny || k > d.nz) return;
-    int im = i - 1, km = k - 1;
-    if (im < 1) im = d.nx;
-    if (km < 1) km = d.nz;
-    const long long c = pidx(d, i, j, k);
-    const double r = __ldg(phi + ridx(d, i, k, j));
-    double u = (__ldg(us + c) - dt_gamma * (r - __ldg(phi + ridx(d, im, k, j))) / dx);
-    double w = (__ldg(ws + c) - dt_gamma * (r - __ldg(phi + ridx(d, i, km, j))) / dz);
-    if (IBM) {
-        u = u / (1.0 + dt_gamma * __ldg(cu + c));
-        w = w / (1.0 + dt_gamma * __ldg(cw + c));
-    } else {
-        u = u / 1.0;
-        w = w / 1.0;
-    }
-    un[c] = u;
-    wn[c] = w;
-    pn[c] = pn[c] + r;
-    if (j >= 2) {
-        double v = (__ldg(vs + c) - dt_gamma * (r - __ldg(phi + ridx(d, i, k, j - 1))) / dy);
-        if (IBM) v = v / (1.0 + dt_gamma * __ldg(cv + c));
-        vn[c] = v;
-    }
+    const int k0 = blockIdx.z * KC + 1;
+    if (i > d.nx || j > d.ny) return;
+    const int nk = min(KC, d.nz + 1 - k0);
+    const int im = i == 1 ? d.nx - 1 : -1;           // phi: the x neighbour's offset
+    const long long plane = (long long)d.nxp * d.nyp, jm = (long long)d.nx * d.nz;
+    const long long c0 = pidx(d, i, j, k0), r0 = ridx(d, i, k0, j);
+    double r[KC], ri[KC], rj[KC], u[KC], v[KC], w[KC], p[KC];
+    double rk = __ldg(phi + ridx(d, i, k0 == 1 ? d.nz : k0 - 1, j));
+#pragma unroll
+    for (int m = 0; m < KC; ++m)
+        if (m < nk) {
+            const long long c = c0 + m * plane, q = r0 + (long long)m * d.nx;
+            r[m] = __ldg(phi + q);
+            ri[m] = __ldg(phi + q + im);
+            u[m] = __ldg(us + c);
+            w[m] = __ldg(ws + c);
+            p[m] = pn[c];
+            if (j >= 2) {
+                rj[m] = __ldg(phi + q - jm);
+                v[m] = __ldg(vs + c);
+            }
+        }
+#pragma unroll
+    for (int m = 0; m < KC; ++m)
+        if (m < nk) {
+            const long long c = c0 + m * plane;
+            double a = u[m] - div_by(dt_gamma * (r[m] - ri[m]), h.dx, h.rdx);
+            double b = w[m] - div_by(dt_gamma * (r[m] - rk), h.dz, h.rdz);
+            if (IBM) {
+                a = a / (1.0 + dt_gamma * __ldg(cu + c));
+                b = b / (1.0 + dt_gamma * __ldg(cw + c));
+            }
+            un[c] = a;
+            wn[c] = b;
+            pn[c] = p[m] + r[m];
+            if (j >= 2) {
+                double e = v[m] - div_by(dt_gamma * (r[m] - rj[m]), h.dy, h.rdy);
+                if (IBM) e = e / (1.0 + dt_gamma * __ldg(cv + c));
+                vn[c] = e;
+            }
+            rk = r[m];
+        }
 }
 
 // Forward real FFT along x of each row of rhs(nx, nz, ny): rows r =
@@ -725,8 +858,9 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
     double2* B = sm + R * M;
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
+    const float rM = 1.0f / (float)M, rN = 1.0f / (float)(M + 1);
     for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
-        const int rl = t / M, n = t - rl * M;
+        const int rl = quot(t, rM), n = t - rl * M;
         const int row = row0 + rl;
         A[rl * M + n] = (row < nrows) ? make_double2(__ldg(rhs + (long long)row * d.nx + 2 * n),
                                                      __ldg(rhs + (long long)row * d.nx + 2 * n + 1))
@@ -736,14 +870,14 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
     double2* Z = smem_fft<false>(A, B, M, R, M, pl, twx, 2);
     const int nxh = M + 1;
     for (int t = threadIdx.x; t < R * nxh; t += blockDim.x) {
-        const int rl = t / nxh, kx = t - rl * nxh;
+        const int rl = quot(t, rN), kx = t - rl * nxh;
         const int row = row0 + rl;
         if (row >= nrows) continue;
         const double2 zk = Z[rl * M + (kx == M ? 0 : kx)];
         const double2 zc = cconj(Z[rl * M + (kx == 0 ? 0 : M - kx)]);
         const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
         const double2 o = cmul_mi(make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y)));
-        spec[(long long)row * nxh + kx] = cadd(e, cmul(__ldg(twx + kx), o));
+        spec[(long long)row * nxh + kx] = cadd(e, cmul_f(__ldg(twx + kx), o));
     }
 }
 
@@ -763,16 +897,15 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
 // rhs(i,k,j) = div(u*)/dt_gamma on the physical grid, the faces as the
 // boundary routine left them (build_fft_rhs's expression,
 // pressure_solver.f90:77-115).
-__global__ void k_div_rhs(mdx_dims d, double dx, double dy, double dz, mdx_dscal dgs, const double* __restrict__ us,
+__global__ void k_div_rhs(mdx_dims d, fft_h h, mdx_dscal dgs, const double* __restrict__ us,
                           const double* __restrict__ vs, const double* __restrict__ ws, double* __restrict__ rhs) {
     const double dt_gamma = dgs.get();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > d.nx || j > d.ny || k > d.nz) return;
-    const long long c = pidx(d, i, j, k);
-    rhs[ridx(d, i, k, j)] = ((__ldg(us + c + 1) - __ldg(us + c)) / dx + (__ldg(vs + c + d.nxp) - __ldg(vs + c)) / dy +
-                             (__ldg(ws + c + (long long)d.nxp * d.nyp) - __ldg(ws + c)) / dz) / dt_gamma;
+    rhs[ridx(d, i, k, j)] = div_rhs(h, dt_gamma, 1.0 / dt_gamma, us, vs, ws, pidx(d, i, j, k), d.nxp,
+                                    (long long)d.nxp * d.nyp);
 }
 
 // The extension: cell I of the solve grid is cell I (I <= n) or its mirror
@@ -846,13 +979,23 @@ k_correct_walls(mdx_dims d, double dx, double dy, double dz, mdx_dscal dgs, cons
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
-static int rows_per_block(int M) { return M >= 1024 ? 1 : 1024 / M; }
-static int ztile(int nz) {
-    int tx = 2048 / (nz + 1);
-    if (tx > 32) tx = 32;
-    if (tx < 1) tx = 1;
-    return tx;
+// x rows per block of the Stockham kernels: 2048 elements (two buffers of 32
+// KB, three blocks per SM), fewer where the grid would leave SMs idle.
+static int rows_per_block(int M, long long nrows) {
+    const long long fill = std::max<long long>(1, nrows / (2 * 148));
+    return (int)std::max<long long>(1, std::min<long long>({2048 / M, fill, MDX_FFT_ROWS}));
 }
+// log2 of the kx columns per block of the Stockham z transform: a 128-byte row
+// segment per kz, more for short lines (2048 elements), fewer for long ones
+// that two buffers must hold and where the grid would leave SMs idle.
+static int lg_ztile(int nz, int nxh, int ny) {
+    int lg = 5;
+    while (lg > 0 && (((nz | 1) << lg) > 4096 || (lg > 3 && ((nz << lg) > 2048)) ||
+                      (lg > 1 && (long long)((nxh + (1 << lg) - 1) >> lg) * ny < 2 * 148)))
+        --lg;
+    return lg;
+}
+static size_t ztile_bytes(int nz, int lg, size_t elem) { return elem * 2 * ((size_t)(nz | 1) << lg); }
 
 // Warp-shuffle transform lengths: 32 P with P = 1, 2, 4, 8, 16 (0: none).
 static int warp_p(int n) {
@@ -906,14 +1049,14 @@ static int launch_div_fftx(mdx_ctx_t* ctx, const char* what, mdx_dscal dg, C2* s
         return with_p(px, [&](auto pc) -> int {
             constexpr int P = decltype(pc)::value;
             auto kern = k_div_fftx_w<P, C2>;
-            MDX_LAUNCH(ctx, MDX_T_FFT_FWD, what, kern, (nrows + 7) / 8, 256, 8 * 32 * P * sizeof(C2), d, g.dx, g.dy,
-                       g.dz, dg, f[MDX_US], f[MDX_VS], f[MDX_WS], spec, twx);
+            MDX_LAUNCH(ctx, MDX_T_FFT_FWD, what, kern, (nrows + 7) / 8, 256, 8 * 32 * P * sizeof(C2), d,
+                       make_h(g.dx, g.dy, g.dz), dg, f[MDX_US], f[MDX_VS], f[MDX_WS], spec, twx);
             return MDX_OK;
         });
-    const int M = d.nx / 2, R = rows_per_block(M);
+    const int M = d.nx / 2, R = rows_per_block(M, nrows);
     auto kern = k_div_fftx<C2>;
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, what, kern, (nrows + R - 1) / R, 256, sizeof(C2) * 2 * R * M, d, R, g.dx, g.dy,
-               g.dz, dg, f[MDX_US], f[MDX_VS], f[MDX_WS], spec, ctx->plan_xh, twx);
+    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, what, kern, (nrows + R - 1) / R, 256, sizeof(C2) * 2 * R * M, d, R,
+               make_h(g.dx, g.dy, g.dz), dg, f[MDX_US], f[MDX_VS], f[MDX_WS], spec, ctx->plan_xh, twx);
     return MDX_OK;
 }
 
@@ -929,10 +1072,10 @@ static int launch_fftz(mdx_ctx_t* ctx, const char* what, C2* spec, const C2* twz
             MDX_LAUNCH(ctx, cls, what, kern, ((d.nxh + TX - 1) / TX) * d.ny, 32 * TX, 32 * P * 128, d, spec, twz);
             return MDX_OK;
         });
-    const int TX = ztile(d.nz);
+    const int lg = lg_ztile(d.nz, d.nxh, d.ny);
     auto kern = k_fftz<INV, C2>;
-    MDX_LAUNCH(ctx, cls, what, kern, ((d.nxh + TX - 1) / TX) * d.ny, 256, sizeof(C2) * 2 * TX * (d.nz + 1), d, TX,
-               spec, ctx->plan_z, twz);
+    MDX_LAUNCH(ctx, cls, what, kern, ((d.nxh + (1 << lg) - 1) >> lg) * d.ny, 256, ztile_bytes(d.nz, lg, sizeof(C2)), d,
+               lg, spec, ctx->plan_z, twz);
     return MDX_OK;
 }
 
@@ -949,7 +1092,7 @@ static int launch_ifftx(mdx_ctx_t* ctx, const char* what, typename cx<C2>::R sca
                        phi, twx);
             return MDX_OK;
         });
-    const int M = d.nx / 2, R = rows_per_block(M);
+    const int M = d.nx / 2, R = rows_per_block(M, nrows);
     auto kern = k_ifftx<C2>;
     MDX_LAUNCH(ctx, MDX_T_FFT_INV, what, kern, (nrows + R - 1) / R, 256, sizeof(C2) * 2 * R * M, d, R, scale, spec,
                phi, ctx->plan_xh, twx);
@@ -1053,14 +1196,11 @@ int mdx_fft_init(mdx_ctx_t* ctx) {
     cudaFree(dkz);
     if (rc != MDX_OK) return rc;
 
-    const int M = D.nx / 2;
-    const size_t smx = sizeof(double2) * 2 * rows_per_block(M) * M;
-    const size_t smz = sizeof(double2) * 2 * ztile(D.nz) * (D.nz + 1);
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_div_fftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftx_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_ifftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_div_fftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftx_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_ifftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
     if (!ctx->fft_ext_x && !ctx->fft_ext_z) MDX_TRY(fft_warp_attrs<double2>(ctx));
     return MDX_OK;
 }
@@ -1093,23 +1233,23 @@ static int projection_fft_walls(mdx_ctx_t* ctx, mdx_dscal dg) {
     double** f = ctx->f;
     dim3 block(32, 4, 2);
     dim3 grid((d.nx + 31) / 32, (d.ny + 3) / 4, (d.nz + 1) / 2);
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "div rhs", k_div_rhs, grid, block, 0, d, g.dx, g.dy, g.dz, dg, f[MDX_US], f[MDX_VS],
+    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "div rhs", k_div_rhs, grid, block, 0, d, make_h(g.dx, g.dy, g.dz), dg, f[MDX_US], f[MDX_VS],
                f[MDX_WS], f[MDX_PHI]);
     const int nb = (int)std::min<long long>((e.nint + 255) / 256, 8192);
     MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "extend rhs", k_extend, nb, 256, 0, d, e, f[MDX_PHI], ctx->phi_ext);
-    const int M = e.nx / 2, R = rows_per_block(M), nrows = e.nz * e.ny;
+    const int M = e.nx / 2, nrows = e.nz * e.ny, R = rows_per_block(M, nrows);
     const size_t smx = sizeof(double2) * 2 * R * M;
     MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "fft x (extended)", k_fftx_r2c, (nrows + R - 1) / R, 256, smx, e, R, ctx->phi_ext,
                ctx->spec, ctx->plan_xh, ctx->tw_x);
-    const int TX = ztile(e.nz);
-    const size_t smz = sizeof(double2) * 2 * TX * (e.nz + 1);
-    const int zblocks = ((e.nxh + TX - 1) / TX) * e.ny;
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "fft z (extended)", (k_fftz<false, double2>), zblocks, 256, smz, e, TX, ctx->spec,
+    const int lg = lg_ztile(e.nz, e.nxh, e.ny);
+    const size_t smz = ztile_bytes(e.nz, lg, sizeof(double2));
+    const int zblocks = ((e.nxh + (1 << lg) - 1) >> lg) * e.ny;
+    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "fft z (extended)", (k_fftz<false, double2>), zblocks, 256, smz, e, lg, ctx->spec,
                ctx->plan_z, ctx->tw_z);
     const int nm = e.nxh * e.nz;
     MDX_LAUNCH(ctx, MDX_T_THOMAS, "thomas (extended)", (k_thomas<double2, false>), (nm + 127) / 128, 128, 0, e,
                1.0 / (g.dy * g.dy), ctx->spec, ctx->thomas_dinv, ctx->thomas_cp);
-    MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft z (extended)", (k_fftz<true, double2>), zblocks, 256, smz, e, TX, ctx->spec,
+    MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft z (extended)", (k_fftz<true, double2>), zblocks, 256, smz, e, lg, ctx->spec,
                ctx->plan_z, ctx->tw_z);
     MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft x (extended)", k_ifftx<double2>, (nrows + R - 1) / R, 256, smx, e, R,
                1.0 / (double)((long long)e.nx * e.nz), ctx->spec, ctx->phi_ext, ctx->plan_xh, ctx->tw_x);
@@ -1160,16 +1300,12 @@ int mdx_k_projection_fft(mdx_ctx_t* ctx, mdx_dscal dg) {
     MDX_TRY((launch_fftz<true, double2>(ctx, "ifft z", ctx->spec, ctx->tw_z)));
     const double scale = 1.0 / (double)(d.nx * d.nz);
     MDX_TRY(launch_ifftx<double2>(ctx, "ifft x", scale, ctx->spec, f[MDX_PHI], ctx->tw_x));
-    dim3 block(32, 4, 2);
-    dim3 grid((d.nx + 31) / 32, (d.ny + 3) / 4, (d.nz + 1) / 2);
-    if (ctx->ibm_zero)
-        MDX_LAUNCH(ctx, MDX_T_CORRECT, "correction", k_correct<false>, grid, block, 0, d, g.dx, g.dy, g.dz, dg,
-                   f[MDX_PHI], f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN],
-                   f[MDX_COEF_U], f[MDX_COEF_V], f[MDX_COEF_W]);
-    else
-        MDX_LAUNCH(ctx, MDX_T_CORRECT, "correction", k_correct<true>, grid, block, 0, d, g.dx, g.dy, g.dz, dg,
-                   f[MDX_PHI], f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN],
-                   f[MDX_COEF_U], f[MDX_COEF_V], f[MDX_COEF_W]);
+    dim3 block(32, 8);
+    dim3 grid((d.nx + 31) / 32, (d.ny + 7) / 8, (d.nz + KC - 1) / KC);
+    auto kcor = ctx->ibm_zero ? k_correct<false> : k_correct<true>;
+    MDX_LAUNCH(ctx, MDX_T_CORRECT, "correction", kcor, grid, block, 0, d, make_h(g.dx, g.dy, g.dz), dg, f[MDX_PHI],
+               f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN], f[MDX_COEF_U],
+               f[MDX_COEF_V], f[MDX_COEF_W]);
     return MDX_OK;
 }
 
@@ -1295,13 +1431,10 @@ static int fft_mixed_alloc(mdx_ctx_t* ctx) {
     const int nb = (int)std::min<long long>((tsize + 255) / 256, 4096);
     MDX_LAUNCH(ctx, MDX_T_OTHER, "thomas tables fp32", k_to_float, nb, 256, 0, tsize, ctx->thomas_dinv, ctx->dinv32);
     MDX_LAUNCH(ctx, MDX_T_OTHER, "thomas tables fp32", k_to_float, nb, 256, 0, tsize, ctx->thomas_cp, ctx->cp32);
-    const int M = d.nx / 2;
-    const size_t smx = sizeof(float2) * 2 * rows_per_block(M) * M;
-    const size_t smz = sizeof(float2) * 2 * ztile(d.nz) * (d.nz + 1);
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_div_fftx<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_ifftx<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<false, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<true, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_div_fftx<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_ifftx<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<false, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<true, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
     MDX_TRY(fft_warp_attrs<float2>(ctx));
     return MDX_OK;
 }
@@ -1509,25 +1642,25 @@ extern "C" int mdx_solve_pressure_fft_noalloc(const double* rhs, double* phi, in
     const int nm = d.nxh * nzh;
     k_thomas_tables<<<(nm + 127) / 128, 128, 0, st>>>(d.nxh, nzh, ny, dyi2, kxp, kzp, dinv, cp);
     const int M = nx / 2;
-    const int R = rows_per_block(M);
     const int nrows = nz * ny;
+    const int R = rows_per_block(M, nrows);
     const size_t smx = sizeof(double2) * 2 * R * M;
     const int xblocks = (nrows + R - 1) / R;
-    const int TX = ztile(nz);
-    const size_t smz = sizeof(double2) * 2 * TX * (nz + 1);
-    const int zblocks = ((d.nxh + TX - 1) / TX) * ny;
-    const cudaError_t a1 = cudaFuncSetAttribute(k_fftx_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
-    const cudaError_t a2 = cudaFuncSetAttribute(k_ifftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
+    const int lg = lg_ztile(nz, d.nxh, ny);
+    const size_t smz = ztile_bytes(nz, lg, sizeof(double2));
+    const int zblocks = ((d.nxh + (1 << lg) - 1) >> lg) * ny;
+    const cudaError_t a1 = cudaFuncSetAttribute(k_fftx_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
+    const cudaError_t a2 = cudaFuncSetAttribute(k_ifftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
     const cudaError_t a3 =
-        cudaFuncSetAttribute(k_fftz<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+        cudaFuncSetAttribute(k_fftz<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
     const cudaError_t a4 =
-        cudaFuncSetAttribute(k_fftz<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+        cudaFuncSetAttribute(k_fftz<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
     if (a1 != cudaSuccess || a2 != cudaSuccess || a3 != cudaSuccess || a4 != cudaSuccess)
         return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: cudaFuncSetAttribute failed");
     k_fftx_r2c<<<xblocks, 256, smx, st>>>(d, R, rhs, spec, plx, twx);
-    k_fftz<false, double2><<<zblocks, 256, smz, st>>>(d, TX, spec, plz, twz);
+    k_fftz<false, double2><<<zblocks, 256, smz, st>>>(d, lg, spec, plz, twz);
     k_thomas<double2, false><<<(d.nxh * nz + 127) / 128, 128, 0, st>>>(d, dyi2, spec, dinv, cp);
-    k_fftz<true, double2><<<zblocks, 256, smz, st>>>(d, TX, spec, plz, twz);
+    k_fftz<true, double2><<<zblocks, 256, smz, st>>>(d, lg, spec, plz, twz);
     k_ifftx<double2><<<xblocks, 256, smx, st>>>(d, R, 1.0 / (double)(nx * nz), spec, phi, plx, twx);
     e = cudaGetLastError();
     if (e != cudaSuccess) return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: launch: %s", cudaGetErrorString(e));
