@@ -100,7 +100,7 @@ template <typename C2> __device__ __forceinline__ C2 cmul_f(C2 a, C2 b) {
 // Twiddle exp(-+2 pi i t / n) from the forward table (conjugated for INV).
 template <bool INV, typename C2>
 __device__ __forceinline__ C2 twid(const C2* __restrict__ tw, int t) {
-    C2 w = __ldg(tw + t);
+    C2 w = tw[t];   // global or shared
     if (INV) w.y = -w.y;
     return w;
 }
@@ -273,6 +273,15 @@ __device__ __forceinline__ double div_rhs(const fft_h& h, double dg, double rdg,
                       div_by(__ldg(ws + c + plane) - __ldg(ws + c), h.dz, h.rdz), dg, rdg);
 }
 
+// exp(-2 pi i t / n), t < n, by the block's threads.
+__device__ __forceinline__ void own_twiddles(double2* T, int n) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        double sn, cs;
+        sincospi(2.0 * (double)t / (double)n, &sn, &cs);
+        T[t] = make_double2(cs, -sn);
+    }
+}
+
 // t / n for 0 <= t < 2^20, rn = 1.0f / n.
 __device__ __forceinline__ int quot(int t, float rn) { return (int)(((float)t + 0.5f) * rn); }
 #define MDX_FFT_ROWS 128   // at most this many x rows per block
@@ -364,11 +373,30 @@ k_fftz(mdx_dims d, int lgTX, C2* __restrict__ spec, mdx_fft_plan pl, const C2* _
 // (kx, kz <= nz/2) the reciprocal pivots dinv_j and c'_j.  kz and nz-kz have
 // bitwise-equal modified wavenumbers (sin is odd), so one table serves both.
 // ---------------------------------------------------------------------------
+// The reciprocal pivots of one mode, `stride` apart (c'_j is dyi2 times them).
+__device__ __forceinline__ void thomas_pivots(int ny, double dyi2, double k_tot, bool zero, double* dinv, int stride) {
+    double cprev = 0.0;
+    for (int j = 1; j <= ny; ++j) {
+        double di = 1.0;
+        if (j > 1 || !zero) {
+            const double b = (j == 1 || j == ny ? -dyi2 : -2.0 * dyi2) - k_tot;
+            di = 1.0 / (j == 1 ? b : b - dyi2 * cprev);
+            cprev = dyi2 * di;
+        }
+        dinv[(long long)(j - 1) * stride] = di;
+    }
+}
+
+// cp null: dinv alone, in the order [kx][j][kz] that k_zty reads.
 __global__ void k_thomas_tables(int nxh, int nzh, int ny, double dyi2, const double* __restrict__ kxp,
                                 const double* __restrict__ kzp, double* __restrict__ dinv, double* __restrict__ cp) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nxh * nzh) return;
     const int kx = m % nxh, kz = m / nxh;
+    if (!cp) {
+        thomas_pivots(ny, dyi2, kxp[kx] + kzp[kz], kx == 0 && kz == 0, dinv + (long long)kx * ny * nzh + kz, nzh);
+        return;
+    }
     const long long plane = (long long)nxh * nzh;
     const double k_tot = kxp[kx] + kzp[kz];
     double cprev;
@@ -479,20 +507,143 @@ k_thomas(mdx_dims d, typename cx<C2>::R dyi2, C2* __restrict__ spec, const typen
 }
 
 // ---------------------------------------------------------------------------
+// The whole middle of the solve for small grids: forward z transforms, the
+// tridiagonal solves in y and the inverse z transforms of one kx, the (z, y)
+// plane of the spectrum in shared memory (two buffers).  One block per kx.
+// As three kernels it took 4 + 19 + 4 us on 64x32x32 (29 + 32 + 28 on the
+// 96x64x96 plane set of a duct): the solve's serial chain ran from global
+// memory on a tenth of the SMs.  Here its operands are in shared memory and a
+// step of the chain is one fused multiply-add, the products with the
+// reciprocal pivots being formed beside it.
+//
+// OWN: twiddles, wavenumbers and pivots are made by the block (a caller
+// without tables); else they are read.  Shared memory: two buffers of ny
+// lines of nz | 1, the pivots [ny][nz/2 + 1], OWN: nz twiddles.
+// ---------------------------------------------------------------------------
+static size_t zty_bytes(int ny, int nz, bool own) {
+    return sizeof(double2) * 2 * (size_t)ny * (nz | 1) + sizeof(double) * (size_t)ny * (nz / 2 + 1) +
+           (own ? sizeof(double2) * (size_t)nz : 0) + 16;
+}
+#define MDX_ZTY_SMEM (224 * 1024)
+static int zty_threads(int ny, int nz) { return ny * nz >= 512 ? 512 : 256; }
+static bool zty_ok(int ny, int nz, bool own) { return zty_bytes(ny, nz, own) <= MDX_ZTY_SMEM; }
+
+// 4/h^2 sin^2(pi k/n) (pressure_fft.f90:53,61)
+__device__ __forceinline__ double wave2(int k, int n, double h) {
+    const double q = sinpi((double)k / (double)n);
+    return (4.0 / (h * h)) * (q * q);
+}
+
+template <bool OWN>
+__global__ void __launch_bounds__(512)
+k_zty(mdx_dims d, double dyi2, double dx, double dz, double2* __restrict__ spec, mdx_fft_plan pl,
+      const double2* __restrict__ twz, const double* __restrict__ dinv) {
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    const int nz = d.nz, ny = d.ny, nxh = d.nxh, nzh = nz / 2 + 1, ls = nz | 1, kx = blockIdx.x;
+    double2* A = reinterpret_cast<double2*>(sm_raw);
+    double2* B = A + ny * ls;
+    double2* T = B + ny * ls;
+    double* D = reinterpret_cast<double*>(T + (OWN ? nz : 0));   // [ny][nzh]
+    const int T0 = OWN ? (nzh + 31) & ~31 : 0;   // the first warps make the pivots, the others load
+    const bool few = T0 >= (int)blockDim.x;
+    const float rz = 1.0f / (float)nz;
+    if (OWN && (int)threadIdx.x < T0)
+        for (int kz = threadIdx.x; kz < nzh; kz += blockDim.x)
+            thomas_pivots(ny, dyi2, wave2(kx, d.nx, dx) + wave2(kz, nz, dz), kx == 0 && kz == 0, D + kz, nzh);
+    if ((int)threadIdx.x >= T0 || few) {
+        const int step = few ? blockDim.x : blockDim.x - T0, t0 = few ? threadIdx.x : threadIdx.x - T0;
+#pragma unroll 4
+        for (int t = t0; t < ny * nz; t += step) {
+            const int j = quot(t, rz), kz = t - j * nz;
+            A[j * ls + kz] = __ldcg(spec + (long long)t * nxh + kx);
+        }
+        if (OWN) {
+            for (int t = t0; t < nz; t += step) {
+                double sn, cs;
+                sincospi(2.0 * (double)t / (double)nz, &sn, &cs);
+                T[t] = make_double2(cs, -sn);
+            }
+        } else {
+            const double* src = dinv + (long long)kx * ny * nzh;
+            for (int t = t0; t < ny * nzh; t += step) D[t] = __ldg(src + t);
+        }
+    }
+    __syncthreads();
+    const double2* tw = OWN ? T : twz;
+    double2* Z = smem_fft<false>(A, B, nz, ny, ls, pl, tw, 1);
+    for (int kz = threadIdx.x; kz < nz; kz += blockDim.x) {
+        double2* col = Z + kz;
+        const double* di = D + (kz <= nz / 2 ? kz : nz - kz);
+        double2 dp = col[0];
+        dp = kx == 0 && kz == 0 ? make_double2(0.0, 0.0) : make_double2(dp.x * di[0], dp.y * di[0]);
+        col[0] = dp;
+        // the operands of TU steps are read before the first of them
+        constexpr int TU = 8;
+        const bool zero = kx == 0 && kz == 0;
+        for (int j0 = 1; j0 < ny; j0 += TU) {   // dp = (r - a dp) di
+            double2 r[TU];
+            double q[TU];
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                if (j0 + u < ny) {
+                    r[u] = col[(j0 + u) * ls];
+                    q[u] = di[(j0 + u) * nzh];
+                }
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                if (j0 + u < ny) {
+                    const double a = -(dyi2 * q[u]);
+                    dp = make_double2(__fma_rn(a, dp.x, r[u].x * q[u]), __fma_rn(a, dp.y, r[u].y * q[u]));
+                    col[(j0 + u) * ls] = dp;
+                }
+        }
+        for (int j0 = ny - 2; j0 >= 0; j0 -= TU) {   // x = dp - c' x; c'_1 of the pinned row is 0
+            double2 r[TU];
+            double c[TU];
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                if (j0 - u >= 0) {
+                    r[u] = col[(j0 - u) * ls];
+                    c[u] = zero && j0 == u ? 0.0 : -(dyi2 * di[(j0 - u) * nzh]);
+                }
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                if (j0 - u >= 0) {
+                    dp = make_double2(__fma_rn(c[u], dp.x, r[u].x), __fma_rn(c[u], dp.y, r[u].y));
+                    col[(j0 - u) * ls] = dp;
+                }
+        }
+    }
+    __syncthreads();
+    Z = smem_fft<true>(Z, Z == A ? B : A, nz, ny, ls, pl, tw, 1);
+    for (int t = threadIdx.x; t < ny * nz; t += blockDim.x) {
+        const int j = quot(t, rz), kz = t - j * nz;
+        spec[(long long)t * nxh + kx] = Z[j * ls + kz];
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Inverse real FFT along x of each row (c2r contract: imaginary parts of the
 // kx = 0 and kx = nx/2 bins are ignored), scaled by 1/(nx*nz) as
 // scale_pressure_correction_* (pressure_backend_fftw.f90:80-93).
 // ---------------------------------------------------------------------------
-template <typename C2>
+// OWN: the block makes the twiddles, behind its two buffers.
+template <typename C2, bool OWN = false>
 __global__ void __launch_bounds__(256)
 k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec, typename cx<C2>::R* __restrict__ phi,
-        mdx_fft_plan pl, const C2* __restrict__ twx) {
+        mdx_fft_plan pl, const C2* __restrict__ tw_g) {
     typedef typename cx<C2>::R RT;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     C2* sm = reinterpret_cast<C2*>(sm_raw);
     const int M = d.nx / 2, nxh = M + 1;
     C2* A = sm;
     C2* B = sm + R * M;
+    const C2* twx = tw_g;
+    if constexpr (OWN) {
+        own_twiddles(B + R * M, d.nx);
+        twx = B + R * M;
+        __syncthreads();
+    }
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
     const float rM = 1.0f / (float)M;
@@ -507,7 +658,7 @@ k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec
             if (k == 0) { xk.y = 0; xm.y = 0; }   // kx = 0 and kx = M bins are real
             const C2 xc = cconj(xm);
             const C2 e = cadd(xk, xc);
-            const C2 o = cmul_f(csub(xk, xc), cconj(__ldg(twx + k)));
+            const C2 o = cmul_f(csub(xk, xc), cconj(twx[k]));
             z = cadd(e, cmul_pi(o));
         }
         A[rl * M + k] = z;
@@ -848,14 +999,20 @@ k_correct(mdx_dims d, fft_h h, mdx_dscal dgs, const double* __restrict__ phi,
 
 // Forward real FFT along x of each row of rhs(nx, nz, ny): rows r =
 // (k-1) + nz*(j-1) of nx reals -> nx/2+1 complex in plane_hat order.
+template <bool OWN>
 __global__ void __launch_bounds__(256)
 k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restrict__ spec, mdx_fft_plan pl,
-           const double2* __restrict__ twx) {
+           const double2* __restrict__ tw_g) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     double2* sm = reinterpret_cast<double2*>(sm_raw);
     const int M = d.nx / 2;
     double2* A = sm;
     double2* B = sm + R * M;
+    const double2* twx = tw_g;
+    if (OWN) {   // the block makes the twiddles, behind its two buffers
+        own_twiddles(B + R * M, d.nx);
+        twx = B + R * M;
+    }
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
     const float rM = 1.0f / (float)M, rN = 1.0f / (float)(M + 1);
@@ -877,7 +1034,7 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
         const double2 zc = cconj(Z[rl * M + (kx == 0 ? 0 : M - kx)]);
         const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
         const double2 o = cmul_mi(make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y)));
-        spec[(long long)row * nxh + kx] = cadd(e, cmul_f(__ldg(twx + kx), o));
+        spec[(long long)row * nxh + kx] = cadd(e, cmul_f(twx[kx], o));
     }
 }
 
@@ -894,86 +1051,143 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
 // the extended grid dfft; the correction then leaves the wall faces alone.
 // ---------------------------------------------------------------------------
 
-// rhs(i,k,j) = div(u*)/dt_gamma on the physical grid, the faces as the
-// boundary routine left them (build_fft_rhs's expression,
-// pressure_solver.f90:77-115).
-__global__ void k_div_rhs(mdx_dims d, fft_h h, mdx_dscal dgs, const double* __restrict__ us,
-                          const double* __restrict__ vs, const double* __restrict__ ws, double* __restrict__ rhs) {
-    const double dt_gamma = dgs.get();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > d.nx || j > d.ny || k > d.nz) return;
-    rhs[ridx(d, i, k, j)] = div_rhs(h, dt_gamma, 1.0 / dt_gamma, us, vs, ws, pidx(d, i, j, k), d.nxp,
-                                    (long long)d.nxp * d.nyp);
-}
-
-// The extension: cell I of the solve grid is cell I (I <= n) or its mirror
-// 2n + 1 - I of the physical grid in a direction with walls.
-__global__ void k_extend(mdx_dims d, mdx_dims e, const double* __restrict__ rhs, double* __restrict__ ext) {
-    const long long n = (long long)e.nx * e.nz * e.ny;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int I = (int)(t % e.nx) + 1;
-        const long long r = t / e.nx;
-        const int K = (int)(r % e.nz) + 1;
-        const int j = (int)(r / e.nz) + 1;
-        const int i = I <= d.nx ? I : 2 * d.nx + 1 - I;
-        const int k = K <= d.nz ? K : 2 * d.nz + 1 - K;
-        ext[t] = __ldg(rhs + ridx(d, i, k, j));
+// Divergence of the physical cells (the faces as the boundary routine left
+// them) and the forward transform of their rows on the solve grid e: in x the
+// mirrored cell 2n + 1 - I stands for cells I > nx; in z the rows k of the
+// physical grid are transformed and written to the mirrored row as well, its
+// values being the same.  One pass for what the divergence, the extension and
+// the transform of the extended rows took in three.
+__global__ void __launch_bounds__(256)
+k_div_fftx_walls(mdx_dims d, mdx_dims e, int R, fft_h h, mdx_dscal dgs, const double* __restrict__ us,
+                 const double* __restrict__ vs, const double* __restrict__ ws, double2* __restrict__ spec,
+                 mdx_fft_plan pl, const double2* __restrict__ twx) {
+    const double dt_gamma = dgs.get(), rdg = 1.0 / dt_gamma;
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ long long rowc[MDX_FFT_ROWS];
+    double2* sm = reinterpret_cast<double2*>(sm_raw);
+    const int M = e.nx / 2, nxh = M + 1;
+    double2* A = sm;
+    double2* B = sm + R * M;
+    const int nrows = d.nz * d.ny;
+    const int row0 = blockIdx.x * R;
+    const long long plane = (long long)d.nxp * d.nyp;
+    const float rM = 1.0f / (float)M, rN = 1.0f / (float)nxh;
+    for (int t = threadIdx.x; t < R; t += blockDim.x) {
+        const int row = row0 + t;
+        rowc[t] = row < nrows ? pidx(d, 0, row / d.nz + 1, row % d.nz + 1) : -1;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
+        const int rl = quot(t, rM), n = t - rl * M;
+        double2 z = make_double2(0.0, 0.0);
+        if (rowc[rl] >= 0) {
+            const int I = 2 * n + 1;
+            const int i0 = I <= d.nx ? I : 2 * d.nx + 1 - I, i1 = I + 1 <= d.nx ? I + 1 : 2 * d.nx - I;
+            z = make_double2(div_rhs(h, dt_gamma, rdg, us, vs, ws, rowc[rl] + i0, d.nxp, plane),
+                             div_rhs(h, dt_gamma, rdg, us, vs, ws, rowc[rl] + i1, d.nxp, plane));
+        }
+        A[rl * M + n] = z;
+    }
+    __syncthreads();
+    double2* Z = smem_fft<false>(A, B, M, R, M, pl, twx, 2);
+    for (int t = threadIdx.x; t < R * nxh; t += blockDim.x) {
+        const int rl = quot(t, rN), kx = t - rl * nxh;
+        const int row = row0 + rl;
+        if (row >= nrows) continue;
+        const double2 zk = Z[rl * M + (kx == M ? 0 : kx)];
+        const double2 zc = cconj(Z[rl * M + (kx == 0 ? 0 : M - kx)]);
+        const double2 ev = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
+        const double2 od = cmul_mi(make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y)));
+        const double2 X = cadd(ev, cmul_f(__ldg(twx + kx), od));
+        const int j = row / d.nz, k = row - j * d.nz;
+        spec[((long long)j * e.nz + k) * nxh + kx] = X;
+        if (e.nz > d.nz) spec[((long long)j * e.nz + e.nz - 1 - k) * nxh + kx] = X;
     }
 }
 
-// phi of the physical cells: the first nx x nz block of each plane.
-__global__ void k_restrict(mdx_dims d, mdx_dims e, const double* __restrict__ ext, double* __restrict__ phi) {
-    const long long n = d.nint;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % d.nx) + 1;
-        const long long r = t / d.nx;
-        const int k = (int)(r % d.nz) + 1;
-        const int j = (int)(r / d.nz) + 1;
-        phi[t] = __ldg(ext + ridx(e, i, k, j));
+// The inverse transform of the rows of the physical planes and their first nx
+// values: phi(i, k, j).
+__global__ void __launch_bounds__(256)
+k_ifftx_walls(mdx_dims d, mdx_dims e, int R, double scale, const double2* __restrict__ spec, double* __restrict__ phi,
+              mdx_fft_plan pl, const double2* __restrict__ twx) {
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ long long rows[MDX_FFT_ROWS];   // the row's place in the spectrum, -1 past the last
+    const int M = e.nx / 2, nxh = M + 1;
+    double2* A = reinterpret_cast<double2*>(sm_raw);
+    double2* B = A + R * M;
+    const int nrows = d.nz * d.ny, row0 = blockIdx.x * R;
+    const float rM = 1.0f / (float)M;
+    for (int t = threadIdx.x; t < R; t += blockDim.x) {
+        const int row = row0 + t;
+        rows[t] = row < nrows ? ((long long)(row / d.nz) * e.nz + row % d.nz) * nxh : -1;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
+        const int rl = quot(t, rM), k = t - rl * M;
+        double2 z = make_double2(0.0, 0.0);
+        if (rows[rl] >= 0) {
+            const double2* X = spec + rows[rl];
+            double2 xk = X[k], xm = X[M - k];
+            if (k == 0) { xk.y = 0; xm.y = 0; }   // kx = 0 and kx = M bins are real
+            const double2 xc = cconj(xm);
+            z = cadd(cadd(xk, xc), cmul_pi(cmul_f(csub(xk, xc), cconj(__ldg(twx + k)))));
+        }
+        A[rl * M + k] = z;
+    }
+    __syncthreads();
+    double2* Z = smem_fft<true>(A, B, M, R, M, pl, twx, 2);
+    for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
+        const int rl = quot(t, rM), n = t - rl * M;
+        const int row = row0 + rl;
+        if (row >= nrows || 2 * n >= d.nx) continue;   // nx is even
+        const double2 z = Z[rl * M + n];
+        double* out = phi + (long long)row * d.nx;
+        out[2 * n] = z.x * scale;
+        out[2 * n + 1] = z.y * scale;
     }
 }
 
 // apply_fft_pressure_correction (pressure_solver.f90:117-173) with walls in
 // x (WX) or z (WZ): a wall face u(1) / w(1) keeps its boundary value (no
 // correction), as the red-black sweeps leave it; other faces as k_correct.
+// The launch covers the ghost layers and copies u* there (and v in row 1):
+// the red-black projection starts with u <- u* on the whole padded arrays
+// (pressure_redblack.f90:63-84), so the edges and corners, which the face
+// rules of apply_bc_redblack do not set and the predictor's diagonal
+// neighbours read, hold u*'s values.
 template <bool IBM, bool WX, bool WZ>
 __global__ void __launch_bounds__(256)
-k_correct_walls(mdx_dims d, double dx, double dy, double dz, mdx_dscal dgs, const double* __restrict__ phi,
+k_correct_walls(mdx_dims d, fft_h h, mdx_dscal dgs, const double* __restrict__ phi,
                 const double* __restrict__ us, const double* __restrict__ vs, const double* __restrict__ ws,
                 double* __restrict__ un, double* __restrict__ vn, double* __restrict__ wn, double* __restrict__ pn,
                 const double* __restrict__ cu, const double* __restrict__ cv, const double* __restrict__ cw) {
     const double dt_gamma = dgs.get();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > d.nx || j > d.ny || k > d.nz) return;
-    int im = i - 1, km = k - 1;
-    if (im < 1) im = d.nx;
-    if (km < 1) km = d.nz;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z * blockDim.z + threadIdx.z;
+    if (i > d.nx + 1 || j > d.ny + 1 || k > d.nz + 1) return;
     const long long c = pidx(d, i, j, k);
-    const double r = __ldg(phi + ridx(d, i, k, j));
-    if (WX && i == 1) {
-        un[c] = __ldg(us + c);
-    } else {
-        double u = (__ldg(us + c) - dt_gamma * (r - __ldg(phi + ridx(d, im, k, j))) / dx);
-        if (IBM) u = u / (1.0 + dt_gamma * __ldg(cu + c));
-        un[c] = u;
+    double u = __ldg(us + c), v = __ldg(vs + c), w = __ldg(ws + c);
+    if (i >= 1 && i <= d.nx && j >= 1 && j <= d.ny && k >= 1 && k <= d.nz) {
+        const int im = i == 1 ? d.nx : i - 1, km = k == 1 ? d.nz : k - 1;
+        const double r = __ldg(phi + ridx(d, i, k, j));
+        if (!(WX && i == 1)) {
+            u = u - div_by(dt_gamma * (r - __ldg(phi + ridx(d, im, k, j))), h.dx, h.rdx);
+            if (IBM) u = u / (1.0 + dt_gamma * __ldg(cu + c));
+        }
+        if (!(WZ && k == 1)) {
+            w = w - div_by(dt_gamma * (r - __ldg(phi + ridx(d, i, km, j))), h.dz, h.rdz);
+            if (IBM) w = w / (1.0 + dt_gamma * __ldg(cw + c));
+        }
+        if (j >= 2) {
+            v = v - div_by(dt_gamma * (r - __ldg(phi + ridx(d, i, k, j - 1))), h.dy, h.rdy);
+            if (IBM) v = v / (1.0 + dt_gamma * __ldg(cv + c));
+        }
+        pn[c] = pn[c] + r;
     }
-    if (WZ && k == 1) {
-        wn[c] = __ldg(ws + c);
-    } else {
-        double w = (__ldg(ws + c) - dt_gamma * (r - __ldg(phi + ridx(d, i, km, j))) / dz);
-        if (IBM) w = w / (1.0 + dt_gamma * __ldg(cw + c));
-        wn[c] = w;
-    }
-    pn[c] = pn[c] + r;
-    if (j >= 2) {
-        double v = (__ldg(vs + c) - dt_gamma * (r - __ldg(phi + ridx(d, i, k, j - 1))) / dy);
-        if (IBM) v = v / (1.0 + dt_gamma * __ldg(cv + c));
-        vn[c] = v;
-    }
+    un[c] = u;
+    vn[c] = v;
+    wn[c] = w;
 }
 
 // ---------------------------------------------------------------------------
@@ -1099,6 +1313,15 @@ static int launch_ifftx(mdx_ctx_t* ctx, const char* what, typename cx<C2>::R sca
     return MDX_OK;
 }
 
+// The middle of the solve on the solve grid (pivots in k_zty's order: no c').
+static int launch_zty(mdx_ctx_t* ctx) {
+    const mdx_dims& e = ctx->dfft;
+    const mdx_grid_t& g = ctx->g;
+    MDX_LAUNCH(ctx, MDX_T_THOMAS, "fft z, thomas, ifft z", k_zty<false>, e.nxh, zty_threads(e.ny, e.nz), zty_bytes(e.ny, e.nz, false), e,
+               1.0 / (g.dy * g.dy), g.dx, g.dz, ctx->spec, ctx->plan_z, ctx->tw_z, ctx->thomas_dinv);
+    return MDX_OK;
+}
+
 // Walls in x or z: the pressure boundary condition must be Neumann (type 1,
 // value 0) on both faces of that direction, and y must have walls with
 // Neumann pressure (the Thomas solve).  Returns MDX_OK and sets the flags.
@@ -1161,7 +1384,6 @@ int mdx_fft_init(mdx_ctx_t* ctx) {
         MDX_CUDA(ctx, cudaMalloc(&ctx->f[MDX_PHI], sizeof(double) * d.nint));
         MDX_CUDA(ctx, cudaMemset(ctx->f[MDX_PHI], 0, sizeof(double) * d.nint));
     }
-    if (ctx->fft_ext_x || ctx->fft_ext_z) MDX_CUDA(ctx, cudaMalloc(&ctx->phi_ext, sizeof(double) * D.nint));
 
     // Modified wavenumbers on the host with libm sin, pressure_fft.f90:53,61
     // (of the solve grid's lengths).
@@ -1185,7 +1407,11 @@ int mdx_fft_init(mdx_ctx_t* ctx) {
     MDX_CUDA(ctx, cudaMemcpy(dkz, kzp.data(), sizeof(double) * D.nz, cudaMemcpyHostToDevice));
     const long long tsize = (long long)D.ny * D.nxh * nzh;
     MDX_CUDA(ctx, cudaMalloc(&ctx->thomas_dinv, sizeof(double) * tsize));
-    MDX_CUDA(ctx, cudaMalloc(&ctx->thomas_cp, sizeof(double) * tsize));
+    // the plane in shared memory where it fits (the mixed path has its own
+    // solve and reads both tables)
+    const bool in_smem = zty_ok(D.ny, D.nz, false) && ctx->opts.precision != MDX_PREC_MIXED && ctx->opts.fft_kernel == 0;
+    if (!in_smem) MDX_CUDA(ctx, cudaMalloc(&ctx->thomas_cp, sizeof(double) * tsize));
+    else MDX_CUDA(ctx, cudaFuncSetAttribute(k_zty<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_ZTY_SMEM));
     const double dyi2 = 1.0 / (ctx->g.dy * ctx->g.dy);
     const int nm = D.nxh * nzh;
     k_thomas_tables<<<(nm + 127) / 128, 128, 0, ctx->stream>>>(D.nxh, nzh, D.ny, dyi2, dkx, dkz, ctx->thomas_dinv,
@@ -1197,7 +1423,8 @@ int mdx_fft_init(mdx_ctx_t* ctx) {
     if (rc != MDX_OK) return rc;
 
     MDX_CUDA(ctx, cudaFuncSetAttribute(k_div_fftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftx_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_div_fftx_walls, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
+    MDX_CUDA(ctx, cudaFuncSetAttribute(k_ifftx_walls, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
     MDX_CUDA(ctx, cudaFuncSetAttribute(k_ifftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
     MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
     MDX_CUDA(ctx, cudaFuncSetAttribute(k_fftz<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM));
@@ -1218,53 +1445,43 @@ void mdx_fft_free(mdx_ctx_t* ctx) {
     cudaFree(ctx->tw_x); ctx->tw_x = nullptr;
     cudaFree(ctx->tw_z); ctx->tw_z = nullptr;
     cudaFree(ctx->thomas_dinv); ctx->thomas_dinv = nullptr;
-    cudaFree(ctx->thomas_cp); ctx->thomas_cp = nullptr;
-    cudaFree(ctx->phi_ext); ctx->phi_ext = nullptr;
+    cudaFree(ctx->thomas_cp); ctx->thomas_cp = nullptr;   // null: the pivots are in k_zty's order
     ctx->fft_ext_x = ctx->fft_ext_z = 0;
 }
 
-// The projection with walls in x or z: divergence on the physical grid,
-// its even extension, the Stockham transforms, Thomas and the inverse on the
-// solve grid, the physical block of phi, the correction.
+// The projection with walls in x or z: divergence on the physical grid and
+// the transforms of its even extension, Thomas and the inverse on the solve
+// grid, the physical block of phi, the correction.
 static int projection_fft_walls(mdx_ctx_t* ctx, mdx_dscal dg) {
     const mdx_dims& d = ctx->d;
     const mdx_dims& e = ctx->dfft;
     const mdx_grid_t& g = ctx->g;
     double** f = ctx->f;
-    dim3 block(32, 4, 2);
-    dim3 grid((d.nx + 31) / 32, (d.ny + 3) / 4, (d.nz + 1) / 2);
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "div rhs", k_div_rhs, grid, block, 0, d, make_h(g.dx, g.dy, g.dz), dg, f[MDX_US], f[MDX_VS],
-               f[MDX_WS], f[MDX_PHI]);
-    const int nb = (int)std::min<long long>((e.nint + 255) / 256, 8192);
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "extend rhs", k_extend, nb, 256, 0, d, e, f[MDX_PHI], ctx->phi_ext);
-    const int M = e.nx / 2, nrows = e.nz * e.ny, R = rows_per_block(M, nrows);
+    const int M = e.nx / 2, nrows = d.nz * d.ny, R = rows_per_block(M, nrows);
     const size_t smx = sizeof(double2) * 2 * R * M;
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "fft x (extended)", k_fftx_r2c, (nrows + R - 1) / R, 256, smx, e, R, ctx->phi_ext,
-               ctx->spec, ctx->plan_xh, ctx->tw_x);
-    const int lg = lg_ztile(e.nz, e.nxh, e.ny);
-    const size_t smz = ztile_bytes(e.nz, lg, sizeof(double2));
-    const int zblocks = ((e.nxh + (1 << lg) - 1) >> lg) * e.ny;
-    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "fft z (extended)", (k_fftz<false, double2>), zblocks, 256, smz, e, lg, ctx->spec,
-               ctx->plan_z, ctx->tw_z);
-    const int nm = e.nxh * e.nz;
-    MDX_LAUNCH(ctx, MDX_T_THOMAS, "thomas (extended)", (k_thomas<double2, false>), (nm + 127) / 128, 128, 0, e,
-               1.0 / (g.dy * g.dy), ctx->spec, ctx->thomas_dinv, ctx->thomas_cp);
-    MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft z (extended)", (k_fftz<true, double2>), zblocks, 256, smz, e, lg, ctx->spec,
-               ctx->plan_z, ctx->tw_z);
-    MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft x (extended)", k_ifftx<double2>, (nrows + R - 1) / R, 256, smx, e, R,
-               1.0 / (double)((long long)e.nx * e.nz), ctx->spec, ctx->phi_ext, ctx->plan_xh, ctx->tw_x);
-    const int nbd = (int)std::min<long long>((d.nint + 255) / 256, 8192);
-    MDX_LAUNCH(ctx, MDX_T_FFT_INV, "restrict phi", k_restrict, nbd, 256, 0, d, e, ctx->phi_ext, f[MDX_PHI]);
-    // u <- u* on the whole padded arrays first, as the red-black projection
-    // starts (pressure_redblack.f90:63-84): the edges and corners of the
-    // ghost layers, which the face rules of apply_bc_redblack do not set and
-    // the predictor's diagonal neighbours read, then hold u*'s values there
-    const size_t bytes = sizeof(double) * (size_t)d.npad;
-    MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_UN], f[MDX_US], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_VN], f[MDX_VS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_WN], f[MDX_WS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    const fft_h h = make_h(g.dx, g.dy, g.dz);
+    MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "div+fft x (extended)", k_div_fftx_walls, (nrows + R - 1) / R, 256, smx, d, e, R, h,
+               dg, f[MDX_US], f[MDX_VS], f[MDX_WS], ctx->spec, ctx->plan_xh, ctx->tw_x);
+    if (!ctx->thomas_cp) {
+        MDX_TRY(launch_zty(ctx));
+    } else {
+        const int lg = lg_ztile(e.nz, e.nxh, e.ny);
+        const size_t smz = ztile_bytes(e.nz, lg, sizeof(double2));
+        const int zblocks = ((e.nxh + (1 << lg) - 1) >> lg) * e.ny;
+        MDX_LAUNCH(ctx, MDX_T_FFT_FWD, "fft z (extended)", (k_fftz<false, double2>), zblocks, 256, smz, e, lg,
+                   ctx->spec, ctx->plan_z, ctx->tw_z);
+        const int nm = e.nxh * e.nz;
+        MDX_LAUNCH(ctx, MDX_T_THOMAS, "thomas (extended)", (k_thomas<double2, false>), (nm + 127) / 128, 128, 0, e,
+                   1.0 / (g.dy * g.dy), ctx->spec, ctx->thomas_dinv, ctx->thomas_cp);
+        MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft z (extended)", (k_fftz<true, double2>), zblocks, 256, smz, e, lg,
+                   ctx->spec, ctx->plan_z, ctx->tw_z);
+    }
+    MDX_LAUNCH(ctx, MDX_T_FFT_INV, "ifft x (extended)", k_ifftx_walls, (nrows + R - 1) / R, 256, smx, d, e, R,
+               1.0 / (double)((long long)e.nx * e.nz), ctx->spec, f[MDX_PHI], ctx->plan_xh, ctx->tw_x);
+    dim3 block(32, 4, 2);
+    dim3 grid((d.nxp + 31) / 32, (d.nyp + 3) / 4, (d.nzp + 1) / 2);
     auto go = [&](auto kern) -> int {
-        MDX_LAUNCH(ctx, MDX_T_CORRECT, "correction (walls)", kern, grid, block, 0, d, g.dx, g.dy, g.dz, dg, f[MDX_PHI],
+        MDX_LAUNCH(ctx, MDX_T_CORRECT, "correction (walls)", kern, grid, block, 0, d, h, dg, f[MDX_PHI],
                    f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN], f[MDX_COEF_U],
                    f[MDX_COEF_V], f[MDX_COEF_W]);
         return MDX_OK;
@@ -1293,11 +1510,15 @@ int mdx_k_projection_fft(mdx_ctx_t* ctx, mdx_dscal dg) {
     double** f = ctx->f;
     auto kth = k_thomas<double2, false>;
     MDX_TRY(launch_div_fftx<double2>(ctx, "div+fft x", dg, ctx->spec, ctx->tw_x));
-    MDX_TRY((launch_fftz<false, double2>(ctx, "fft z", ctx->spec, ctx->tw_z)));
-    const int nm = d.nxh * d.nz;
-    MDX_LAUNCH(ctx, MDX_T_THOMAS, "thomas", kth, (nm + 127) / 128, 128, 0, d, 1.0 / (g.dy * g.dy), ctx->spec,
-               ctx->thomas_dinv, ctx->thomas_cp);
-    MDX_TRY((launch_fftz<true, double2>(ctx, "ifft z", ctx->spec, ctx->tw_z)));
+    if (!ctx->thomas_cp) {
+        MDX_TRY(launch_zty(ctx));
+    } else {
+        MDX_TRY((launch_fftz<false, double2>(ctx, "fft z", ctx->spec, ctx->tw_z)));
+        const int nm = d.nxh * d.nz;
+        MDX_LAUNCH(ctx, MDX_T_THOMAS, "thomas", kth, (nm + 127) / 128, 128, 0, d, 1.0 / (g.dy * g.dy), ctx->spec,
+                   ctx->thomas_dinv, ctx->thomas_cp);
+        MDX_TRY((launch_fftz<true, double2>(ctx, "ifft z", ctx->spec, ctx->tw_z)));
+    }
     const double scale = 1.0 / (double)(d.nx * d.nz);
     MDX_TRY(launch_ifftx<double2>(ctx, "ifft x", scale, ctx->spec, f[MDX_PHI], ctx->tw_x));
     dim3 block(32, 8);
@@ -1631,6 +1852,33 @@ extern "C" int mdx_solve_pressure_fft_noalloc(const double* rhs, double* phi, in
     double* kxp = (double*)(base + b_spec + 2 * b_tab + b_twx + b_twz);
     double* kzp = (double*)(base + b_spec + 2 * b_tab + b_twx + b_twz + b_kx);
 
+    const double dyi2 = 1.0 / (dy * dy);
+    const int M = nx / 2;
+    const int nrows = nz * ny;
+    const int R = rows_per_block(M, nrows);
+    const size_t smx = sizeof(double2) * 2 * R * M;
+    const int xblocks = (nrows + R - 1) / R;
+    const double scale = 1.0 / (double)(nx * nz);
+    // A (z, y) plane that fits a block's shared memory: three launches, every
+    // block making the twiddles and pivots it needs (seven launches with the
+    // tables in the scratch otherwise; 56 -> 15 us on 32x24x32).
+    if (zty_ok(ny, nz, true) && nx <= 2048) {
+        const size_t smo = smx + sizeof(double2) * (size_t)nx;
+        const size_t smz = zty_bytes(ny, nz, true), dflt = 48 * 1024;   // above it a kernel needs the attribute
+        cudaError_t b = cudaSuccess;
+        const auto cap = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if (smo > dflt) b = cudaFuncSetAttribute(k_fftx_r2c<true>, cap, MDX_FFT_SMEM);
+        if (smo > dflt && b == cudaSuccess) b = cudaFuncSetAttribute(k_ifftx<double2, true>, cap, MDX_FFT_SMEM);
+        if (smz > dflt && b == cudaSuccess) b = cudaFuncSetAttribute(k_zty<true>, cap, MDX_ZTY_SMEM);
+        if (b != cudaSuccess) return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: cudaFuncSetAttribute failed");
+        k_fftx_r2c<true><<<xblocks, 256, smo, st>>>(d, R, rhs, spec, plx, nullptr);
+        k_zty<true><<<d.nxh, zty_threads(ny, nz), smz, st>>>(d, dyi2, dx, dz, spec, plz, nullptr, nullptr);
+        k_ifftx<double2, true><<<xblocks, 256, smo, st>>>(d, R, scale, spec, phi, plx, nullptr);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: launch: %s", cudaGetErrorString(e));
+        return MDX_OK;
+    }
+
     // Twiddles and modified wavenumbers (pressure_fft.f90:53,61) are built on
     // the device in the scratch, so the call copies nothing from the host.
     {
@@ -1638,18 +1886,12 @@ extern "C" int mdx_solve_pressure_fft_noalloc(const double* rhs, double* phi, in
         k_noalloc_trig<<<(nmax + 255) / 256, 256, 0, st>>>(nx, nz, d.nxh, dx, dz, twx, twz, kxp, kzp);
     }
 
-    const double dyi2 = 1.0 / (dy * dy);
     const int nm = d.nxh * nzh;
     k_thomas_tables<<<(nm + 127) / 128, 128, 0, st>>>(d.nxh, nzh, ny, dyi2, kxp, kzp, dinv, cp);
-    const int M = nx / 2;
-    const int nrows = nz * ny;
-    const int R = rows_per_block(M, nrows);
-    const size_t smx = sizeof(double2) * 2 * R * M;
-    const int xblocks = (nrows + R - 1) / R;
     const int lg = lg_ztile(nz, d.nxh, ny);
     const size_t smz = ztile_bytes(nz, lg, sizeof(double2));
     const int zblocks = ((d.nxh + (1 << lg) - 1) >> lg) * ny;
-    const cudaError_t a1 = cudaFuncSetAttribute(k_fftx_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
+    const cudaError_t a1 = cudaFuncSetAttribute(k_fftx_r2c<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
     const cudaError_t a2 = cudaFuncSetAttribute(k_ifftx<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
     const cudaError_t a3 =
         cudaFuncSetAttribute(k_fftz<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
@@ -1657,11 +1899,11 @@ extern "C" int mdx_solve_pressure_fft_noalloc(const double* rhs, double* phi, in
         cudaFuncSetAttribute(k_fftz<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDX_FFT_SMEM);
     if (a1 != cudaSuccess || a2 != cudaSuccess || a3 != cudaSuccess || a4 != cudaSuccess)
         return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: cudaFuncSetAttribute failed");
-    k_fftx_r2c<<<xblocks, 256, smx, st>>>(d, R, rhs, spec, plx, twx);
+    k_fftx_r2c<false><<<xblocks, 256, smx, st>>>(d, R, rhs, spec, plx, twx);
     k_fftz<false, double2><<<zblocks, 256, smz, st>>>(d, lg, spec, plz, twz);
     k_thomas<double2, false><<<(d.nxh * nz + 127) / 128, 128, 0, st>>>(d, dyi2, spec, dinv, cp);
     k_fftz<true, double2><<<zblocks, 256, smz, st>>>(d, lg, spec, plz, twz);
-    k_ifftx<double2><<<xblocks, 256, smx, st>>>(d, R, 1.0 / (double)(nx * nz), spec, phi, plx, twx);
+    k_ifftx<double2><<<xblocks, 256, smx, st>>>(d, R, scale, spec, phi, plx, twx);
     e = cudaGetLastError();
     if (e != cudaSuccess) return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: launch: %s", cudaGetErrorString(e));
     return MDX_OK;

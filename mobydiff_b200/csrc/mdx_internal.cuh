@@ -197,7 +197,6 @@ struct mdx_ctx {
     // sized for dfft instead of d
     int fft_ext_x = 0, fft_ext_z = 0;
     mdx_dims dfft{};                         // the solve grid (d itself without walls in x and z)
-    double* phi_ext = nullptr;               // right-hand side, then phi, on dfft in rhs(i,k,j) order
     // mixed-precision FFT path: FP32 spectrum, correction, twiddles, Thomas
     // tables; FP64 zero-wavenumber right-hand side and solution per y
     float2 *spec32 = nullptr, *tw_x32 = nullptr, *tw_z32 = nullptr;
