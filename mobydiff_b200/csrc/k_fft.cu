@@ -538,6 +538,7 @@ template <bool OWN>
 __global__ void __launch_bounds__(512)
 k_zty(mdx_dims d, double dyi2, double dx, double dz, double2* __restrict__ spec, mdx_fft_plan pl,
       const double2* __restrict__ twz, const double* __restrict__ dinv) {
+    if (OWN) mdx_grid_next();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const int nz = d.nz, ny = d.ny, nxh = d.nxh, nzh = nz / 2 + 1, ls = nz | 1, kx = blockIdx.x;
     double2* A = reinterpret_cast<double2*>(sm_raw);
@@ -550,20 +551,21 @@ k_zty(mdx_dims d, double dyi2, double dx, double dz, double2* __restrict__ spec,
     if (OWN && (int)threadIdx.x < T0)
         for (int kz = threadIdx.x; kz < nzh; kz += blockDim.x)
             thomas_pivots(ny, dyi2, wave2(kx, d.nx, dx) + wave2(kz, nz, dz), kx == 0 && kz == 0, D + kz, nzh);
-    if ((int)threadIdx.x >= T0 || few) {
-        const int step = few ? blockDim.x : blockDim.x - T0, t0 = few ? threadIdx.x : threadIdx.x - T0;
+    const int step = few || !OWN ? blockDim.x : blockDim.x - T0, t0 = few || !OWN ? threadIdx.x : threadIdx.x - T0;
+    if (OWN && t0 >= 0)
+        for (int t = t0; t < nz; t += step) {
+            double sn, cs;
+            sincospi(2.0 * (double)t / (double)nz, &sn, &cs);
+            T[t] = make_double2(cs, -sn);
+        }
+    if (OWN) mdx_grid_wait();   // the tables depend on nothing before
+    if (t0 >= 0) {
 #pragma unroll 4
         for (int t = t0; t < ny * nz; t += step) {
             const int j = quot(t, rz), kz = t - j * nz;
             A[j * ls + kz] = __ldcg(spec + (long long)t * nxh + kx);
         }
-        if (OWN) {
-            for (int t = t0; t < nz; t += step) {
-                double sn, cs;
-                sincospi(2.0 * (double)t / (double)nz, &sn, &cs);
-                T[t] = make_double2(cs, -sn);
-            }
-        } else {
+        if (!OWN) {
             const double* src = dinv + (long long)kx * ny * nzh;
             for (int t = t0; t < ny * nzh; t += step) D[t] = __ldg(src + t);
         }
@@ -632,6 +634,7 @@ template <typename C2, bool OWN = false>
 __global__ void __launch_bounds__(256)
 k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec, typename cx<C2>::R* __restrict__ phi,
         mdx_fft_plan pl, const C2* __restrict__ tw_g) {
+    if (OWN) mdx_grid_next();
     typedef typename cx<C2>::R RT;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     C2* sm = reinterpret_cast<C2*>(sm_raw);
@@ -644,6 +647,7 @@ k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec
         twx = B + R * M;
         __syncthreads();
     }
+    if (OWN) mdx_grid_wait();
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
     const float rM = 1.0f / (float)M;
@@ -1003,6 +1007,7 @@ template <bool OWN>
 __global__ void __launch_bounds__(256)
 k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restrict__ spec, mdx_fft_plan pl,
            const double2* __restrict__ tw_g) {
+    if (OWN) mdx_grid_next();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     double2* sm = reinterpret_cast<double2*>(sm_raw);
     const int M = d.nx / 2;
@@ -1013,6 +1018,7 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
         own_twiddles(B + R * M, d.nx);
         twx = B + R * M;
     }
+    if (OWN) mdx_grid_wait();
     const int nrows = d.nz * d.ny;
     const int row0 = blockIdx.x * R;
     const float rM = 1.0f / (float)M, rN = 1.0f / (float)(M + 1);
@@ -1871,9 +1877,10 @@ extern "C" int mdx_solve_pressure_fft_noalloc(const double* rhs, double* phi, in
         if (smo > dflt && b == cudaSuccess) b = cudaFuncSetAttribute(k_ifftx<double2, true>, cap, MDX_FFT_SMEM);
         if (smz > dflt && b == cudaSuccess) b = cudaFuncSetAttribute(k_zty<true>, cap, MDX_ZTY_SMEM);
         if (b != cudaSuccess) return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: cudaFuncSetAttribute failed");
-        k_fftx_r2c<true><<<xblocks, 256, smo, st>>>(d, R, rhs, spec, plx, nullptr);
-        k_zty<true><<<d.nxh, zty_threads(ny, nz), smz, st>>>(d, dyi2, dx, dz, spec, plz, nullptr, nullptr);
-        k_ifftx<double2, true><<<xblocks, 256, smo, st>>>(d, R, scale, spec, phi, plx, nullptr);
+        (void)mdx_launch_chained(st, k_fftx_r2c<true>, xblocks, 256, smo, d, R, rhs, spec, plx, nullptr);
+        (void)mdx_launch_chained(st, k_zty<true>, d.nxh, zty_threads(ny, nz), smz, d, dyi2, dx, dz, spec, plz, nullptr,
+                                 nullptr);
+        (void)mdx_launch_chained(st, k_ifftx<double2, true>, xblocks, 256, smo, d, R, scale, spec, phi, plx, nullptr);
         e = cudaGetLastError();
         if (e != cudaSuccess) return mdx_fail(nullptr, MDX_ERR_CUDA, "noalloc solve: launch: %s", cudaGetErrorString(e));
         return MDX_OK;
