@@ -627,13 +627,16 @@ int mdx_divergence_norms(mdx_ctx_t* ctx, double* l2, double* linf) {
 static int rk_step_eager(mdx_ctx_t* ctx, double dt, long long* iters, const double* dtp = nullptr) {
     double a[3], b[3], c[3];
     mdx_rk_coeffs(a, b, c);
+    const bool gh = ctx->opts.solver == MDX_SOLVER_FFT && mdx_fft_ghosts(ctx);
     for (int s = 0; s < 3; ++s) {
         const double da = dt * a[s], db = dt * b[s], dg = dt * c[s];
-        if (dtp) {
-            MDX_TRY(mdx_k_momentum(ctx, mdx_dscal(dtp, a[s]), mdx_dscal(dtp, b[s]), mdx_dscal(dtp, c[s])));
-            MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_STAR));
-            MDX_TRY(mdx_k_projection_fft(ctx, mdx_dscal(dtp, c[s])));
-            MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_N));
+        if (gh || dtp) {
+            const mdx_dscal xa = dtp ? mdx_dscal(dtp, a[s]) : mdx_dscal(da), xb = dtp ? mdx_dscal(dtp, b[s]) : mdx_dscal(db),
+                            xg = dtp ? mdx_dscal(dtp, c[s]) : mdx_dscal(dg);
+            MDX_TRY(mdx_k_momentum(ctx, xa, xb, xg, gh));
+            if (!gh) MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_STAR));
+            MDX_TRY(mdx_k_projection_fft(ctx, xg, gh));
+            if (!gh) MDX_TRY(mdx_k_apply_bc(ctx, MDX_BC_N));
             continue;
         }
         MDX_TRY(mdx_k_momentum(ctx, da, db, dg));

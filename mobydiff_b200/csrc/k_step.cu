@@ -23,7 +23,8 @@
 
 // DTD: the three step scalars come from the device's dt (adaptive-dt graph);
 // otherwise their values are kernel parameters.
-template <bool IBM, bool DTD, int KZ>
+// GH: the ghost values of u*, v*, w* are set too (bc_fft_ghosts).
+template <bool IBM, bool DTD, int KZ, bool GH>
 __global__ void __launch_bounds__(256, 4)
 k_momentum(mdx_dims d, mdx_step_params p, mdx_dscal da, mdx_dscal db, mdx_dscal dg,
            const double* __restrict__ un, const double* __restrict__ vn, const double* __restrict__ wn,
@@ -67,6 +68,7 @@ k_momentum(mdx_dims d, mdx_step_params p, mdx_dscal da, mdx_dscal db, mdx_dscal 
         n.w_c_v = w_c; n.w_km_v = w_km; n.w_im_v = w_im; n.w_jm_v = w_jm;
         n.p_km_v = p_km;
         momentum_vals<IBM>(n, p, dt_alpha, dt_beta, dt_gamma, us, vs, ws, ou, ov, ow, cu, cv, cw, c, q, c, i, j, k);
+        if (GH && bc_fft_edge(d, i, j, k)) bc_fft_ghosts(d, us, vs, ws, nullptr, i, j, k);
         u_km = u_c; u_c = n.u_kp_v; u_ip_km = n.u_ip_v;
         v_km = v_c; v_c = n.v_kp_v; v_jp_km = n.v_jp_v;
         w_km = w_c; w_c = n.w_kp_v; w_im = n.w_im_kp_v; w_jm = n.w_jm_kp_v;
@@ -89,7 +91,7 @@ mdx_step_params mdx_make_params(const mdx_ctx_t* ctx) {
     return p;
 }
 
-int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg) {
+int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg, bool ghosts) {
     const mdx_dims& d = ctx->d;
     dim3 block(32, 8, 1);
     // planes per block: 8 (the values carried from plane to plane), fewer while
@@ -103,8 +105,10 @@ int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg) {
     const bool dev = da.p || db.p || dg.p;
     auto go = [&](auto kc) -> int {
         constexpr int K = decltype(kc)::value;
-        auto kfn = ctx->ibm_zero ? (dev ? k_momentum<false, true, K> : k_momentum<false, false, K>)
-                                 : (dev ? k_momentum<true, true, K> : k_momentum<true, false, K>);
+        auto kfn = ghosts ? (ctx->ibm_zero ? (dev ? k_momentum<false, true, K, true> : k_momentum<false, false, K, true>)
+                                           : (dev ? k_momentum<true, true, K, true> : k_momentum<true, false, K, true>))
+                          : (ctx->ibm_zero ? (dev ? k_momentum<false, true, K, false> : k_momentum<false, false, K, false>)
+                                           : (dev ? k_momentum<true, true, K, false> : k_momentum<true, false, K, false>));
         MDX_LAUNCH(ctx, MDX_T_MOMENTUM, "momentum", kfn, grid, block, 0, d, p, da, db, dg, f[MDX_UN], f[MDX_VN],
                    f[MDX_WN], f[MDX_PN], f[MDX_US], f[MDX_VS], f[MDX_WS], f[MDX_OLDRHSU], f[MDX_OLDRHSV],
                    f[MDX_OLDRHSW], f[MDX_COEF_U], f[MDX_COEF_V], f[MDX_COEF_W]);

@@ -372,6 +372,40 @@ __device__ __forceinline__ void bcrb_z_col(const mdx_dims& d, const mdx_bc_dev& 
     }
 }
 
+// The ghost values that follow from cell (i, j, k), as apply_bc of the FFT
+// builds leaves them (src/modules/boundary.f90:23-170; k_bc_fft composes its
+// phases): the cell's copies beyond the periodic x and z, u and w negated
+// beyond a y wall, v 0 on the wall rows.  Called by the thread that wrote the
+// cell; p may be null.
+__device__ __forceinline__ bool bc_fft_edge(const mdx_dims& d, int i, int j, int k) {
+    return i == 1 || i == d.nx || j == 1 || j == d.ny || k == 1 || k == d.nz;
+}
+__device__ __forceinline__ void bc_fft_ghosts(const mdx_dims& d, double* un, double* vn, double* wn, double* pn, int i,
+                                              int j, int k) {
+    const long long c = pidx(d, i, j, k);
+    const double u = un[c], w = wn[c], v = j == 1 ? 0.0 : vn[c], p = pn ? pn[c] : 0.0;
+    const int gi = i == 1 ? d.nx + 1 : i == d.nx ? 0 : -1, gk = k == 1 ? d.nz + 1 : k == d.nz ? 0 : -1;
+    const int gj = j == 1 ? 0 : j == d.ny ? d.ny + 1 : -1;
+    if (j == 1) vn[c] = 0.0;
+    for (int a = 0; a < 4; ++a) {
+        const int ii = (a & 1) ? gi : i, kk = (a & 2) ? gk : k;
+        if (ii < 0 || kk < 0) continue;
+        if (a) {
+            const long long g = pidx(d, ii, j, kk);
+            un[g] = u;
+            vn[g] = v;
+            wn[g] = w;
+            if (pn) pn[g] = p;
+        }
+        if (gj >= 0) {
+            const long long g = pidx(d, ii, gj, kk);
+            un[g] = -u;
+            wn[g] = -w;
+            if (gj > 0) vn[g] = 0.0;
+        }
+    }
+}
+
 // Seeded channel initial condition (counter-based SplitMix64 finaliser of
 // Steele, Lea & Flood 2014 on seed + golden*(field<<40 | padded index)).
 __device__ __forceinline__ uint64_t ic_hash(uint64_t seed, uint64_t field, uint64_t lin) {

@@ -333,16 +333,19 @@ __device__ __forceinline__ void mdx_grid_next() { asm volatile("griddepcontrol.l
 
 // ---- per-module entry points (internal) --------------------------------------
 mdx_step_params mdx_make_params(const mdx_ctx_t* ctx);
-int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg);
+int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg, bool ghosts = false);
 // apply_bc on the n arrays (un, vn, wn, pn), the * arrays or both.  Inside a
 // step the * arrays need it after the predictor and the n arrays after the
 // projection: the other set has not changed since it was last set.
 enum { MDX_BC_N = 1, MDX_BC_STAR = 2, MDX_BC_ALL = 3 };
 int mdx_k_apply_bc(mdx_ctx_t* ctx, int which = MDX_BC_ALL);
+// Whether a step's predictor and FFT projection set the ghost values of what
+// they write themselves (`ghosts` below), in place of apply_bc.
+bool mdx_fft_ghosts(const mdx_ctx_t* ctx);
 int mdx_k_apply_bc_redblack(mdx_ctx_t* ctx);
 int mdx_fft_init(mdx_ctx_t* ctx);
 void mdx_fft_free(mdx_ctx_t* ctx);
-int mdx_k_projection_fft(mdx_ctx_t* ctx, mdx_dscal dg);
+int mdx_k_projection_fft(mdx_ctx_t* ctx, mdx_dscal dg, bool ghosts = false);
 int mdx_k_projection_fft_mixed(mdx_ctx_t* ctx, double dg);
 int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st);
 int mdx_k_div_norms(mdx_ctx_t* ctx, const double* u, const double* v, const double* w, double* l2, double* linf,
