@@ -225,11 +225,11 @@ __global__ void __launch_bounds__(256) k_conv3(lvl L, int pery, const bf16* __re
 
 template <int CIN, int COUT>
 __host__ __device__ constexpr int wgrad_warps() {
-    return CIN * COUT == 1024 ? 16 : 8;
+    return 16;
 }
 template <int CIN, int COUT>
 __host__ __device__ constexpr int wgrad_smem() {
-    return HV * CIN * 2 + TV * COUT * 2;
+    return 2 * (HV * CIN * 2 + TV * COUT * 2);   // two tiles: one computed, one on its way
 }
 template <int CIN, int COUT>
 __host__ __device__ constexpr int wgrad_len() {
@@ -245,8 +245,7 @@ __global__ void __launch_bounds__(wgrad_warps<CIN, COUT>() * 32, 1)
     constexpr int NW = wgrad_warps<CIN, COUT>(), NTH = NW * 32;
     constexpr int MT = COUT / 16, U = 27 * MT, UPW = (U + NW - 1) / NW, NTN = CIN / 8;
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char* sx = smem;
-    unsigned char* sg = smem + HV * CIN * 2;
+    constexpr int TILE = HV * CIN * 2 + TV * COUT * 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mi = lane >> 3, r8 = lane & 7;
     float acc[UPW][NTN][4];
@@ -258,10 +257,11 @@ __global__ void __launch_bounds__(wgrad_warps<CIN, COUT>() * 32, 1)
             for (int e = 0; e < 4; ++e) acc[u][n][e] = 0.f;
     float bsum = 0.f;
     const int ntiles = tiles_of(L);
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    auto stage = [&](int tile, int buf) {
         int x0, y0, z0;
         tile_origin(L, tile, x0, y0, z0);
-        __syncthreads();   // the previous tile's reads are done
+        unsigned char* sx = smem + buf * TILE;
+        unsigned char* sg = sx + HV * CIN * 2;
         stage_halo<CIN, NTH>(sx, X, L, pery, x0, y0, z0);
         constexpr int GCH = COUT / 8;
         for (int q = threadIdx.x; q < TV * GCH; q += NTH) {
@@ -273,10 +273,23 @@ __global__ void __launch_bounds__(wgrad_warps<CIN, COUT>() * 32, 1)
             else
                 *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
         }
-        cp_commit_wait();
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    if ((int)blockIdx.x < ntiles) stage(blockIdx.x, 0);
+    int buf = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+        const int next = tile + (int)gridDim.x;
+        if (next < ntiles) stage(next, buf ^ 1);
+        if (next < ntiles) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
+        const unsigned char* sx = smem + buf * TILE;
+        const unsigned char* sg = sx + HV * CIN * 2;
         if (threadIdx.x < COUT) {
+            // one warp's serial sum before its share of the products: its loads
+            // go ahead of the additions, or the block waits for it at each tile
             const int co = threadIdx.x;
+#pragma unroll 32
             for (int v = 0; v < TV; ++v)
                 bsum += __bfloat162float(*reinterpret_cast<const bf16*>(sg + sw_off<COUT>(v, co >> 3) + (co & 7) * 2));
         }
@@ -301,6 +314,7 @@ __global__ void __launch_bounds__(wgrad_warps<CIN, COUT>() * 32, 1)
                 }
             }
         }
+        __syncthreads();   // this tile's reads are done before its buffer is staged again
     }
     float* P = part + (long long)blockIdx.x * wgrad_len<CIN, COUT>();
     const int g = lane >> 2, t4 = lane & 3;
@@ -323,12 +337,29 @@ __global__ void __launch_bounds__(wgrad_warps<CIN, COUT>() * 32, 1)
 }
 
 // out[j] = sum_b part[b][j] in block order.
-__global__ void k_sum_parts(int nblk, int len, const float* __restrict__ part, float* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= len) return;
+// Sum of the blocks' partials in block order: a block takes 32 values, its
+// threads bring SUM_ROWS partials of each to shared memory together and one
+// warp adds them up in order (one thread per value waited for a load every
+// few additions: 57 us for the head's 1024 partials of 18 values).
+constexpr int SUM_ROWS = 128;
+__global__ void __launch_bounds__(256) k_sum_parts(int nblk, int len, const float* __restrict__ part, float* __restrict__ out) {
+    __shared__ float buf[SUM_ROWS][32];
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int b = 0; b < nblk; ++b) s += part[(long long)b * len + j];
-    out[j] = s;
+    for (int b0 = 0; b0 < nblk; b0 += SUM_ROWS) {
+        const int n = min(SUM_ROWS, nblk - b0);
+#pragma unroll
+        for (int r = 0; r < SUM_ROWS; r += 8)
+            if (j < len && r + row < n) buf[r + row][lane] = __ldg(part + (long long)(b0 + r + row) * len + j);
+        __syncthreads();
+        if (row == 0 && j < len) {
+#pragma unroll 16
+            for (int r = 0; r < n; ++r) s += buf[r][lane];
+        }
+        __syncthreads();
+    }
+    if (row == 0 && j < len) out[j] = s;
 }
 
 struct bf8 {
@@ -974,7 +1005,7 @@ int wgrad_launch(mdx_ctx_t* ctx, mdx_unet* U, const conv_layer& c, const bf16* X
     constexpr int nth = wgrad_warps<CIN, COUT>() * 32, smem = wgrad_smem<CIN, COUT>();
     MDX_LAUNCH(ctx, MDX_T_OTHER, "unet wgrad", kfn, nb, nth, smem, L, U->pery, X, Gd, U->part);
     // W block then bias block: both contiguous in the parameter layout
-    MDX_LAUNCH(ctx, MDX_T_OTHER, "unet wgrad sum", k_sum_parts, (len + 255) / 256, 256, 0, nb, len, U->part,
+    MDX_LAUNCH(ctx, MDX_T_OTHER, "unet wgrad sum", k_sum_parts, (len + 31) / 32, 256, 0, nb, len, U->part,
                U->grad + c.w_off);
     return MDX_OK;
 }
@@ -1080,7 +1111,7 @@ int head_train(mdx_ctx_t* ctx, mdx_unet* U, const float* target, float tscale, f
     MDX_LAUNCH(ctx, MDX_T_OTHER, "unet head", k_head_train<16>, nb, HEAD_THREADS, 0, n, U->act.back(),
                U->param + U->head_off, target, tscale, (float)U->o.slope, U->G[0], U->head_part, out);
     // dw (16) and db land at head_off; the squared error after them
-    MDX_LAUNCH(ctx, MDX_T_OTHER, "unet head sum", k_sum_parts, 1, 32, 0, nb, len, U->head_part, U->out);
+    MDX_LAUNCH(ctx, MDX_T_OTHER, "unet head sum", k_sum_parts, (len + 31) / 32, 256, 0, nb, len, U->head_part, U->out);
     MDX_CUDA(ctx, cudaMemcpyAsync(U->grad + U->head_off, U->out, sizeof(float) * (len - 1), cudaMemcpyDeviceToDevice,
                                   ctx->stream));
     return MDX_OK;
@@ -1575,8 +1606,7 @@ int mdx_unet_loss_grad(mdx_ctx_t* ctx, const float* in4, const float* target, do
     MDX_CUDA(ctx, cudaMemcpyAsync(U->in, in4, sizeof(float) * NIN * n, cudaMemcpyHostToDevice, ctx->stream));
     MDX_CUDA(ctx, cudaMemcpyAsync(t, target, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
     MDX_CUDA(ctx, cudaMemsetAsync(U->grad, 0, sizeof(float) * U->nparam, ctx->stream));
-    float* dout = nullptr;
-    if (out) MDX_TRY(dalloc(ctx, &dout, n));
+    float* dout = out ? reinterpret_cast<float*>(U->delta) : nullptr;   // scratch for the output
     int rc = loss_grad(ctx, U, U->in, t, 1.0f, dout);
     float sse = 0.f;
     if (rc == MDX_OK) {
@@ -1586,7 +1616,6 @@ int mdx_unet_loss_grad(mdx_ctx_t* ctx, const float* in4, const float* target, do
         const cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = mdx_fail(ctx, MDX_ERR_CUDA, "unet loss/grad: %s", cudaGetErrorString(e));
     }
-    if (dout) cudaFree(dout);
     if (loss) *loss = (double)sse / (double)n;
     if (rc == MDX_OK) rc = check_tc(ctx, U);
     return rc;
