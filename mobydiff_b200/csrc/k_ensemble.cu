@@ -27,6 +27,7 @@
 // autotuner whose choice is cached in a JSON file.
 #include "mdx_cell.cuh"
 #include "mdx_cell32.cuh"
+#include "mdx_resident_dev.cuh"
 
 #include <cooperative_groups.h>
 
@@ -140,6 +141,12 @@ struct ens_args {
     // 0: the whole substage; 1: up to the warm start, then the network's
     // inputs; 2: from the learned correction on (the network ran between)
     int split;
+    // on-chip FP32 face sweeps (res_* below); rbox null: not used
+    struct ens_plan* rplan;          // per member: its blocks and their boxes
+    int* rstate;                     // {this round's plan holds, a block gave up a wait}
+    unsigned* rseq;                  // last sequence number used
+    word* rbox;                      // inboxes, rstride words each
+    int rstride, rsmem;              // rsmem: shared memory of a block for its box
     const int* learn_ok;             // per member: the network wrote a correction
     int gate_period;                 // > 0: apply it per substage only while it takes fewer iterations
 };
@@ -474,6 +481,110 @@ __device__ void sweep32_active(const ens_args& A, int parity) {
         sweep32_tile(A, parity, active_tile(pref, A.half_begin, A.nmem, vt).y);
 }
 
+// ---------------------------------------------------------------------------
+// FP32 face sweeps on chip.  While the sweeping members' cells fit the
+// blocks' registers, a round of check_every iterations runs as
+// k_sor_resident.cu's does: each member has a share of the blocks by its
+// cells, cut into boxes, and a block exchanges face values with its
+// neighbours only -- instead of one grid-wide barrier per colour sweep of all
+// members, with the state in L2.  The blocks are dealt out again each round,
+// so the members that need the most iterations end up with all of them.
+// Measured on six members of 49 k to 246 k cells: 108 -> 61 ms per step, the
+// host's copies of the fields included.
+// ---------------------------------------------------------------------------
+constexpr int RES_KZ = 8;            // planes a thread holds
+struct ens_plan { int first, nyb, nzb, by, bz; };
+
+struct ens_faces {                   // a member as face_run_box wants it
+    typedef float T;
+    static constexpr bool HAS_R = true;
+    mdx_dims d;
+    mixed_params P;
+    float *u, *v, *w, *q;
+    const float *r, *mu, *fac;
+    __device__ __forceinline__ long long at(int i, int j, int k) const { return cidx(d, i, j, k); }
+    __device__ __forceinline__ T res(int i, int j, int k) const { return r[cidx(d, i, j, k)]; }
+    __device__ __forceinline__ void column(face_col<T>& c, int i, int j) const {
+        const int np = split_plane_elems(d), ip = i == d.nx ? 1 : i + 1;
+        c.mu_u = mu[pidx2(d, i, j)];
+        c.mu_ux = mu[pidx2(d, ip, j)];
+        c.mu_v = mu[np + pidx2(d, i, j)];
+        c.mu_vy = mu[np + pidx2(d, i, j + 1)];
+        c.mu_w = mu[2 * np + pidx2(d, i, j)];
+        c.fac = fac[pidx2(d, i, j)];
+    }
+    __device__ __forceinline__ void cell(const face_col<T>& c, T rc, T& u_i, T& u_ip, T& v_j, T& v_jp, T& w_k, T& w_kp,
+                                         T& pc, int j, bool) const {
+        sweep32_update(P, rc, u_i, u_ip, v_j, v_jp, w_k, w_kp, pc, c.mu_u, c.mu_ux, c.mu_v, c.mu_vy, c.mu_w, c.fac,
+                       j > 1, j < d.ny);
+    }
+};
+
+// The blocks of this round, by block 0: a share of the grid per sweeping
+// member, cut where the largest box is cheapest (make_plan of
+// k_sor_resident.cu).  rstate[0] = 0 when a member does not fit its share.
+__device__ void plan_resident(const ens_args& A) {
+    if (blockIdx.x != 0) return;
+    __shared__ int bad;
+    if (threadIdx.x == 0) bad = 0;
+    __syncthreads();
+    const int G = (int)gridDim.x, nt = (int)blockDim.x;
+    const int total = A.act[2 * A.nmem + 1];   // cell tiles of the sweeping members
+    if ((long long)total * ETILE > 2LL * RES_KZ * G * nt) {
+        if (threadIdx.x == 0) A.rstate[0] = 0;
+        return;
+    }
+    for (int m = threadIdx.x; m < A.nmem; m += nt) {
+        ens_plan p{0, 0, 0, 0, 0};
+        if (A.st[m].active) {
+            const int ny = A.mem[m].d.ny, nz = A.mem[m].d.nz, tpr = A.mem[m].d.nx / 2;
+            const int share = max(1, (int)((long long)G * (A.cell_begin[m + 1] - A.cell_begin[m]) / total));
+            int best = 0x7fffffff;
+            for (int by0 = 1; by0 <= ny && by0 * tpr <= nt; ++by0) {
+                const int nyb = (ny + by0 - 1) / by0, by = (ny + nyb - 1) / nyb;
+                const int nzb = min(nz, share / nyb);
+                if (nzb < 1) continue;
+                const int bz = (nz + nzb - 1) / nzb;
+                if (bz > RES_KZ || (int)face_smem<float>(by, bz, tpr) > A.rsmem) continue;
+                const int cost = bz * max(12 * ((by * tpr + 31) / 32), 100) + (by + bz) * tpr;
+                if (cost < best) {
+                    best = cost;
+                    p = ens_plan{0, nyb, nzb, by, bz};
+                }
+            }
+            if (p.nyb == 0 || 2 * (p.by + p.bz) * tpr > A.rstride) bad = 1;
+        }
+        A.rplan[m] = p;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int at = 0;
+        for (int m = 0; m < A.nmem; ++m) {
+            A.rplan[m].first = at;
+            at += A.rplan[m].nyb * A.rplan[m].nzb;
+        }
+        A.rstate[0] = !bad && at <= G;
+    }
+}
+
+// `iters` iterations of every sweeping member, this block its box of its member.
+__device__ void sweeps_resident(const ens_args& A, int iters) {
+    extern __shared__ __align__(16) unsigned char ens_sm[];
+    for (int m = 0; m < A.nmem; ++m) {
+        const ens_plan p = A.rplan[m];
+        const int at = (int)blockIdx.x - p.first;
+        if (at < 0 || at >= p.nyb * p.nzb) continue;
+        const ens_member& M = A.mem[m];
+        const float* p32 = A.st[m].p32;
+        const ens_faces a{M.d, mixed_params{p32[0], p32[1], p32[2], p32[3]}, M.du, M.dv, M.dw, M.dp, M.r32, M.mu32, M.fac32};
+        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride};
+        const res_box b = make_box<0>(M.d.ny, M.d.nz, p.nyb, p.nzb, R.tpr, p.first, at);
+        if (!face_run_box<ens_faces, 0, RES_KZ>(a, b, R, iters, A.rbox, *(volatile unsigned*)A.rseq, ens_sm) && threadIdx.x == 0)
+            A.rstate[1] = 1;
+        break;
+    }
+}
+
 __device__ __forceinline__ mdx_sor_params proj_params(const ens_member& M, double dg) {
     mdx_sor_params p = M.sp;
     p.idt = 1.0 / dg;
@@ -566,6 +677,7 @@ __device__ __forceinline__ void guess_cell(const ens_member& M, double dg, unsig
 // the latency-bound sweeps.  The autotuner picks one.
 template <int MINB>
 __global__ void __launch_bounds__(MAX_THREADS, MINB) k_ens_substage(ens_args A) {
+    constexpr bool RES = MINB == 1;   // the 64-register variant has no room for the on-chip sweeps
     cg::grid_group grid = cg::this_grid();
     const int s = A.substage;
     const bool warm = A.momentum && A.guess_mode != MDX_GUESS_ZERO;
@@ -887,14 +999,32 @@ __global__ void __launch_bounds__(MAX_THREADS, MINB) k_ens_substage(ens_args A) 
             }
             grid.sync();
             compact_active(A);
+            const bool res = RES && A.rbox;
+            if constexpr (RES)
+                if (res) {
+                    __syncthreads();
+                    plan_resident(A);
+                }
             grid.sync();
             if (A.act[A.nmem] == 0) break;   // every member done
             const int mm = A.check_every;
-            for (int q = 0; q < mm; ++q)
-                for (int parity = 0; parity < 2; ++parity) {
-                    sweep32_active(A, parity);
-                    grid.sync();
+            if (RES && res && A.rstate[0]) {
+                if constexpr (RES) sweeps_resident(A, mm);
+                grid.sync();
+                if (blockIdx.x == 0 && threadIdx.x == 0) *A.rseq += 2u * (unsigned)mm;   // read again after barriers
+                if (A.rstate[1]) {   // a block gave up a wait: the run ends here
+                    if (blockIdx.x == 0)
+                        for (int m = threadIdx.x; m < A.nmem; m += blockDim.x)
+                            if (A.st[m].phase != 2) A.st[m].status = MDX_ERR_TIMEOUT;
+                    break;
                 }
+            } else {
+                for (int q = 0; q < mm; ++q)
+                    for (int parity = 0; parity < 2; ++parity) {
+                        sweep32_active(A, parity);
+                        grid.sync();
+                    }
+            }
             for (int ti = blockIdx.x; ti < A.cell.n; ti += gridDim.x)
                 if (A.st[A.cell.t[ti].x].phase == 1) corr_residual_tile(A, ti);
             grid.sync();
@@ -1101,6 +1231,16 @@ struct mdx_ensemble {
     double* net_scal = nullptr;      // 4 per member
     int* learn_ok = nullptr;         // per member
     int gate_period = 0;             // of the loaded network's options
+    // on-chip sweeps: per-member plans, {plan holds, gave up}, the last
+    // sequence number (and a bound of it on the host), the inboxes of rgrid
+    // blocks of rthreads threads
+    ens_plan* rplan = nullptr;
+    int* rstate = nullptr;
+    unsigned* rseq = nullptr;
+    void* rbox = nullptr;
+    size_t rbytes = 0;
+    int rstride = 0, rsmem = 0;
+    double rseq_bound = 0.0;
 };
 
 namespace {
@@ -1140,9 +1280,33 @@ const void* kernel_of(int variant) {
     return variant ? (const void*)k_ens_substage<2> : (const void*)k_ens_substage<1>;
 }
 
+// Whether the on-chip sweeps may be used at all (FP32 faces, the
+// full-register variant), the shared memory they take per block and the words
+// of an inbox: the largest box a block of `threads` can hold of any member.
+bool res_shape(const mdx_ensemble_t* E, int variant, int threads, int* smem, int* stride) {
+    if (variant != 0 || E->opts.precision != MDX_PREC_MIXED || !(E->opts.tol > 0.0) || E->opts.inner_form == 2) return false;
+    *smem = *stride = 0;
+    for (const auto& M : E->hm) {
+        const int tpr = M.d.nx / 2;
+        if (tpr > threads || tpr > 128) return false;
+        const int by = std::max(1, threads / tpr);
+        *smem = std::max(*smem, (int)face_smem<float>(by, RES_KZ, tpr));
+        *stride = std::max(*stride, 2 * (by + RES_KZ) * tpr);
+    }
+    return true;
+}
+
+int res_smem(const mdx_ensemble_t* E, int variant, int threads) {
+    int smem = 0, stride = 0;
+    return res_shape(E, variant, threads, &smem, &stride) ? smem : 0;
+}
+
 int grid_for(mdx_ensemble_t* E, int variant, int threads, int bps, int* grid) {
     int occ = 0;
-    ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_of(variant), threads, 0));
+    const int smem = res_smem(E, variant, threads);
+    if (smem > 48 * 1024)
+        ENS_CUDA(E, cudaFuncSetAttribute(kernel_of(variant), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_of(variant), threads, smem));
     int sms = 0;
     ENS_CUDA(E, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
     if (occ < 1) return efail(E, MDX_ERR_ARG, "ensemble kernel does not fit %d threads per block", threads);
@@ -1179,16 +1343,65 @@ ens_args make_args(mdx_ensemble_t* E, int s, int momentum) {
     A.pot = A.mixed && E->opts.inner_form == 2;
     A.inner_sor = E->opts.inner_sor;
     A.split = 0;
+    A.rplan = E->rplan;
+    A.rstate = E->rstate;
+    A.rseq = E->rseq;
     A.learn_ok = E->learn_ok;
     A.gate_period = E->gate_period;
     return A;
 }
 
+size_t res_bytes(int grid, int stride) { return sizeof(word) * 2 * (size_t)grid * stride; }
+
+// Before launches (outside a capture) of `substages` substages of this shape:
+// the inboxes, and cleared ones before the sequence numbers run out.
+int res_prepare(mdx_ensemble_t* E, int variant, int threads, int grid, int substages) {
+    int smem = 0, stride = 0;
+    if (!res_shape(E, variant, threads, &smem, &stride)) return MDX_OK;
+    if (!E->rplan) {
+        MDX_TRY(ealloc(E, &E->rplan, E->n));
+        MDX_TRY(ealloc(E, &E->rstate, 2));
+        MDX_TRY(ealloc(E, &E->rseq, 1));
+        free_graph(E);
+    }
+    const size_t bytes = res_bytes(grid, stride);
+    const double rounds = (double)E->opts.max_iter + 64.0 * std::max(E->opts.check_every, 1);
+    E->rseq_bound += 2.0 * rounds * substages;
+    bool clear = E->rseq_bound > 4.0e9;
+    if (E->rbytes < bytes) {
+        cudaFree(E->rbox);
+        E->rbox = nullptr;
+        E->rbytes = 0;
+        if (cudaMalloc(&E->rbox, bytes) != cudaSuccess) {   // without them the sweeps run from L2
+            cudaGetLastError();
+            return MDX_OK;
+        }
+        E->rbytes = bytes;
+        free_graph(E);
+        clear = true;
+    }
+    if (clear) {
+        ENS_CUDA(E, cudaMemsetAsync(E->rbox, 0, E->rbytes, E->stream));
+        ENS_CUDA(E, cudaMemsetAsync(E->rseq, 0, sizeof(unsigned), E->stream));
+        E->rseq_bound = 2.0 * rounds * substages;
+    }
+    ENS_CUDA(E, cudaMemsetAsync(E->rstate, 0, 2 * sizeof(int), E->stream));
+    return MDX_OK;
+}
+
 int launch_substage(mdx_ensemble_t* E, int s, int momentum, int variant, int threads, int grid, int split = 0) {
     ens_args A = make_args(E, s, momentum);
     A.split = split;
+    int smem = 0, stride = 0;
+    if (res_shape(E, variant, threads, &smem, &stride) && E->rbytes >= res_bytes(grid, stride)) {
+        A.rbox = (word*)E->rbox;
+        A.rstride = stride;
+        A.rsmem = smem;
+    } else {
+        smem = res_smem(E, variant, threads);
+    }
     void* args[] = {&A};
-    ENS_CUDA(E, cudaLaunchCooperativeKernel(kernel_of(variant), dim3(grid), dim3(threads), args, 0, E->stream));
+    ENS_CUDA(E, cudaLaunchCooperativeKernel(kernel_of(variant), dim3(grid), dim3(threads), args, smem, E->stream));
     E->launches++;
     return MDX_OK;
 }
@@ -1361,6 +1574,7 @@ int mdx_ensemble_destroy(mdx_ensemble_t* E) {
     cudaFree(E->dhalf_begin);
     cudaFree(E->dact);
     cudaFree(E->part);
+    cudaFree(E->rbox);
     for (auto& e : E->ev)
         if (e) cudaEventDestroy(e);
     if (E->stream) cudaStreamDestroy(E->stream);
@@ -1587,6 +1801,7 @@ int mdx_ensemble_ic(mdx_ensemble_t* E) {
     std::vector<ens_state> hs(E->n);
     std::memset(hs.data(), 0, sizeof(ens_state) * E->n);
     ENS_CUDA(E, cudaMemcpyAsync(E->dst, hs.data(), sizeof(ens_state) * E->n, cudaMemcpyHostToDevice, E->stream));
+    MDX_TRY(res_prepare(E, E->variant, E->threads, E->grid, 1));
     MDX_TRY(launch_substage(E, 0, 0, E->variant, E->threads, E->grid));   // the t=0 projection, dt_gamma = 1
     for (int m = 0; m < E->n; ++m)
         ENS_CUDA(E, cudaMemsetAsync(E->hm[m].pn, 0, sizeof(double) * E->hm[m].d.npad, E->stream));
@@ -1714,6 +1929,7 @@ int mdx_ensemble_step(mdx_ensemble_t* E, int nsteps, long long* total_iters) {
     MDX_TRY(read_stats(E, before));
     ENS_CUDA(E, cudaEventRecord(E->ev[0], E->stream));
     for (int q = 0; q < nsteps; ++q) {
+        MDX_TRY(res_prepare(E, E->variant, E->threads, E->grid, 3));
         if (E->use_graph && E->graph_ok && !E->graph) {
             cudaGraph_t g = nullptr;
             ENS_CUDA(E, cudaStreamBeginCapture(E->stream, cudaStreamCaptureModeThreadLocal));
@@ -1749,7 +1965,8 @@ int mdx_ensemble_step(mdx_ensemble_t* E, int nsteps, long long* total_iters) {
     }
     if (total_iters) *total_iters = it;
     if (bad >= 0)
-        return efail(E, after[bad].status == MDX_ERR_NONFINITE ? MDX_ERR_NONFINITE : MDX_NOT_CONVERGED,
+        return efail(E, after[bad].status == MDX_ERR_NONFINITE ? MDX_ERR_NONFINITE
+                        : after[bad].status == MDX_ERR_TIMEOUT ? MDX_ERR_TIMEOUT : MDX_NOT_CONVERGED,
                      "member %d: last projection status %d", bad, after[bad].status);
     return MDX_OK;
 }
@@ -1826,6 +2043,7 @@ int mdx_ensemble_tune(mdx_ensemble_t* E, const char* cache_path, int* threads_ou
                 MDX_TRY(grid_for(E, v, cand_t[ti], cand_b[bi], &grid));
                 MDX_TRY(snapshot(E, true));
                 ENS_CUDA(E, cudaEventRecord(E->ev[0], E->stream));
+                MDX_TRY(res_prepare(E, v, cand_t[ti], grid, 3));
                 MDX_TRY(step_eager(E, v, cand_t[ti], grid));
                 ENS_CUDA(E, cudaEventRecord(E->ev[1], E->stream));
                 ENS_CUDA(E, cudaEventSynchronize(E->ev[1]));
