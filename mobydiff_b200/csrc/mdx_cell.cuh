@@ -133,6 +133,10 @@ struct mdx_mom_nb {
     MDX_MOM_STENCIL(MDX_MOM_GET)
 #undef MDX_MOM_FIELD
 #undef MDX_MOM_GET
+    double ou_v, ov_v, ow_v;   // the stored right-hand sides
+    __device__ __forceinline__ double ou_old(const double*, long long) const { return ou_v; }
+    __device__ __forceinline__ double ov_old(const double*, long long) const { return ov_v; }
+    __device__ __forceinline__ double ow_old(const double*, long long) const { return ow_v; }
 };
 struct mdx_mom_ld {
     const double *un, *vn, *wn, *pn;
@@ -168,6 +172,9 @@ struct mdx_mom_ld {
     __device__ __forceinline__ double p_im() const { return __ldg(pn + c - SX); }
     __device__ __forceinline__ double p_jm() const { return __ldg(pn + c - SY); }
     __device__ __forceinline__ double p_km() const { return __ldg(pn + c - SZ); }
+    __device__ __forceinline__ double ou_old(const double* o, long long q) const { return o[q]; }
+    __device__ __forceinline__ double ov_old(const double* o, long long q) const { return o[q]; }
+    __device__ __forceinline__ double ow_old(const double* o, long long q) const { return o[q]; }
 };
 
 // The predictor of one cell (i,j,k), src/modules/step.f90:76-204, from its
@@ -201,7 +208,7 @@ __device__ __forceinline__ void momentum_vals(const NB& n, const mdx_step_params
         const double dpx = (p_c - n.p_im()) * idx;
         const double rhsu = -((uu_p - uu_m) * idx) - (uv_p - uv_m) * idy - (uw_p - uw_m) * idz + p.fx +
                             ire * (diff_ux + diff_uy + diff_uz);
-        double val = u_c + dt_alpha * rhsu + dt_beta * ou[q] - dt_gamma * dpx;
+        double val = u_c + dt_alpha * rhsu + dt_beta * n.ou_old(ou, q) - dt_gamma * dpx;
         if (IBM) val = val * (1.0 / (1.0 + dt_gamma * __ldg(cu + cc)));
         us[c] = val;
         ou[q] = rhsu;
@@ -223,7 +230,7 @@ __device__ __forceinline__ void momentum_vals(const NB& n, const mdx_step_params
         const double dpy = (p_c - n.p_jm()) * idy;
         const double rhsv = -((vu_p - vu_m) * idx) - (vv_p - vv_m) * idy - (vw_p - vw_m) * idz + p.fy +
                             ire * (diff_vx + diff_vy + diff_vz);
-        double val = v_c + dt_alpha * rhsv + dt_beta * ov[q] - dt_gamma * dpy;
+        double val = v_c + dt_alpha * rhsv + dt_beta * n.ov_old(ov, q) - dt_gamma * dpy;
         if (IBM) val = val * (1.0 / (1.0 + dt_gamma * __ldg(cv + cc)));
         vs[c] = val;
         ov[q] = rhsv;
@@ -245,7 +252,7 @@ __device__ __forceinline__ void momentum_vals(const NB& n, const mdx_step_params
         const double dpz = (p_c - n.p_km()) * idz;
         const double rhsw = -((wu_p - wu_m) * idx) - (wv_p - wv_m) * idy - (ww_p - ww_m) * idz + p.fz +
                             ire * (diff_wx + diff_wy + diff_wz);
-        double val = w_c + dt_alpha * rhsw + dt_beta * ow[q] - dt_gamma * dpz;
+        double val = w_c + dt_alpha * rhsw + dt_beta * n.ow_old(ow, q) - dt_gamma * dpz;
         if (IBM) val = val * (1.0 / (1.0 + dt_gamma * __ldg(cw + cc)));
         ws[c] = val;
         ow[q] = rhsw;

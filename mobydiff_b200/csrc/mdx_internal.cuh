@@ -325,6 +325,7 @@ cudaError_t mdx_launch_chained(cudaStream_t st, void (*kernel)(P...), dim3 grid,
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 #ifdef __CUDACC__
+__device__ __forceinline__ void prefetch_l2(const void* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 // What ran before is complete and visible / the next kernel's blocks may be
 // placed.
 __device__ __forceinline__ void mdx_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
