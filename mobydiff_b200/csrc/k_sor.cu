@@ -332,11 +332,15 @@ double mdx_div_floor(const mdx_ctx_t* ctx, double umax) {
 // One colour sweep for periodic x and z (the configurations of every run
 // here): boundary flags are compile-time constants, in-plane offsets are
 // 32-bit, and registers are bounded for occupancy.
-template <int MU, int PY>
+// FIRST: the faces are read from u*, v*, w* and written to u, v, w, in place
+// of the copy that starts a projection: a sweep of one colour touches every
+// face between two cells, and k_shell_copy sets the rest before it.
+template <int MU, int PY, bool FIRST>
 __global__ void __launch_bounds__(256, 4)
 k_sor_sweep_pxz(mdx_dims d, mdx_bc_dev bc, mdx_sor_params p, int parity, int reverse, double* __restrict__ un,
                 double* __restrict__ vn, double* __restrict__ wn, double* __restrict__ pn,
-                const double* __restrict__ mu) {
+                const double* __restrict__ mu, const double* __restrict__ us, const double* __restrict__ vs,
+                const double* __restrict__ ws) {
     const int ni = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int kk = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -362,7 +366,22 @@ k_sor_sweep_pxz(mdx_dims d, mdx_bc_dev bc, mdx_sor_params p, int parity, int rev
         mu_v_jp = __ldg(mu + plane + qjp);
         mu_w = __ldg(mu + 2 * plane + q);
     }
-    double u_i = U[q], u_ip = U[qip], v_j = Vv[q], v_jp = Vv[qjp], w_k = W[q], w_kp = Wn[q], pc = Pp[q];
+    double u_i, u_ip, v_j, v_jp, w_k, w_kp, pc = Pp[q];
+    if (FIRST) {
+        u_i = __ldg(us + k * plane + q);
+        u_ip = __ldg(us + k * plane + qip);
+        v_j = __ldg(vs + k * plane + q);
+        v_jp = __ldg(vs + k * plane + qjp);
+        w_k = __ldg(ws + k * plane + q);
+        w_kp = __ldg(ws + kp * plane + q);
+    } else {
+        u_i = U[q];
+        u_ip = U[qip];
+        v_j = Vv[q];
+        v_jp = Vv[qjp];
+        w_k = W[q];
+        w_kp = Wn[q];
+    }
     const double fac = sor_factor(mu_u_i, mu_u_ip, mu_v_j, mu_v_jp, mu_w, mu_w, p);
     sor_cell_fac<1, PY, 1>(u_i, u_ip, v_j, v_jp, w_k, w_kp, pc, mu_u_i, mu_u_ip, mu_v_j, mu_v_jp, mu_w, mu_w, fac, p,
                            bc, i, j, k, nx, ny, nz);
@@ -373,6 +392,35 @@ k_sor_sweep_pxz(mdx_dims d, mdx_bc_dev bc, mdx_sor_params p, int parity, int rev
     W[q] = w_k;
     Wn[q] = w_kp;
     Pp[q] = pc;
+}
+
+// u, v, w <- u*, v*, w* where no cell pair's face lies: the ghost layers and
+// the wall rows v(1), v(ny+1).  Faces of the box as in k_bc_fft.
+__global__ void k_shell_copy(mdx_dims d, double* __restrict__ un, double* __restrict__ vn, double* __restrict__ wn,
+                             const double* __restrict__ us, const double* __restrict__ vs,
+                             const double* __restrict__ ws) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
+    auto put = [&](int i, int j, int k) {
+        const long long c = pidx(d, i, j, k);
+        un[c] = us[c];
+        vn[c] = vs[c];
+        wn[c] = ws[c];
+    };
+    if (blockIdx.z == 0) {
+        if (a > d.nx + 1 || b > d.ny + 1) return;
+        put(a, b, 0);
+        put(a, b, d.nz + 1);
+    } else if (blockIdx.z == 1) {
+        if (a > d.nx + 1 || b >= d.nz) return;
+        put(a, 0, b + 1);
+        put(a, d.ny + 1, b + 1);
+        const long long c = pidx(d, a, 1, b + 1);
+        vn[c] = vs[c];
+    } else {
+        if (a >= d.ny || b >= d.nz) return;
+        put(0, a + 1, b + 1);
+        put(d.nx + 1, a + 1, b + 1);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -594,21 +642,35 @@ static mdx_sor_params sor_params(const mdx_ctx_t* ctx, double dg) {
     return p;
 }
 
-static int sor_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p) {
+static bool sor_pxz(const mdx_ctx_t* ctx) {
+    return ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL;
+}
+
+// first: u, v, w are not set yet, the red sweep reads u*, v*, w* (sor_pxz only).
+static int sor_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p, bool first = false) {
     const mdx_dims& d = ctx->d;
     double** f = ctx->f;
     const int na = d.nx / 2;
     dim3 block(32, 4, 2);
     dim3 grid((na + 31) / 32, (d.ny + 3) / 4, (d.nz + 1) / 2);
-    const bool pxz = ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL;
+    const bool pxz = sor_pxz(ctx);
     const bool py = ctx->bc.is_periodic[1] != 0;
+    if (first)
+        MDX_LAUNCH(ctx, MDX_T_OTHER, "shell copy", k_shell_copy,
+                   dim3((std::max(d.nxp, d.ny) + 31) / 32, (std::max(d.nyp, d.nz) + 7) / 8, 3), dim3(32, 8), 0, d,
+                   f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_US], f[MDX_VS], f[MDX_WS]);
     for (int parity = 0; parity < 2; ++parity) {
         const int rev = parity;   // red sweeps walk k up, black sweeps walk k down
         if (pxz) {
-            auto kfn = ctx->mu_mode == MU_PLANE ? (py ? k_sor_sweep_pxz<MU_PLANE, 1> : k_sor_sweep_pxz<MU_PLANE, 0>)
-                                                : (py ? k_sor_sweep_pxz<MU_ONE, 1> : k_sor_sweep_pxz<MU_ONE, 0>);
+            auto kfn = ctx->mu_mode == MU_PLANE
+                           ? (py ? k_sor_sweep_pxz<MU_PLANE, 1, false> : k_sor_sweep_pxz<MU_PLANE, 0, false>)
+                           : (py ? k_sor_sweep_pxz<MU_ONE, 1, false> : k_sor_sweep_pxz<MU_ONE, 0, false>);
+            if (first && parity == 0)
+                kfn = ctx->mu_mode == MU_PLANE
+                          ? (py ? k_sor_sweep_pxz<MU_PLANE, 1, true> : k_sor_sweep_pxz<MU_PLANE, 0, true>)
+                          : (py ? k_sor_sweep_pxz<MU_ONE, 1, true> : k_sor_sweep_pxz<MU_ONE, 0, true>);
             MDX_LAUNCH(ctx, MDX_T_SOR_SWEEP, "sor sweep", kfn, grid, block, 0, d, ctx->bcd, p, parity, rev,
-                       f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN], ctx->mu);
+                       f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN], ctx->mu, f[MDX_US], f[MDX_VS], f[MDX_WS]);
         } else if (ctx->mu_mode == MU_ONE)
             MDX_LAUNCH(ctx, MDX_T_SOR_SWEEP, "sor sweep", k_sor_sweep<MU_ONE>, grid, block, 0, d, ctx->bcd, p, parity,
                        rev, f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_PN], ctx->mu);
@@ -797,12 +859,30 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     const mdx_dims& d = ctx->d;
     double** f = ctx->f;
     const size_t bytes = sizeof(double) * d.npad;
-    // :63-84 -- u <- u* over the whole padded arrays
-    MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_UN], f[MDX_US], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_VN], f[MDX_VS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_WN], f[MDX_WS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     MDX_TRY(mu_tables(ctx, dg));
     const mdx_solver_opts_t& o = ctx->opts;
+    // kernel variant: the requested one, the tuned one, or -- while tuning --
+    // the next untried candidate for each residual-check block
+    const bool fok = fused_ok(ctx);
+    int want = ctx->opts.sor_variant;
+    if (want < MDX_SORV_AUTO || want > MDX_SORV_RESIDENT) want = MDX_SORV_AUTO;
+    // where the state fits the SMs the on-chip run is taken without tuning:
+    // it was the fastest on every such grid measured
+    if ((want == MDX_SORV_AUTO || want == MDX_SORV_RESIDENT))
+        want = mdx_res_face64_ok(ctx) ? MDX_SORV_RESIDENT : MDX_SORV_AUTO;
+    if (want != MDX_SORV_SWEEPS && !fok) want = MDX_SORV_SWEEPS;
+    const bool warm = mdx_guess_supported(ctx) && (ctx->guess_mode != MDX_GUESS_ZERO || ctx->record_increments);
+    // :63-84 -- u <- u* over the whole padded arrays; a fixed number of plain
+    // sweeps does it in its first sweep (three copies of 30 MB, 35 us, on
+    // 180x150x140)
+    const int fixed_v = want == MDX_SORV_AUTO && ctx->sor_tuned > 0 ? ctx->sor_tuned : want;
+    const bool copy_in_sweep = o.tol <= 0.0 && o.n_iter > 0 && !warm && sor_pxz(ctx) &&
+                               (fixed_v == MDX_SORV_AUTO || fixed_v == MDX_SORV_SWEEPS);
+    if (!copy_in_sweep) {
+        MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_UN], f[MDX_US], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_VN], f[MDX_VS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_WN], f[MDX_WS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    }
     // Residual scale of this projection, on u* before any guess: converged
     // when ||div u|| <= max(tol*||div u*||, atol); the default atol is the
     // round-off level of the divergence, below which a relative target
@@ -815,7 +895,6 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
         target = std::max(o.tol * r0, atol);
     }
     // warm start: record this projection's increment; apply a guess
-    const bool warm = mdx_guess_supported(ctx) && (ctx->guess_mode != MDX_GUESS_ZERO || ctx->record_increments);
     if (warm) MDX_TRY(mdx_warm_begin(ctx));
     bool guessed = false;
     double rg = r0;   // ||div u|| after the guess
@@ -830,16 +909,6 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
             return MDX_OK;
         }
     }
-    // kernel variant: the requested one, the tuned one, or -- while tuning --
-    // the next untried candidate for each residual-check block
-    const bool fok = fused_ok(ctx);
-    int want = ctx->opts.sor_variant;
-    if (want < MDX_SORV_AUTO || want > MDX_SORV_RESIDENT) want = MDX_SORV_AUTO;
-    // where the state fits the SMs the on-chip run is taken without tuning:
-    // it was the fastest on every such grid measured
-    if ((want == MDX_SORV_AUTO || want == MDX_SORV_RESIDENT))
-        want = mdx_res_face64_ok(ctx) ? MDX_SORV_RESIDENT : MDX_SORV_AUTO;
-    if (want != MDX_SORV_SWEEPS && !fok) want = MDX_SORV_SWEEPS;
     const bool splitv = want == MDX_SORV_AUTO || want == MDX_SORV_SPLITV;
     if (want == MDX_SORV_AUTO || want == MDX_SORV_SPLIT || splitv) MDX_TRY(split_alloc(ctx));
     const mdx_sor_params p = sor_params(ctx, dg);
@@ -877,8 +946,9 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
         MDX_TRY(layout_for(v));
         mdx_event_pair run{};
         mdx_sweep_run_begin(ctx, &run);
-        MDX_TRY(sor_iterations(ctx, p, v, o.n_iter));
-        mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT ? 2LL * o.n_iter : -1);
+        if (copy_in_sweep) MDX_TRY(sor_iteration(ctx, p, true));
+        MDX_TRY(sor_iterations(ctx, p, v, o.n_iter - (copy_in_sweep ? 1 : 0)));
+        mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT || copy_in_sweep ? 2LL * o.n_iter : -1);
         MDX_TRY(layout_for(MDX_SORV_SWEEPS));
         s.variant = v;
         s.iterations = o.n_iter;
