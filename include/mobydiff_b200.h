@@ -96,8 +96,9 @@ typedef struct {
                           FP32), one launch per run of sweeps with the state on chip;
                           else the first projection times each variant on one residual-check
                           block of its own iterations and keeps the fastest; 1 one
-                          launch per colour; 2 fused red+black pass, 32x8 tiles;
-                          3 fused pass, 32x16 tiles; 4 one launch per colour on
+                          launch per colour; 2 red+black pass, 60x5 tiles; 3 the same,
+                          60x17 or (IBM factors) 60x13 tiles, which 0 takes for a
+                          fixed count on large grids; 4 one launch per colour on
                           colour-split copies of u, v, w, p made once per projection;
                           5 the same with two cells per thread and 16-byte accesses
                           (2-5: periodic x and z, IBM factors 1 or z-invariant);
@@ -111,7 +112,8 @@ typedef struct {
                           form (inner_form 0 or 2): 1-15 pin one shape of its sweep
                           kernels, 0 the fastest of those the grid allows (all give the
                           same bits), 16 the on-chip run */
-    int sor_kz;        /* z planes per block of the fused pass (0: default 16) */
+    int sor_kz;        /* z planes per block of the FP64 red+black pass (0: the count
+                          that fills the GPU best) */
     int check_mode;    /* red-black, tol > 0: 0 (default) residual checks at multiples of check_every,
                           up to 8 blocks apart while the residual falls at a steady rate that
                           puts the target more than twice as far; 1: every check_every

@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 // mu = 1/(1 + dt_gamma*coef) over n elements of each component.
 __global__ void k_mu_tables(long long n, double dg, const double* __restrict__ cu, const double* __restrict__ cv,
@@ -89,238 +90,254 @@ k_sor_sweep(mdx_dims d, mdx_bc_dev bc, mdx_sor_params p, int parity, int reverse
 // ---------------------------------------------------------------------------
 // One full red+black iteration in one pass (periodic x and z).
 //
-// Each block owns the cells of a TX x TY tile in x-y and a chunk of KZ z
-// planes.  It walks its z range with a ring of four planes in shared memory
-// holding u, v, w, p of the tile plus a two-cell halo ring in x and y; the
-// plane two ahead is fetched with cp.async while the current ones compute.
-// On plane q it runs the red update on every red cell of the halo region,
-// then the black update of plane q-1 on the tile plus a one-cell ring, then
-// writes the owned faces of plane q-1 (u(i), v(j), w(k) and p of the tile
-// cells; v(ny+1) for a y wall).  All reads come from the old state (u0..p0)
-// and all writes go to the new state (u1..p1), so blocks never see each
-// other's updates; red cells of the halo are recomputed from the same old
-// values their owners use, so every face ends with exactly the value of a
-// red sweep followed by a black sweep.  The state crosses HBM once per
-// iteration instead of twice.
+// A block owns 60 x (RY-3) columns of cells and a chunk of KZ planes and
+// walks it in z.  u, v, w are read from one state and written to another, so
+// blocks never see each other's updates; a block recomputes its halo (two
+// cells below, one above, in every direction) from the values their owners
+// use, so every face ends with the value of a red sweep followed by a black
+// one, bit for bit.  p belongs to one cell and is updated in place.
 //
-// Shared-memory rows store even columns then odd columns, so the cells of
-// one colour in a row (every other column) are contiguous: a warp's accesses
-// fall in distinct banks.
+// A warp is one row of 64 cells, a lane two neighbouring ones.  The red cells
+// of plane m+2 and the black cells of plane m do not depend on each other and
+// lie in different columns of a lane's two: a phase updates both, with one
+// barrier.  u and v, which neighbours share, are in a ring of six planes in
+// shared memory (m-1 on its way out, m .. m+2 in work, m+3 and m+4 in flight,
+// cp.async); w and p stay with their columns, in registers, read and written
+// 16 bytes a lane.  Rows store even cells, then odd cells: one colour of a
+// row is contiguous, and so is a fetch.
+//
+// A colour sweep each moves u, v, w, p twice through HBM: 78 us an iteration
+// of 180x150x140, at 6.2 TB/s.  A pass moves them once: 59 us (DRAM at 43 %,
+// shared-memory pipe at 52 %; the chain of a phase, shared memory - 12 FP64
+// operations - shared memory - barrier, is what is left).  On the way: slots
+// and plane numbers by remainders 90, 20 registers' worth of values moved
+// along each phase 88, w and p a lane at a time and selected as soon as read
+// 97, selected a phase later 62.  Its predecessor, u, v, w, p in shared
+// memory and four barriers a plane, took 254.
+// RY: 20 rows where the factors are 1 (94 registers), 16 with factors per
+// column (20 would spill: 111 against 63 us); 8 for MDX_SORV_FUSED8.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    const int n = valid ? 8 : 0;   // 0 source bytes: the 8 destination bytes are zero-filled
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
-template <int TX, int TY, int NTH>
-struct fused_geom {
-    static constexpr int NT = NTH;
-    static constexpr int WX = TX + 3, WY = TY + 3;   // halo: x in [x0-2, x0+TX], y in [y0-2, y0+TY]
-    static constexpr int UX = WX + 1;                // u rows also hold the right face of the last cell
-    static constexpr int H = (UX + 1) / 2;           // even columns, then odd columns
-    static constexpr int R = 2 * H;                  // row stride
-    static constexpr int NU = WY * R, NV = (WY + 1) * R, NC = WY * R;
-    static constexpr int SLOT = NU + NV + 2 * NC;
-    static constexpr int LU = WY * UX, LV = (WY + 1) * WX, LC = WY * WX;   // elements fetched per plane
-    static constexpr int LTOT = LU + LV + 2 * LC;
-    static constexpr int NLD = (LTOT + NT - 1) / NT;
-    static constexpr int HR = (WX + 1) / 2;          // red candidates per row
-    static constexpr int HB = (WX - 1) / 2;          // black candidates per row (columns 1..WX-2)
-    __device__ static __forceinline__ int col(int lx) { return (lx & 1) * H + (lx >> 1); }
+constexpr int PASS_TX = 60, PASS_SLOTS = 6;
+constexpr int PASS_H = 40, PASS_R = 72;   // a row: even cells from 0, odd cells from PASS_H (other banks)
+template <int RY> struct pass_geom {
+    static constexpr int TY = RY - 3;
+    static constexpr int NU = RY * PASS_R, NV = (RY + 1) * PASS_R, SLOT = NU + NV;
+    static constexpr size_t SMEM = sizeof(double) * PASS_SLOTS * SLOT;
 };
 
-template <int MU, int PY, int TX, int TY, int NTH>
-__global__ void __launch_bounds__(NTH)
-k_sor_fused(mdx_dims d, mdx_bc_dev bc, mdx_sor_params P, int KZ, const double* __restrict__ u0,
-            const double* __restrict__ v0, const double* __restrict__ w0, const double* __restrict__ p0,
-            double* __restrict__ u1, double* __restrict__ v1, double* __restrict__ w1, double* __restrict__ p1,
-            const double* __restrict__ mu) {
-    using G = fused_geom<TX, TY, NTH>;
-    constexpr int NT = G::NT, WX = G::WX, WY = G::WY, UX = G::UX, R = G::R;
-    constexpr int NU = G::NU, NV = G::NV, NC = G::NC, SLOT = G::SLOT;
-    constexpr int LU = G::LU, LV = G::LV, LC = G::LC, LTOT = G::LTOT, NLD = G::NLD;
-    constexpr int HR = G::HR, HB = G::HB;
-    static_assert(WY * HR <= NT && (WY - 2) * HB <= NT && TX * TY <= NT, "one cell per thread per phase");
+template <int MU, int PY, int RY>
+__global__ void __launch_bounds__(32 * RY, RY == 8 ? 2 : 1)
+k_sor_pass(mdx_dims d, mdx_bc_dev bc, mdx_sor_params P, int KZ, const double* __restrict__ u0,
+           const double* __restrict__ v0, const double* __restrict__ w0, double* __restrict__ u1,
+           double* __restrict__ v1, double* __restrict__ w1, double* __restrict__ pn,
+           const double* __restrict__ mu) {
+    using G = pass_geom<RY>;
     extern __shared__ double sm[];
-    double* smu = sm + 4 * SLOT;              // mu_u (NU), mu_v (NV), mu_w (NC)  [MU_PLANE]
-    double* sfac = smu + (MU == MU_PLANE ? NU + NV + NC : 0);   // -omega/denom per column (NC)
-    int* gxt = (int*)(sfac + NC);             // global x of local column (UX)
-    int* gyt = gxt + UX;                      // global y of local row (WY+1), -1 outside
-
     const int nx = d.nx, ny = d.ny, nz = d.nz;
-    const int x0 = blockIdx.x * TX + 1, y0 = blockIdx.y * TY + 1;
-    const int k0 = blockIdx.z * KZ + 1;
-    const int k1 = min(k0 + KZ, nz + 1);
-    const int tid = threadIdx.x;
-    const long long plane = (long long)d.nxp * d.nyp;
+    const int l = threadIdx.x & 31, r = threadIdx.x >> 5;
+    const int x0 = blockIdx.x * PASS_TX + 1, y0 = blockIdx.y * G::TY + 1, k0 = blockIdx.z * KZ + 1;
+    const int k1 = min(k0 + KZ - 1, nz);
+    const unsigned plane = (unsigned)(d.nxp * d.nyp);   // offsets into an array: 32 bits (pass_fits)
+    auto wrapx = [&](int c) { return ((x0 - 4 + c) % nx + nx) % nx + 1; };          // cell c of the row
+    auto rowy = [&](int q) {                                                         // row q of the tile
+        const int g = y0 - 2 + q;
+        return PY ? ((g - 1) % ny + ny) % ny + 1 : min(max(g, 0), ny + 1);
+    };
+    const int j = y0 - 2 + r, gj = rowy(r);
+    const bool row_in = PY || (j >= 1 && j <= ny);
 
-    for (int t = tid; t < UX; t += NT) gxt[t] = ((x0 - 2 + t - 1) % nx + nx) % nx + 1;
-    for (int t = tid; t <= WY; t += NT) {
-        int g = y0 - 2 + t;
-        if (PY) g = ((g - 1) % ny + ny) % ny + 1;
-        else if (g < 0 || g > ny + 1) g = -1;
-        gyt[t] = g;
+    // fetched and written as cells l and l + 32 of a row, which are contiguous
+    const unsigned f0 = wrapx(l) + d.nxp * gj, f1 = wrapx(l + 32) + d.nxp * gj;
+    const unsigned fx = wrapx(64) + d.nxp * gj;             // the face right of the last cell
+    const unsigned h = d.nxp * (rowy(RY) - gj);             // from row 0 of the tile to row RY
+    const int t0 = r * PASS_R + (l & 1) * PASS_H + (l >> 1), t1 = t0 + 16;   // their places in a plane
+    auto fetch = [&](int slot, unsigned o) {
+        double* s = sm + slot * G::SLOT;
+        cp_async8(s + t0, u0 + (o + f0));
+        cp_async8(s + t1, u0 + (o + f1));
+        if (l == 0) cp_async8(s + r * PASS_R + 32, u0 + (o + fx));
+        cp_async8(s + G::NU + t0, v0 + (o + f0));
+        cp_async8(s + G::NU + t1, v0 + (o + f1));
+        if (r == 0) {
+            cp_async8(s + G::NU + RY * PASS_R + t0, v0 + (o + f0 + h));
+            cp_async8(s + G::NU + RY * PASS_R + t1, v0 + (o + f1 + h));
+        }
+    };
+
+    // The lane's cells are 2l and 2l + 1, x = x0-3+2l even: 16 bytes together
+    // but where the period ends between them.  Column A is red on planes of
+    // k0's parity, column B on the others; a: A is the second cell.
+    const int a = (j + k0 + 1) & 1, cA = 2 * l + a, cB = 2 * l + 1 - a;
+    const int xe = x0 - 3 + 2 * l;
+    const bool ends = wrapx(2 * l) == nx;
+    const unsigned ge = (xe >= 0 && xe <= nx ? xe : wrapx(2 * l)) + d.nxp * gj;
+    const unsigned g0 = wrapx(2 * l) + d.nxp * gj, g1 = wrapx(2 * l + 1) + d.nxp * gj;
+    const bool own_row = row_in && r >= 2 && r <= RY - 2 && j <= ny;
+    auto owned = [&](int c) { return own_row && c >= 3 && c <= 62 && x0 - 3 + c <= nx; };
+    const bool o0 = owned(2 * l), o1 = owned(2 * l + 1), own = o0 || o1;
+    const bool full = o0 && o1;
+    auto put2 = [&](double* q, unsigned o, double x, double y, auto FULL) {
+        if (FULL) *reinterpret_cast<double2*>(q + (o + ge)) = make_double2(x, y);
+        else if (o0) q[o + ge] = x;
+        else q[o + ge + 1] = y;
+    };
+    auto get_w = [&](unsigned o) {
+        if (!ends) return __ldg(reinterpret_cast<const double2*>(w0 + (o + ge)));
+        return make_double2(__ldg(w0 + (o + g0)), __ldg(w0 + (o + g1)));
+    };
+    auto get_p = [&](unsigned o) { return *reinterpret_cast<const double2*>(pn + (o + ge)); };
+    auto to_cols = [&](double2 t, double& A, double& B) {
+        A = a ? t.y : t.x;
+        B = a ? t.x : t.y;
+    };
+    const bool wall = !PY && j == ny;
+    struct factors { double u_i, u_ip, v_j, v_jp, w, fac; };
+    auto column = [&](int c) {
+        factors m{1.0, 1.0, 1.0, 1.0, 1.0, 0.0};
+        const unsigned g = wrapx(c) + d.nxp * gj;
+        if (MU == MU_PLANE) {
+            m.u_i = __ldg(mu + g);
+            m.u_ip = __ldg(mu + wrapx(c + 1) + d.nxp * gj);
+            m.v_j = __ldg(mu + plane + g);
+            m.v_jp = __ldg(mu + plane + wrapx(c) + d.nxp * rowy(r + 1));
+            m.w = __ldg(mu + 2 * plane + g);
+        }
+        m.fac = sor_factor(m.u_i, m.u_ip, m.v_j, m.v_jp, m.w, m.w, P);
+        return m;
+    };
+    const factors FA = column(cA), FB = column(cB);
+    // places in a plane of the columns' faces and of cell c + 1's
+    const int sA = r * PASS_R + a * PASS_H + l, sB = r * PASS_R + (1 - a) * PASS_H + l;
+    const int nA = a ? r * PASS_R + l + 1 : sB, nB = a ? sA : r * PASS_R + l + 1;
+    struct faces { double u_i, u_ip, v_j, v_jp; };
+    auto get = [&](int slot, int s0, int s1) {
+        const double *su = sm + slot * G::SLOT, *sv = su + G::NU;
+        return faces{su[s0], su[s1], sv[s0], sv[s0 + PASS_R]};
+    };
+    auto put = [&](int slot, int s0, int s1, const faces& f) {
+        double *su = sm + slot * G::SLOT, *sv = su + G::NU;
+        su[s0] = f.u_i;
+        su[s1] = f.u_ip;
+        sv[s0] = f.v_j;
+        sv[s0 + PASS_R] = f.v_jp;
+    };
+    auto update = [&](faces& f, const factors& m, double& wk, double& wkp, double& pc) {
+        sor_cell_fac<1, PY, 1>(f.u_i, f.u_ip, f.v_j, f.v_jp, wk, wkp, pc, m.u_i, m.u_ip, m.v_j, m.v_jp, m.w, m.w,
+                               m.fac, P, bc, 0, j, 0, nx, ny, nz);
+    };
+    auto cell = [&](int slot, int s0, int s1, const factors& m, double& wk, double& wkp, double& pc) {
+        faces f = get(slot, s0, s1);
+        update(f, m, wk, wkp, pc);
+        put(slot, s0, s1, f);
+    };
+    auto put_uv = [&](int slot, unsigned o, auto FULL) {
+        const double* su = sm + slot * G::SLOT + r * PASS_R + l;
+        const double* sv = su + G::NU;
+        put2(u1, o, su[0], su[PASS_H], FULL);
+        put2(v1, o, sv[0], sv[PASS_H], FULL);
+        if (wall) put2(v1, o + d.nxp, sv[PASS_R], sv[PASS_R + PASS_H], FULL);
+    };
+    // Plane k is in slot (k - k0 + 2) mod 6 and its w and p in entry (k - k0 + 1)
+    // mod 6: the loop is unrolled by 6 so that both are constants.
+    const unsigned top = (unsigned)nz * plane;
+    auto next = [&](unsigned o) { return o == top ? plane : o + plane; };
+    unsigned o = (unsigned)(((k0 - 3) % nz + nz) % nz + 1) * plane;   // plane k0-2
+    double wA[6], wB[6], pA[6], pB[6], wl, none = 0.0;
+    double2 wq[5], wnext, pnext = make_double2(0.0, 0.0), p0 = pnext;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {   // planes k0-2 .. k0+2
+        if (k0 - 2 + q <= k1 + 1) fetch(q, o);
+        cp_async_commit();
+        wq[q] = get_w(o);
+        o = next(o);
+    }
+    unsigned om = (unsigned)k0 * plane - plane;   // plane k0-1
+    if (own) {
+        p0 = get_p(om + plane);
+        if (k0 + 1 <= k1) pnext = get_p(om + 2 * plane);
+    }
+    to_cols(wq[0], wl, none);
+    none = 0.0;
+    to_cols(wq[1], wA[0], wB[0]);
+    to_cols(wq[2], wA[1], wB[1]);
+    to_cols(wq[3], wA[2], wB[2]);
+    wnext = wq[4];
+    pA[0] = pB[0] = 0.0;
+    to_cols(p0, pA[1], pB[1]);
+    cp_async_wait<1>();   // planes up to k0 + 1
+    __syncthreads();
+    if (row_in) {   // red cells of planes k0-2, k0-1, k0
+        cell(0, sA, nA, FA, wl, wA[0], none);
+        cell(1, sB, nB, FB, wB[0], wB[1], none);
+        cell(2, sA, nA, FA, wA[1], wA[2], pA[1]);
     }
     __syncthreads();
-    if (MU == MU_PLANE) {
-        for (int t = tid; t < LU; t += NT) {
-            const int ly = t / UX, lx = t - ly * UX, gy = gyt[ly];
-            smu[ly * R + G::col(lx)] = gy >= 0 ? __ldg(mu + gxt[lx] + (long long)d.nxp * gy) : 1.0;
-        }
-        for (int t = tid; t < LV; t += NT) {
-            const int ly = t / WX, lx = t - ly * WX, gy = gyt[ly];
-            smu[NU + ly * R + G::col(lx)] = gy >= 0 ? __ldg(mu + plane + gxt[lx] + (long long)d.nxp * gy) : 1.0;
-        }
-        for (int t = tid; t < LC; t += NT) {
-            const int ly = t / WX, lx = t - ly * WX, gy = gyt[ly];
-            smu[NU + NV + ly * R + G::col(lx)] =
-                gy >= 0 ? __ldg(mu + 2 * plane + gxt[lx] + (long long)d.nxp * gy) : 1.0;
-        }
-        __syncthreads();
-    }
-    // -omega/denom of every column (:124-126,186); z-invariant in both modes
-    for (int t = tid; t < LC; t += NT) {
-        const int ly = t / WX, lx = t - ly * WX;
-        double mu_u_i = 1.0, mu_u_ip = 1.0, mu_v_j = 1.0, mu_v_jp = 1.0, mu_w = 1.0;
-        if (MU == MU_PLANE) {
-            mu_u_i = smu[ly * R + G::col(lx)];
-            mu_u_ip = smu[ly * R + G::col(lx + 1)];
-            mu_v_j = smu[NU + ly * R + G::col(lx)];
-            mu_v_jp = smu[NU + (ly + 1) * R + G::col(lx)];
-            mu_w = smu[NU + NV + ly * R + G::col(lx)];
-        }
-        sfac[ly * R + G::col(lx)] = sor_factor(mu_u_i, mu_u_ip, mu_v_j, mu_v_jp, mu_w, mu_w, P);
-    }
 
-    // Per-thread fetch descriptors: plane-relative global offset (-1 outside
-    // the domain: zero-filled) and the shared-memory index in a slot.
-    int ldoff[NLD], lddst[NLD];
-#pragma unroll
-    for (int m = 0; m < NLD; ++m) {
-        const int e = tid + m * NT;
-        int off = -1, dst = -1;
-        if (e < LTOT) {
-            int lx, ly, base;
-            if (e < LU) {
-                ly = e / UX;
-                lx = e - ly * UX;
-                base = 0;
-            } else if (e < LU + LV) {
-                const int t = e - LU;
-                ly = t / WX;
-                lx = t - ly * WX;
-                base = NU;
-            } else {
-                const int t = e - LU - LV;
-                const int t2 = t < LC ? t : t - LC;
-                ly = t2 / WX;
-                lx = t2 - ly * WX;
-                base = t < LC ? NU + NV : NU + NV + NC;
-            }
-            dst = base + ly * R + G::col(lx);
-            const int gy = gyt[ly];
-            if (gy >= 0) off = gxt[lx] + d.nxp * gy;
-        }
-        ldoff[m] = off;
-        lddst[m] = dst;
-    }
-    auto slot = [&](int q) { return sm + ((q - k0 + 2) & 3) * SLOT; };
-    auto issue = [&](int q, int gk) {
-        double* s = slot(q);
-        const long long pk = (long long)gk * plane;
-#pragma unroll
-        for (int m = 0; m < NLD; ++m) {
-            const int e = tid + m * NT;
-            if (e < LTOT) {
-                const double* src = e < LU ? u0 : (e < LU + LV ? v0 : (e < LU + LV + LC ? w0 : p0));
-                const int off = ldoff[m];
-                cp_async8(s + lddst[m], off >= 0 ? src + pk + off : u0, off >= 0);
-            }
+    // Plane m = k0-1+U (mod 6): red cells of m+2 in column R, black ones of m
+    // in column K.  o: plane m+4 in the periodic array, om: plane m.
+    // Both cells are updated by every lane, their chains side by side: what
+    // the tile's outermost cells and, at the end, plane k1+2 get is wrong and
+    // reaches no owned face.
+    auto phase = [&](auto UC, int m, int sR, int sK, int nR, int nK, const factors& FR, const factors& FK,
+                     double (&wR)[6], double (&wK)[6], double (&pR)[6], double (&pK)[6]) {
+        constexpr int U = decltype(UC)::value;
+        // what the last plane read, a barrier ago; nothing waits for a read of its own plane
+        to_cols(wnext, wA[(U + 3) % 6], wB[(U + 3) % 6]);
+        to_cols(pnext, pA[(U + 2) % 6], pB[(U + 2) % 6]);
+        if (m + 4 <= k1 + 2) {
+            if (m + 4 <= k1 + 1) fetch((U + 5) % 6, o);
+            wnext = get_w(o);
+            o = next(o);
         }
         cp_async_commit();
-    };
-    const int r_ly = tid / HR, r_m = tid % HR;
-    const int b_ly = 1 + tid / HB, b_m = tid % HB;
-    const bool r_ok = tid < WY * HR, b_ok = tid < (WY - 2) * HB;
-    auto cell = [&](int q, int ly, int lx, int gy, int gk) {
-        double* s = slot(q);
-        double* su = s;
-        double* sv = s + NU;
-        double* sw = s + NU + NV;
-        double* sp = s + NU + NV + NC;
-        double* swn = slot(q + 1) + NU + NV;
-        const int c0 = ly * R + G::col(lx), c1 = ly * R + G::col(lx + 1), cn = c0 + R;
-        double mu_u_i = 1.0, mu_u_ip = 1.0, mu_v_j = 1.0, mu_v_jp = 1.0, mu_w = 1.0;
-        if (MU == MU_PLANE) {
-            mu_u_i = smu[c0];
-            mu_u_ip = smu[c1];
-            mu_v_j = smu[NU + c0];
-            mu_v_jp = smu[NU + cn];
-            mu_w = smu[NU + NV + c0];
+        if (own && m + 3 <= k1) pnext = get_p(om + 3 * plane);
+        if (row_in) {
+            faces fK = get((U + 1) % 6, sK, nK), fR = get((U + 3) % 6, sR, nR);
+            update(fK, FK, wK[U], wK[(U + 1) % 6], pK[U]);
+            update(fR, FR, wR[(U + 2) % 6], wR[(U + 3) % 6], pR[(U + 2) % 6]);
+            put((U + 1) % 6, sK, nK, fK);
+            put((U + 3) % 6, sR, nR, fR);
         }
-        double ui = su[c0], uip = su[c1], vj = sv[c0], vjp = sv[cn], wk = sw[c0], wkp = swn[c0], pc = sp[c0];
-        sor_cell_fac<1, PY, 1>(ui, uip, vj, vjp, wk, wkp, pc, mu_u_i, mu_u_ip, mu_v_j, mu_v_jp, mu_w, mu_w, sfac[c0],
-                               P, bc, 0, gy, gk, nx, ny, nz);
-        su[c0] = ui;
-        su[c1] = uip;
-        sv[c0] = vj;
-        sv[cn] = vjp;
-        sw[c0] = wk;
-        swn[c0] = wkp;
-        sp[c0] = pc;
-    };
-    auto red = [&](int q, int gk) {   // red: (i+j+k) odd, whole halo region
-        if (!r_ok) return;
-        const int gy = gyt[r_ly];
-        if (gy < 1 || gy > ny) return;
-        const int lx = ((x0 + gy + gk + 1) & 1) + 2 * r_m;
-        if (lx < WX) cell(q, r_ly, lx, gy, gk);
-    };
-    auto black = [&](int q, int gk) {   // black: (i+j+k) even, tile plus one ring
-        if (!b_ok) return;
-        const int gy = gyt[b_ly];
-        if (gy < 1 || gy > ny) return;
-        const int lx = 1 + ((x0 + 1 + gy + gk) & 1) + 2 * b_m;
-        if (lx < WX - 1) cell(q, b_ly, lx, gy, gk);
-    };
-    // owned cell of this thread
-    const int o_gx = x0 + tid % TX, o_gy = y0 + tid / TX;
-    const bool o_ok = o_gx <= nx && o_gy <= ny;
-    const int o_s = (2 + tid / TX) * R + G::col(2 + tid % TX);
-    const int o_off = o_gx + d.nxp * o_gy;
-    auto store = [&](int q, int gk) {
-        if (!o_ok) return;
-        const double* s = slot(q);
-        const long long c = (long long)gk * plane + o_off;
-        u1[c] = s[o_s];
-        v1[c] = s[NU + o_s];
-        w1[c] = s[NU + NV + o_s];
-        p1[c] = s[NU + NV + NC + o_s];
-        if (!PY && o_gy == ny) v1[c + d.nxp] = s[NU + o_s + R];
-    };
-    auto wrapz = [&](int q) { return ((q - 1) % nz + nz) % nz + 1; };
-
-    issue(k0 - 2, wrapz(k0 - 2));
-    issue(k0 - 1, wrapz(k0 - 1));
-    int gkm = wrapz(k0 - 3);   // plane q-1
-    int gk = wrapz(k0 - 2);    // plane q
-    for (int q = k0 - 2; q <= k1; ++q) {
-        if (q + 2 <= k1 + 1) issue(q + 2, wrapz(q + 2));
-        else cp_async_commit();           // empty group keeps the wait count uniform
-        cp_async_wait1();                 // planes up to q+1 have landed
+        auto store = [&](auto FULL) {
+            put2(w1, om, a ? wB[U] : wA[U], a ? wA[U] : wB[U], FULL);
+            put2(pn, om, a ? pB[U] : pA[U], a ? pA[U] : pB[U], FULL);
+            if (m > k0) put_uv(U, om - plane, FULL);
+        };
+        if (m >= k0) {
+            if (full) store(std::true_type{});
+            else if (own) store(std::false_type{});
+        }
+        om += plane;
+        cp_async_wait<1>();   // plane m + 3
         __syncthreads();
-        red(q, gk);                       // halo region of plane q
-        __syncthreads();
-        if (q - 1 >= k0 - 1) black(q - 1, gkm);   // tile + one ring of plane q-1
-        __syncthreads();
-        if (q - 1 >= k0) store(q - 1, gkm);
-        __syncthreads();                  // slot of q-1 is refilled by the next issue
-        gkm = gk;
-        gk = gk == nz ? 1 : gk + 1;
+    };
+    auto odd = [&](auto UC, int m) { phase(UC, m, sB, sA, nB, nA, FB, FA, wB, wA, pB, pA); };
+    auto even = [&](auto UC, int m) { phase(UC, m, sA, sB, nA, nB, FA, FB, wA, wB, pA, pB); };
+    for (int m = k0 - 1;; m += 6) {
+        odd(std::integral_constant<int, 0>{}, m);
+        if (m + 1 > k1) break;
+        even(std::integral_constant<int, 1>{}, m + 1);
+        if (m + 2 > k1) break;
+        odd(std::integral_constant<int, 2>{}, m + 2);
+        if (m + 3 > k1) break;
+        even(std::integral_constant<int, 3>{}, m + 3);
+        if (m + 4 > k1) break;
+        odd(std::integral_constant<int, 4>{}, m + 4);
+        if (m + 5 > k1) break;
+        even(std::integral_constant<int, 5>{}, m + 5);
+        if (m + 6 > k1) break;
     }
+    if (full) put_uv((k1 - k0 + 2) % 6, om - plane, std::true_type{});
+    else if (own) put_uv((k1 - k0 + 2) % 6, om - plane, std::false_type{});
 }
 
 double mdx_div_floor(const mdx_ctx_t* ctx, double umax) {
@@ -646,6 +663,15 @@ static bool sor_pxz(const mdx_ctx_t* ctx) {
     return ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL;
 }
 
+static int shell_copy(mdx_ctx_t* ctx) {
+    const mdx_dims& d = ctx->d;
+    double** f = ctx->f;
+    MDX_LAUNCH(ctx, MDX_T_OTHER, "shell copy", k_shell_copy,
+               dim3((std::max(d.nxp, d.ny) + 31) / 32, (std::max(d.nyp, d.nz) + 7) / 8, 3), dim3(32, 8), 0, d,
+               f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_US], f[MDX_VS], f[MDX_WS]);
+    return MDX_OK;
+}
+
 // first: u, v, w are not set yet, the red sweep reads u*, v*, w* (sor_pxz only).
 static int sor_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p, bool first = false) {
     const mdx_dims& d = ctx->d;
@@ -655,10 +681,7 @@ static int sor_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p, bool first = f
     dim3 grid((na + 31) / 32, (d.ny + 3) / 4, (d.nz + 1) / 2);
     const bool pxz = sor_pxz(ctx);
     const bool py = ctx->bc.is_periodic[1] != 0;
-    if (first)
-        MDX_LAUNCH(ctx, MDX_T_OTHER, "shell copy", k_shell_copy,
-                   dim3((std::max(d.nxp, d.ny) + 31) / 32, (std::max(d.nyp, d.nz) + 7) / 8, 3), dim3(32, 8), 0, d,
-                   f[MDX_UN], f[MDX_VN], f[MDX_WN], f[MDX_US], f[MDX_VS], f[MDX_WS]);
+    if (first) MDX_TRY(shell_copy(ctx));
     for (int parity = 0; parity < 2; ++parity) {
         const int rev = parity;   // red sweeps walk k up, black sweeps walk k down
         if (pxz) {
@@ -687,8 +710,8 @@ static int sor_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p, bool first = f
 // ---- red-black kernel variants and their autotuner ---------------------------
 // Variants (all bit-identical per iteration):
 //   MDX_SORV_SWEEPS    one launch per colour sweep
-//   MDX_SORV_FUSED8    fused red+black pass, 32x8 tiles, 256 threads
-//   MDX_SORV_FUSED16   fused red+black pass, 32x16 tiles, 512 threads
+//   MDX_SORV_FUSED8    red+black pass, 60x5 tiles, two blocks per SM
+//   MDX_SORV_FUSED16   red+black pass, 60x17 or (IBM factors) 60x13 tiles
 //   MDX_SORV_SPLIT     one launch per colour sweep on colour-split copies
 //                      (tol > 0 only: the copies cost two passes over u, v,
 //                      w, p per projection)
@@ -759,71 +782,113 @@ static int sor_split_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p) {
     return MDX_OK;
 }
 
-template <int MU, int TY, int NT>
-static size_t fused_smem() {
-    using G = fused_geom<32, TY, NT>;
-    return sizeof(double) * (4 * G::SLOT + (MU == MU_PLANE ? G::NU + G::NV + G::NC : 0) + G::NC) +
-           sizeof(int) * (G::UX + G::WY + 1);
-}
-
 static bool fused_ok(const mdx_ctx_t* ctx) {
     return ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL;
 }
 
-template <int TY, int NT>
-static int fused_attrs(mdx_ctx_t* ctx) {
-    const int s_one = (int)fused_smem<MU_ONE, TY, NT>(), s_plane = (int)fused_smem<MU_PLANE, TY, NT>();
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_sor_fused<MU_ONE, 0, 32, TY, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_one));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_sor_fused<MU_ONE, 1, 32, TY, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_one));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_sor_fused<MU_PLANE, 0, 32, TY, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_plane));
-    MDX_CUDA(ctx, cudaFuncSetAttribute(k_sor_fused<MU_PLANE, 1, 32, TY, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_plane));
+// The second u, v, w.
+static int pass_alloc(mdx_ctx_t* ctx) {
+    for (int t = 0; t < 3; ++t)
+        if (!ctx->sor_alt[t]) MDX_CUDA(ctx, cudaMalloc(&ctx->sor_alt[t], sizeof(double) * ctx->d.npad));
     return MDX_OK;
 }
 
-static int fused_prepare(mdx_ctx_t* ctx) {
-    const size_t bytes = sizeof(double) * ctx->d.npad;
-    for (int t = 0; t < 4; ++t)
-        if (!ctx->sor_alt[t]) MDX_CUDA(ctx, cudaMalloc(&ctx->sor_alt[t], bytes));
-    // the second state starts as a copy, so faces the sweeps never touch
-    // (ghosts) are equal in both
-    const int ids[4] = {MDX_UN, MDX_VN, MDX_WN, MDX_PN};
-    for (int t = 0; t < 4; ++t)
-        MDX_CUDA(ctx, cudaMemcpyAsync(ctx->sor_alt[t], ctx->f[ids[t]], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    if (!ctx->fused_attr) {
-        MDX_TRY((fused_attrs<8, 256>(ctx)));
-        MDX_TRY((fused_attrs<16, 512>(ctx)));
-        ctx->fused_attr = true;
-    }
-    return MDX_OK;
+// The second state without an error where there is no room for it, or no
+// allocation may be made: the sweeps do without.
+static bool pass_ready(mdx_ctx_t* ctx) {
+    if (ctx->sor_alt[2]) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    for (int t = 0; t < 3; ++t)
+        if (!ctx->sor_alt[t] && cudaMalloc(&ctx->sor_alt[t], sizeof(double) * ctx->d.npad) != cudaSuccess) {
+            (void)cudaGetLastError();
+            ctx->sor_alt[t] = nullptr;
+            return false;
+        }
+    return true;
 }
 
-template <int TY, int NT>
-static int sor_fused_iteration(mdx_ctx_t* ctx, const mdx_sor_params& p) {
+// The pass counts elements of an array in 32 bits.
+static bool pass_fits(const mdx_ctx_t* ctx) { return ctx->d.npad < 1LL << 31; }
+
+// Planes per block: the count that ends first, waves of resident blocks times
+// (planes + 5 for the halo and the start); steps: those phases.
+template <int RY>
+static int pass_planes(const mdx_ctx_t* ctx, long long* steps) {
+    using G = pass_geom<RY>;
     const mdx_dims& d = ctx->d;
+    const long long tiles = (long long)((d.nx + PASS_TX - 1) / PASS_TX) * ((d.ny + G::TY - 1) / G::TY);
+    const int slots = 148 * (RY == 8 ? 2 : 1);
+    int best = d.nz;
+    *steps = -1;
+    for (int kz = d.nz; kz >= 4 || kz == d.nz; --kz) {
+        const long long t = (tiles * ((d.nz + kz - 1) / kz) + slots - 1) / slots * (kz + 5);
+        if (*steps < 0 || t < *steps) {
+            *steps = t;
+            best = kz;
+        }
+    }
+    return best;
+}
+
+// One pass or two colour sweeps?  A phase of all blocks takes 1.75 us at 20
+// rows, 1.57 at 16, the time of the two sweeps for 85 000 and 76 000 cells
+// (20.6 us a million), whatever the grid; the sweeps win where tiles are
+// ragged or the chunks short.  Measured, us an iteration, pass / sweeps:
+// 180x150x140 59 / 78, 512x256x256 443 / 733, 240x102x96 37 / 49, 300x300x40
+// 61 / 77, 256x128x128 (a fifth column of tiles with 16 of 60 cells) 82 / 86,
+// 64x128x256 58 / 45, 128x64x64 17 / 16; with factors 180x150x140 63 / 78,
+// 320x200x200 196 / 272.
+static bool pass_wins(const mdx_ctx_t* ctx) {
+    if (!sor_pxz(ctx) || !pass_fits(ctx)) return false;
+    long long steps = 0;
+    if (ctx->mu_mode == MU_PLANE) {
+        pass_planes<16>(ctx, &steps);
+        return steps * 76000 < ctx->d.nint;
+    }
+    pass_planes<20>(ctx, &steps);
+    return steps * 85000 < ctx->d.nint;
+}
+
+// One iteration, u, v, w read from src and written to dst, p in place.
+template <int RY>
+static int sor_pass(mdx_ctx_t* ctx, const mdx_sor_params& p, double* const* src, double* const* dst) {
+    using G = pass_geom<RY>;
+    const mdx_dims& d = ctx->d;
+    const bool py = ctx->bc.is_periodic[1] != 0, plane = ctx->mu_mode == MU_PLANE;
+    // the factors' mode is the caller's: MU_PLANE never runs 20 rows, nor 1 16
+    constexpr int M0 = RY == 16 ? MU_PLANE : MU_ONE, M1 = RY == 20 ? MU_ONE : MU_PLANE;
+    auto kfn = plane ? (py ? k_sor_pass<M1, 1, RY> : k_sor_pass<M1, 0, RY>)
+                     : (py ? k_sor_pass<M0, 1, RY> : k_sor_pass<M0, 0, RY>);
+    const unsigned bit = 1u << ((RY == 8 ? 0 : 4) + (plane ? 2 : 0) + (py ? 1 : 0));
+    if (!(ctx->pass_attr & bit)) {
+        MDX_CUDA(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
+        ctx->pass_attr |= bit;
+    }
+    long long steps = 0;
+    const int KZ = ctx->opts.sor_kz > 0 ? ctx->opts.sor_kz : pass_planes<RY>(ctx, &steps);
+    const dim3 grid((d.nx + PASS_TX - 1) / PASS_TX, (d.ny + G::TY - 1) / G::TY, (d.nz + KZ - 1) / KZ);
+    MDX_LAUNCH(ctx, MDX_T_SOR_SWEEP, "sor pass", kfn, grid, 32 * RY, G::SMEM, d, ctx->bcd, p, KZ, src[0], src[1],
+               src[2], dst[0], dst[1], dst[2], ctx->f[MDX_PN], ctx->mu);
+    return MDX_OK;
+}
+
+// u, v, w and the second state change places.
+template <int RY>
+static int sor_pass_swap(mdx_ctx_t* ctx, const mdx_sor_params& p) {
     double** f = ctx->f;
-    const int KZ = ctx->opts.sor_kz > 0 ? ctx->opts.sor_kz : 16;
-    dim3 grid((d.nx + 31) / 32, (d.ny + TY - 1) / TY, (d.nz + KZ - 1) / KZ);
-    double** a = ctx->sor_alt;
-    const bool py = ctx->bc.is_periodic[1] != 0;
-    const bool plane = ctx->mu_mode == MU_PLANE;
-    auto kfn = plane ? (py ? k_sor_fused<MU_PLANE, 1, 32, TY, NT> : k_sor_fused<MU_PLANE, 0, 32, TY, NT>)
-                     : (py ? k_sor_fused<MU_ONE, 1, 32, TY, NT> : k_sor_fused<MU_ONE, 0, 32, TY, NT>);
-    const size_t smem = plane ? fused_smem<MU_PLANE, TY, NT>() : fused_smem<MU_ONE, TY, NT>();
-    MDX_LAUNCH(ctx, MDX_T_SOR_SWEEP, "sor fused", kfn, grid, NT, smem, d, ctx->bcd, p, KZ, f[MDX_UN], f[MDX_VN],
-               f[MDX_WN], f[MDX_PN], a[0], a[1], a[2], a[3], ctx->mu);
-    // the new state becomes the current one
-    std::swap(f[MDX_UN], a[0]);
-    std::swap(f[MDX_VN], a[1]);
-    std::swap(f[MDX_WN], a[2]);
-    std::swap(f[MDX_PN], a[3]);
+    const int ids[3] = {MDX_UN, MDX_VN, MDX_WN};
+    double* cur[3] = {f[MDX_UN], f[MDX_VN], f[MDX_WN]};
+    MDX_TRY(sor_pass<RY>(ctx, p, cur, ctx->sor_alt));
+    for (int t = 0; t < 3; ++t) std::swap(f[ids[t]], ctx->sor_alt[t]);
     return MDX_OK;
 }
 
 static int sor_iterate(mdx_ctx_t* ctx, const mdx_sor_params& p, int variant) {
     if (variant == MDX_SORV_SPLIT) return sor_split_iteration(ctx, p);
     if (variant == MDX_SORV_SPLITV) return sor_splitv_iteration(ctx, p);
-    if (variant == MDX_SORV_FUSED8) return sor_fused_iteration<8, 256>(ctx, p);
-    if (variant == MDX_SORV_FUSED16) return sor_fused_iteration<16, 512>(ctx, p);
+    if (variant == MDX_SORV_FUSED8) return sor_pass_swap<8>(ctx, p);
+    if (variant == MDX_SORV_FUSED16) return (ctx->mu_mode == MU_PLANE ? sor_pass_swap<16>(ctx, p) : sor_pass_swap<20>(ctx, p));
     return sor_iteration(ctx, p);
 }
 
@@ -871,13 +936,19 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     if ((want == MDX_SORV_AUTO || want == MDX_SORV_RESIDENT))
         want = mdx_res_face64_ok(ctx) ? MDX_SORV_RESIDENT : MDX_SORV_AUTO;
     if (want != MDX_SORV_SWEEPS && !fok) want = MDX_SORV_SWEEPS;
+    if ((want == MDX_SORV_FUSED8 || want == MDX_SORV_FUSED16) && !pass_fits(ctx)) want = MDX_SORV_SWEEPS;
     const bool warm = mdx_guess_supported(ctx) && (ctx->guess_mode != MDX_GUESS_ZERO || ctx->record_increments);
     // :63-84 -- u <- u* over the whole padded arrays; a fixed number of plain
     // sweeps does it in its first sweep (three copies of 30 MB, 35 us, on
     // 180x150x140)
-    const int fixed_v = want == MDX_SORV_AUTO && ctx->sor_tuned > 0 ? ctx->sor_tuned : want;
+    int fixed_v = want;
+    if (want == MDX_SORV_AUTO) {
+        fixed_v = ctx->sor_tuned > 0 ? ctx->sor_tuned : MDX_SORV_SWEEPS;
+        if (o.tol <= 0.0 && !warm && ctx->sor_tuned == 0 && pass_wins(ctx) && pass_ready(ctx)) fixed_v = MDX_SORV_FUSED16;
+    }
+    const bool fixed_pass = fixed_v == MDX_SORV_FUSED8 || fixed_v == MDX_SORV_FUSED16;
     const bool copy_in_sweep = o.tol <= 0.0 && o.n_iter > 0 && !warm && sor_pxz(ctx) &&
-                               (fixed_v == MDX_SORV_AUTO || fixed_v == MDX_SORV_SWEEPS);
+                               (fixed_v == MDX_SORV_SWEEPS || fixed_pass);
     if (!copy_in_sweep) {
         MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_UN], f[MDX_US], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
         MDX_CUDA(ctx, cudaMemcpyAsync(f[MDX_VN], f[MDX_VS], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -909,8 +980,9 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
             return MDX_OK;
         }
     }
-    const bool splitv = want == MDX_SORV_AUTO || want == MDX_SORV_SPLITV;
-    if (want == MDX_SORV_AUTO || want == MDX_SORV_SPLIT || splitv) MDX_TRY(split_alloc(ctx));
+    const int may = o.tol > 0.0 ? want : fixed_v;   // a fixed count never tunes
+    const bool splitv = may == MDX_SORV_AUTO || may == MDX_SORV_SPLITV;
+    if (may == MDX_SORV_SPLIT || splitv) MDX_TRY(split_alloc(ctx));
     const mdx_sor_params p = sor_params(ctx, dg);
     if (splitv) MDX_TRY(split_tables(ctx, p));
     // where u, v, w, p live while the sweeps run: the colour-split copies for
@@ -919,7 +991,11 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     bool fused_ready = false;
     auto layout_for = [&](int v) -> int {
         if ((v == MDX_SORV_FUSED8 || v == MDX_SORV_FUSED16) && !fused_ready) {
-            MDX_TRY(fused_prepare(ctx));
+            // the passes write neither ghosts nor the values beyond y walls
+            MDX_TRY(pass_alloc(ctx));
+            const int ids[3] = {MDX_UN, MDX_VN, MDX_WN};
+            for (int t = 0; t < 3; ++t)
+                MDX_CUDA(ctx, cudaMemcpyAsync(ctx->sor_alt[t], f[ids[t]], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
             fused_ready = true;
         }
         if ((v == MDX_SORV_SPLIT || v == MDX_SORV_SPLITV) != in_split) {
@@ -931,23 +1007,39 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     auto pick = [&]() -> int {
         if (want != MDX_SORV_AUTO) return want;
         if (ctx->sor_tuned > 0) return ctx->sor_tuned;
+        auto out = [&](int v) { return !pass_fits(ctx) && (v == MDX_SORV_FUSED8 || v == MDX_SORV_FUSED16); };
         for (int v = MDX_SORV_SWEEPS; v < MDX_SORV_NUM; ++v)
-            if (ctx->sor_tune_ms[v] <= 0.0) return v;
+            if (ctx->sor_tune_ms[v] <= 0.0 && !out(v)) return v;
         int best = MDX_SORV_SWEEPS;
         for (int v = MDX_SORV_SWEEPS; v < MDX_SORV_NUM; ++v)
-            if (ctx->sor_tune_ms[v] < ctx->sor_tune_ms[best]) best = v;
+            if (ctx->sor_tune_ms[v] < ctx->sor_tune_ms[best] && !out(v)) best = v;
         ctx->sor_tuned = best;
         return best;
     };
     mdx_solve_stats_t s{};
     s.guessed = guessed ? 1 : 0;
     if (o.tol <= 0.0) {
-        const int v = (want == MDX_SORV_AUTO) ? (ctx->sor_tuned > 0 ? ctx->sor_tuned : MDX_SORV_SWEEPS) : want;
-        MDX_TRY(layout_for(v));
+        const int v = fixed_v;
+        if (!copy_in_sweep) MDX_TRY(layout_for(v));
+        if (copy_in_sweep && fixed_pass) MDX_TRY(pass_alloc(ctx));
         mdx_event_pair run{};
         mdx_sweep_run_begin(ctx, &run);
-        if (copy_in_sweep) MDX_TRY(sor_iteration(ctx, p, true));
-        MDX_TRY(sor_iterations(ctx, p, v, o.n_iter - (copy_in_sweep ? 1 : 0)));
+        if (copy_in_sweep && fixed_pass) {   // u* -> ... -> u, by turns through the second state
+            MDX_TRY(shell_copy(ctx));
+            double* const us[3] = {f[MDX_US], f[MDX_VS], f[MDX_WS]};
+            double* const un[3] = {f[MDX_UN], f[MDX_VN], f[MDX_WN]};
+            double* const* src = us;
+            for (int left = o.n_iter; left > 0; --left) {
+                double* const* dst = left % 2 ? un : ctx->sor_alt;
+                MDX_TRY(v == MDX_SORV_FUSED8 ? sor_pass<8>(ctx, p, src, dst)
+                        : ctx->mu_mode == MU_PLANE ? sor_pass<16>(ctx, p, src, dst)
+                                                   : sor_pass<20>(ctx, p, src, dst));
+                src = dst;
+            }
+        } else {
+            if (copy_in_sweep) MDX_TRY(sor_iteration(ctx, p, true));
+            MDX_TRY(sor_iterations(ctx, p, v, o.n_iter - (copy_in_sweep ? 1 : 0)));
+        }
         mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT || copy_in_sweep ? 2LL * o.n_iter : -1);
         MDX_TRY(layout_for(MDX_SORV_SWEEPS));
         s.variant = v;

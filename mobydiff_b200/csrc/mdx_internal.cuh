@@ -129,11 +129,11 @@ struct mdx_ctx {
     double* f[MDX_NUM_FIELDS] = {nullptr};   // device mirrors (MDX_PHI -> phi)
     bool ibm_zero = true;                    // all IBM coefficients zero
     bool coef_zinv = false;                  // coefficients equal on every z plane
-    double* sor_alt[4] = {nullptr};          // second u,v,w,p state of the fused red-black pass
+    double* sor_alt[3] = {nullptr};          // second u,v,w state of the red-black pass
     double* split_f[4] = {nullptr};          // colour-split copies of u,v,w,p (split sweeps)
     double* split_tab = nullptr;             // their column factors: mu_u, mu_v, mu_w, fac planes (pidx2)
     bool split_norms = false;                // divergence norms read colour-split arrays
-    bool fused_attr = false;
+    unsigned pass_attr = 0;                  // k_sor_pass: shared-memory attribute set, bit per kernel
     // mixed-precision red-black: FP32 corrections, FP32 residual, IBM tables,
     // carved from one allocation (mx_du is its base) of mx_bytes
     float *mx_du = nullptr, *mx_dv = nullptr, *mx_dw = nullptr, *mx_dp = nullptr, *mx_r = nullptr;
