@@ -161,9 +161,10 @@ C3_GATE_PERIOD = 16   # the learned_gated guess re-tries the other choice every 
 SOR_VARIANT = 0   # --sor-variant: red-black kernel variant (0: the autotuner's choice)
 FFT_KERNEL = 0    # --fft-kernel: 0 warp-shuffle transforms where the lengths allow, 1 Stockham
 INNER_FORM = 0    # --inner-form: FP32 correction sweeps of the mixed path, 0 potential form, 1 face form
-SOR_NAMES = {1: "one launch per colour sweep", 2: "fused red+black pass 32x8", 3: "fused red+black pass 32x16",
+SOR_NAMES = {1: "one launch per colour sweep", 2: "red+black pass, 60x5 tiles", 3: "red+black pass, 60x17 or 60x13 tiles",
              4: "one launch per colour sweep on colour-split copies",
-             5: "one launch per colour sweep on colour-split copies, 2 cells per thread"}
+             5: "one launch per colour sweep on colour-split copies, 2 cells per thread",
+             6: "k_face_resident: a run of sweeps per launch, the state on chip"}
 
 
 # FP32 correction sweeps of the mixed path, by the hundreds digit of the
@@ -171,10 +172,10 @@ SOR_NAMES = {1: "one launch per colour sweep", 2: "fused red+black pass 32x8", 3
 SOR32_NAMES = {1: "k_sor_sweep32: one launch per colour, one cell per thread",
                3: "k_rb32_fused: one launch per red+black iteration",
                5: "k_sor_sweep32v: one launch per colour, 2 or 4 cells per thread",
-               7: "potential form: the autotuner's pick among k_pot_sweep (2 or 4 cells per thread), k_pot_sweep_w "
-                  "(one warp per row), k_pot_sweep_a (planes staged by cp.async) and k_pot_run_w (one warp per row, "
-                  "a block of iterations per cooperative launch; the pick on 256x128x128)"}
-SOR32_TRAFFIC = {1: "sor_sweep32", 3: "rb32_fused", 5: "sor_sweep32v", 7: "pot_run_w"}
+               7: "potential form: k_pot_resident (a block of iterations per cooperative launch, phi in registers) "
+                  "where the grid fits the SMs, as 256x128x128 does; else the autotuner's pick among k_pot_sweep, "
+                  "k_pot_sweep_w, k_pot_sweep_a and k_pot_run_w"}
+SOR32_TRAFFIC = {1: "sor_sweep32", 3: "rb32_fused", 5: "sor_sweep32v", 7: "pot_resident"}
 # algorithmic bytes per cell of one FP32 colour sweep launch (a fused
 # red+black launch does both colours): the face form reads and writes 4
 # floats per cell of one colour (16 B per cell of the grid); the potential
@@ -185,7 +186,8 @@ SOR32_ALG = {1: 16.0, 3: 32.0, 5: 16.0, 7: 8.0}
 
 def _sor64_traffic_key(variant):
     """traffic.json entry of the FP64 sweep kernel a solve ran."""
-    return {4: "sor_sweep_split", 5: "sor_sweep_splitv"}.get(variant, "sor_sweep")
+    return {2: "sor_pass", 3: "sor_pass", 4: "sor_sweep_split", 5: "sor_sweep_splitv",
+            6: "face_resident"}.get(variant, "sor_sweep")
 
 
 def _setup(cfg, M, device, profile=False, tol=None, precision=None, seed=None):
@@ -1212,8 +1214,8 @@ def run_learned_mixed(args, cfg):
                          traffic_key=SOR32_TRAFFIC.get(kind, "sor_sweep32"))
     roofline["sor_kernel"] = SOR32_NAMES.get(kind, "?")
     if kind == 7:
-        roofline["note"] = ("phi and r~ (37 MB) stay resident in the 126 MB L2 across sweeps, so the sweeps "
-                            "run from L2 and can pass the HBM copy rate")
+        roofline["note"] = ("phi and r~ stay in registers across the sweeps of a run, so the sweeps "
+                            "can pass the HBM copy rate")
     step_hbm = _step_hbm(cells, ms_all / K, iters / K, 16.0 if kind == 7 else 32.0)
 
     # ---- the same steps without the network: extrapolated increment only ----

@@ -13,13 +13,15 @@
 //   k_fftz<inv>  spec -> spec
 //   k_ifftx      spec -> phi             inverse real FFT of one row, *1/(nx nz)
 //   k_correct    us,vs,ws,phi,pn -> un,vn,wn,pn
+// Where a (ny, nz) plane fits shared memory, k_zty makes the three middle
+// passes in one.
 //
 // Where nx/2 and nz are 32 P (P = 1, 2, 4, 8, 16) each line is one warp's
 // four-step transform: a P-point DFT in registers and a 32-point DFT across
 // the lanes by shuffles (k_div_fftx_w, k_fftz_w, k_ifftx_w).  Other lengths
 // use shared-memory Stockham transforms (the formulation of Govindaraju et
 // al., "High performance discrete Fourier transforms on graphics
-// processors", SC 2008) with radices 4, 2, 3, 5, 7.  The real transform of
+// processors", SC 2008) with radices 7, 5, 3, 8, 4, 2, each its own code.  The real transform of
 // length nx is a complex transform of length nx/2 on packed even/odd samples
 // plus the standard split step.  Twiddles are tables built on the host with
 // long-double cosl/sinl.

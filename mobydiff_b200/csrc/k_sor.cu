@@ -1040,7 +1040,8 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
             if (copy_in_sweep) MDX_TRY(sor_iteration(ctx, p, true));
             MDX_TRY(sor_iterations(ctx, p, v, o.n_iter - (copy_in_sweep ? 1 : 0)));
         }
-        mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT || copy_in_sweep ? 2LL * o.n_iter : -1);
+        mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT || (copy_in_sweep && !fixed_pass) ? 2LL * o.n_iter
+                                     : copy_in_sweep ? o.n_iter : -1);
         MDX_TRY(layout_for(MDX_SORV_SWEEPS));
         s.variant = v;
         s.iterations = o.n_iter;
