@@ -565,7 +565,8 @@ k_zty(mdx_dims d, double dyi2, double dx, double dz, double2* __restrict__ spec,
 #pragma unroll 4
         for (int t = t0; t < ny * nz; t += step) {
             const int j = quot(t, rz), kz = t - j * nz;
-            A[j * ls + kz] = __ldcg(spec + (long long)t * nxh + kx);
+            const double2* x = spec + (long long)t * nxh + kx;
+            A[j * ls + kz] = OWN ? ld_l2(x) : __ldcg(x);
         }
         if (!OWN) {
             const double* src = dinv + (long long)kx * ny * nzh;
@@ -660,7 +661,14 @@ k_ifftx(mdx_dims d, int R, typename cx<C2>::R scale, const C2* __restrict__ spec
         C2 z = cx<C2>::mk(0, 0);
         if (row < nrows) {
             const C2* X = spec + (long long)row * nxh;
-            C2 xk = X[k], xm = X[M - k];
+            C2 xk, xm;
+            if constexpr (OWN) {
+                xk = ld_l2(X + k);
+                xm = ld_l2(X + M - k);
+            } else {
+                xk = X[k];
+                xm = X[M - k];
+            }
             if (k == 0) { xk.y = 0; xm.y = 0; }   // kx = 0 and kx = M bins are real
             const C2 xc = cconj(xm);
             const C2 e = cadd(xk, xc);
@@ -1029,9 +1037,12 @@ k_fftx_r2c(mdx_dims d, int R, const double* __restrict__ rhs, double2* __restric
     for (int t = threadIdx.x; t < R * M; t += blockDim.x) {
         const int rl = quot(t, rM), n = t - rl * M;
         const int row = row0 + rl;
-        A[rl * M + n] = (row < nrows) ? make_double2(__ldg(rhs + (long long)row * d.nx + 2 * n),
-                                                     __ldg(rhs + (long long)row * d.nx + 2 * n + 1))
-                                      : make_double2(0.0, 0.0);
+        double2 x = make_double2(0.0, 0.0);
+        if (row < nrows) {
+            const double* q = rhs + (long long)row * d.nx + 2 * n;
+            x = OWN ? make_double2(ld_l2(q), ld_l2(q + 1)) : make_double2(__ldg(q), __ldg(q + 1));
+        }
+        A[rl * M + n] = x;
     }
     __syncthreads();
     double2* Z = smem_fft<false>(A, B, M, R, M, pl, twx, 2);

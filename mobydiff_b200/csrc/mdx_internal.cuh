@@ -330,6 +330,20 @@ __device__ __forceinline__ void prefetch_l2(const void* a) { asm volatile("prefe
 // placed.
 __device__ __forceinline__ void mdx_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mdx_grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// What a kernel before may still write while this one's blocks are placed:
+// from L2, after mdx_grid_wait() (volatile, as that is, so not moved before
+// it).  Read-only loads (__ldg, a const __restrict__ pointer) may return an
+// older line and are for data that is constant over the kernel's whole life.
+__device__ __forceinline__ double ld_l2(const double* a) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ double2 ld_l2(const double2* a) {
+    double2 v;
+    asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(a));
+    return v;
+}
 #endif
 
 // ---- per-module entry points (internal) --------------------------------------
