@@ -574,6 +574,14 @@ int mdx_channel_ic(mdx_ctx_t* ctx, uint64_t seed, double amp_u, double amp_vw, d
  * (synchronises). */
 int mdx_divergence_norms(mdx_ctx_t* ctx, double* l2, double* linf);
 
+/* How often a block of an on-chip red-black run reads a neighbour's word that
+ * has not come before the run gives up (< 0: the default, about a second;
+ * 0: at the first miss).  The fields are half swept then: MDX_ERR_TIMEOUT,
+ * from the tolerance solve itself or, for a fixed count of iterations, from
+ * the next call that waits for the stream and returns fields or numbers made
+ * of them, or starts another run. */
+int mdx_set_wait_limit(mdx_ctx_t* ctx, int polls);
+
 /* Per-kernel-class device timing with CUDA events on the context stream.
  * on = 1: every 8th launch of a class is bracketed by an event pair, and
  * every run of back-to-back sweeps (MDX_T_SOR_BLOCK) as well; on = 2: only

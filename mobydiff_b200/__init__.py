@@ -193,6 +193,7 @@ def lib():
         "mdx_channel_ic": (i, [vp, C.c_uint64, d, d, d, d, d, P(SolveStatsT)]),
         "mdx_divergence_norms": (i, [vp, P(d), P(d)]),
         "mdx_set_timing": (i, [vp, i]),
+        "mdx_set_wait_limit": (i, [vp, i]),
         "mdx_get_timing": (i, [vp, P(TimingT)]),
         "mdx_launch_count": (C.c_longlong, [vp]),
         "mdx_last_solve_stats": (i, [vp, P(SolveStatsT)]),
@@ -546,6 +547,11 @@ class Solver:
         b = C.c_double(0.0)
         self._c(lib().mdx_divergence_norms(self.h, C.byref(a), C.byref(b)))
         return a.value, b.value
+
+    def set_wait_limit(self, polls: int) -> None:
+        """Reads of a missing word before an on-chip red-black run gives up with
+        MDX_ERR_TIMEOUT (-1: the default, about a second)."""
+        self._c(lib().mdx_set_wait_limit(self.h, int(polls)))
 
     def set_timing(self, on):
         """0/False off; 1/True sampled launches of every class plus whole

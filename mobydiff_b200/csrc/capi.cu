@@ -410,6 +410,7 @@ int mdx_copy_field(mdx_ctx_t* ctx, int field, double* host, int direction) {
     if (direction == 0) {
         MDX_CUDA(ctx, cudaMemcpyAsync(host, ctx->f[field], bytes, cudaMemcpyDeviceToHost, ctx->stream));
         MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        MDX_TRY(mdx_res_check(ctx));
     } else {
         MDX_CUDA(ctx, cudaMemcpyAsync(ctx->f[field], host, bytes, cudaMemcpyHostToDevice, ctx->stream));
         MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -456,6 +457,7 @@ int mdx_write_field_h5(mdx_ctx_t* ctx, const char* filename) {
         MDX_CUDA(ctx, cudaMemcpyAsync(h.data() + t * n, ctx->f[ids[t]], sizeof(double) * n, cudaMemcpyDeviceToHost,
                                       ctx->stream));
     MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    MDX_TRY(mdx_res_check(ctx));
     const mdx_grid_t& g = ctx->g;
     if (fdm_h5_write_field(filename, g.nx, g.ny, g.nz, g.lx, g.ly, g.lz, g.dx, g.dy, g.dz, g.re, g.dt, g.t_current,
                            h.data(), h.data() + n, h.data() + 2 * n, h.data() + 3 * n) != 0)
@@ -616,6 +618,7 @@ int mdx_divergence_norms(mdx_ctx_t* ctx, double* l2, double* linf) {
     MDX_TRY(need_fields(ctx));
     double a = 0.0, b = 0.0;
     MDX_TRY(mdx_k_div_norms(ctx, ctx->f[MDX_UN], ctx->f[MDX_VN], ctx->f[MDX_WN], &a, &b));
+    MDX_TRY(mdx_res_check(ctx));
     if (l2) *l2 = a;
     if (linf) *linf = b;
     return MDX_OK;
@@ -833,9 +836,16 @@ int mdx_channel_ic(mdx_ctx_t* ctx, uint64_t seed, double amp_u, double amp_vw, d
     MDX_TRY(rc);
     MDX_CUDA(ctx, cudaMemsetAsync(f[MDX_PN], 0, bytes, ctx->stream));
     MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    MDX_TRY(mdx_res_check(ctx));
     if (stats) *stats = s;
     if (s.status == MDX_ERR_NONFINITE) return mdx_fail(ctx, MDX_ERR_NONFINITE, "non-finite divergence in the t=0 projection");
     if (s.status == MDX_NOT_CONVERGED) return mdx_fail(ctx, MDX_NOT_CONVERGED, "t=0 projection not converged");
+    return MDX_OK;
+}
+
+int mdx_set_wait_limit(mdx_ctx_t* ctx, int polls) {
+    if (!ctx) return mdx_fail(nullptr, MDX_ERR_ARG, "null context");
+    ctx->rs_polls = polls;
     return MDX_OK;
 }
 

@@ -577,7 +577,7 @@ __device__ void sweeps_resident(const ens_args& A, int iters) {
         const ens_member& M = A.mem[m];
         const float* p32 = A.st[m].p32;
         const ens_faces a{M.d, mixed_params{p32[0], p32[1], p32[2], p32[3]}, M.du, M.dv, M.dw, M.dp, M.r32, M.mu32, M.fac32};
-        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride};
+        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride, POLLS};
         const res_box b = make_box<0>(M.d.ny, M.d.nz, p.nyb, p.nzb, R.tpr, p.first, at);
         if (!face_run_box<ens_faces, 0, RES_KZ>(a, b, R, iters, A.rbox, *(volatile unsigned*)A.rseq, ens_sm) && threadIdx.x == 0)
             A.rstate[1] = 1;

@@ -228,7 +228,7 @@ k_pot_resident(pot_geom L, res_geom R, int iters, float* __restrict__ phi, const
 #pragma unroll
             for (int u = 0; u < NB; ++u)
                 if (t + u * T < nw) {
-                    ok = wait_word(in + t + u * T, sq, v[u]) && ok;
+                    ok = wait_word(in + t + u * T, sq, v[u], R.polls) && ok;
                     st2s(W + DT[t + u * T], (f2)v[u].a | (f2)v[u].b << 32);
                 }
         }
@@ -376,7 +376,7 @@ bool make_plan(const mdx_ctx_t* ctx, int tpr, const res_shape* shapes, int nshap
             const double cost = (double)bz * std::max(issue * warps, 100) + (double)(by + bz) * tpr + 0.01 * s;
             if (out->shape >= 0 && cost >= best) continue;
             best = cost;
-            out->R = res_geom{nyb, by, bz, tpr, 2 * (by + bz) * tpr};
+            out->R = res_geom{nyb, by, bz, tpr, 2 * (by + bz) * tpr, ctx->rs_polls < 0 ? POLLS : ctx->rs_polls};
             out->blocks = nyb * nzb;
             out->threads = (by * tpr + 31) & ~31;
             out->shape = s;
@@ -511,6 +511,7 @@ int mdx_res_face64_run(mdx_ctx_t* ctx, const mdx_sor_params& p, int iters) {
 
 int mdx_res_check(mdx_ctx_t* ctx) {
     if (!ctx->red_host || *(volatile int*)err_word(ctx) == 0) return MDX_OK;
+    MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // runs queued behind it may set the word too
     *err_word(ctx) = 0;
     ctx->rs_seq = 0;   // the inboxes are cleared before the next run
     return mdx_fail(ctx, MDX_ERR_TIMEOUT, "resident red-black sweeps: a block gave up waiting for its neighbour");

@@ -456,7 +456,7 @@ int mdx_k_cfl(mdx_ctx_t* ctx, double* cfl) {
     MDX_CUDA(ctx, cudaMemcpyAsync(ctx->red_host, ctx->red_out, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *cfl = ctx->red_host[1];
-    return MDX_OK;
+    return mdx_res_check(ctx);
 }
 
 // ---------------------------------------------------------------------------
@@ -497,7 +497,7 @@ int mdx_k_center_vel(mdx_ctx_t* ctx, double* uc, double* vc, double* wc) {
         if (e != cudaSuccess) rc = mdx_fail(ctx, MDX_ERR_CUDA, "center_vel copy: %s", cudaGetErrorString(e));
     }
     cudaFreeAsync(buf, ctx->stream);
-    return rc;
+    return rc == MDX_OK ? mdx_res_check(ctx) : rc;
 }
 
 // ---------------------------------------------------------------------------

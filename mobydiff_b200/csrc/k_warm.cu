@@ -263,5 +263,5 @@ extern "C" int mdx_get_increment(mdx_ctx_t* ctx, int substage, double* host) {
     MDX_CUDA(ctx, cudaMemcpyAsync(host, ctx->dp_hist[substage], sizeof(double) * ctx->d.nint, cudaMemcpyDeviceToHost,
                                   ctx->stream));
     MDX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return MDX_OK;
+    return mdx_res_check(ctx);
 }

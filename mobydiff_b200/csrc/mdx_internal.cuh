@@ -164,6 +164,7 @@ struct mdx_ctx {
     void* rs_box = nullptr;
     size_t rs_bytes = 0;
     unsigned rs_seq = 0;
+    int rs_polls = -1;                       // mdx_set_wait_limit
     // warm starts: increments of the last projection of each RK substage
     int guess_mode = 0;                      // MDX_GUESS_*
     bool record_increments = false;
@@ -348,6 +349,11 @@ __device__ __forceinline__ double2 ld_l2(const double2* a) {
 
 // ---- per-module entry points (internal) --------------------------------------
 mdx_step_params mdx_make_params(const mdx_ctx_t* ctx);
+// MDX_ERR_TIMEOUT when an on-chip run (k_sor_resident.cu) gave up a wait and
+// left the fields half swept.  Called after a synchronisation wherever fields,
+// or numbers made of them, go to the caller: a fixed count of iterations
+// returns before its runs have ended.
+int mdx_res_check(mdx_ctx_t* ctx);
 int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg, bool ghosts = false);
 // apply_bc on the n arrays (un, vn, wn, pn), the * arrays or both.  Inside a
 // step the * arrays need it after the predictor and the n arrays after the

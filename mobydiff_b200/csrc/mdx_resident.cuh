@@ -17,6 +17,4 @@ int mdx_res_pot_run(mdx_ctx_t* ctx, const pot_geom& L, int iters);
 int mdx_res_face32_run(mdx_ctx_t* ctx, const mixed_params& P, int iters);
 struct mdx_sor_params;
 int mdx_res_face64_run(mdx_ctx_t* ctx, const mdx_sor_params& p, int iters);
-// After a synchronisation: MDX_ERR_TIMEOUT when a run gave up a wait.
-int mdx_res_check(mdx_ctx_t* ctx);
 void mdx_res_free(mdx_ctx_t* ctx);

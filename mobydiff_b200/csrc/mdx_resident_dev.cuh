@@ -68,11 +68,11 @@ __device__ __forceinline__ word ld_word(const word* p) {
                  : "memory");
     return w;
 }
-// Polls about as long as a second; false when the word did not come.
-constexpr int POLLS = 1 << 20;
-__device__ __forceinline__ bool wait_word(const word* p, unsigned seq, word& w) {
+// False when the word did not come within `polls` more reads of it.
+constexpr int POLLS = 1 << 20;   // about a second, the default
+__device__ __forceinline__ bool wait_word(const word* p, unsigned seq, word& w, int polls) {
     for (int n = 0; w.sa != seq || w.sb != seq; ++n) {
-        if (n == POLLS) return false;
+        if (n >= polls) return false;
         w = ld_word(p);
     }
     return true;
@@ -86,6 +86,7 @@ struct res_geom {
     int nyb, by, bz;   // blocks along y; rows and planes of the largest box
     int tpr;           // words per row
     int stride;        // words of one inbox, at least 2 (by + bz) tpr
+    int polls;         // reads of a word that has not come before a block gives up
 };
 __device__ __forceinline__ word* inbox(word* box, const res_geom& R, int block, int parity) {
     return box + ((long long)block * 2 + parity) * R.stride;
@@ -240,15 +241,15 @@ __device__ __forceinline__ bool face_run_box(const A& a, const res_box& b, const
 #pragma unroll
             for (int e = 0; e < 2; ++e)
                 if (t + e * NTH < nw) {
-                    ok = wait_word(in + 2 * nzw + t + e * NTH, sq, w[e]) && ok;
+                    ok = wait_word(in + 2 * nzw + t + e * NTH, sq, w[e], R.polls) && ok;
                     const int dst = DT[t + e * NTH];
                     value(w[e], V[(dst >> 1) + ((dst ^ PAR) & 1 ? tpr : 0)]);
                 }
         }
         // the z faces: those of the columns this block did not sweep there
         if (act) {
-            ok = wait_word(in + at, sq, zl) && ok;
-            ok = wait_word(in + nzw + at, sq, zh) && ok;
+            ok = wait_word(in + at, sq, zl, R.polls) && ok;
+            ok = wait_word(in + nzw + at, sq, zh, R.polls) && ok;
             value(zl, wY[0]);
             T v;
             value(zh, v);
