@@ -1540,7 +1540,13 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
                 MDX_TRY(sweeps(m));
                 it += m;
                 MDX_TRY(corr_residual(&e));
-                MDX_TRY(mdx_res_check(ctx));
+                if (const int rc = mdx_res_check(ctx)) {   // the corrections are half swept: the next solve starts from 0
+                    if (pot) MDX_CUDA(ctx, cudaMemsetAsync(ctx->pt_phi, 0, sizeof(float) * 2 * (size_t)L.H, ctx->stream));
+                    else
+                        for (float* a : {ctx->mx_du, ctx->mx_dv, ctx->mx_dw, ctx->mx_dp})
+                            MDX_CUDA(ctx, cudaMemsetAsync(a, 0, sizeof(float) * (size_t)split_elems(d), ctx->stream));
+                    return rc;
+                }
                 if (!std::isfinite(e)) break;
                 if (e <= inner_target) break;
                 // FP32 stagnation: less than 0.1 % per check_every iterations for 20 x check_every

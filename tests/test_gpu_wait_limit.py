@@ -67,3 +67,41 @@ def test_tolerance_solve_reports_itself(precision, form):
         for n in ("us", "vs", "ws", "pn"):
             s.set(n, getattr(f, n))
         assert s.pressure_projection(1e-3).residual <= 1.0000001e-6
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_mixed_solve_after_a_timeout_equals_a_fresh_one(form):
+    """Nothing of the abandoned FP32 corrections reaches the next solve: the
+    same bits as in a context that never gave up.  Runs of one iteration, so
+    that some blocks finish and write while others give up; limits from no
+    reads up to where whole runs succeed before one does not."""
+    g, bc = channel_case(*SHAPE)
+    f = random_fields(g, 9, scale=0.1)
+    f.vs[:, 1, :] = f.vs[:, g.ny + 1, :] = 0.0
+    opts = M.make_solver_opts(M.SOLVER_REDBLACK, sor=1.7, tol=1e-6, check_every=1, precision=M.PREC_MIXED,
+                              inner_form=form, adaptive_checks=False)
+
+    def solve(s):
+        for n in ("us", "vs", "ws", "pn"):
+            s.set(n, getattr(f, n))
+        st = s.pressure_projection(1e-3, check=False)
+        return st.rc, st.iterations
+
+    with to_device(M, g, bc, f) as s:
+        s.init_pressure_solver(opts)
+        fresh = solve(s)
+        assert fresh[0] == M.MDX_OK
+        want = {n: s.get(n) for n in ("un", "vn", "wn", "pn")}
+    gave_up = 0
+    with to_device(M, g, bc, f) as s:
+        s.init_pressure_solver(opts)
+        for polls in (0, 1, 2, 3, 4, 6, 8, 12, 16, 32):
+            s.set_wait_limit(polls)
+            rc, _ = solve(s)
+            assert rc in (M.MDX_OK, M.MDX_ERR_TIMEOUT)
+            gave_up += rc == M.MDX_ERR_TIMEOUT
+            s.set_wait_limit(-1)
+            assert solve(s) == fresh, polls
+            for n, a in want.items():
+                assert np.array_equal(s.get(n), a), (polls, n)
+    assert gave_up > 0
