@@ -409,7 +409,8 @@ int mdx_ensemble_set_guess(mdx_ensemble_t* ens, int mode);
 int mdx_ensemble_ic(mdx_ensemble_t* ens);
 /* nsteps RK3 steps of every member; *total_iters = red-black iterations of
  * all members (synchronises).  MDX_NOT_CONVERGED / MDX_ERR_NONFINITE when a
- * member's projection ended so. */
+ * member's last projection ended so, MDX_ERR_TIMEOUT when a block of the
+ * on-chip sweeps gave up a wait in any of the steps. */
 int mdx_ensemble_step(mdx_ensemble_t* ens, int nsteps, long long* total_iters);
 int mdx_ensemble_member_stats(mdx_ensemble_t* ens, int member, mdx_solve_stats_t* last, long long* iters_total);
 /* Padded field MDX_UN, MDX_VN, MDX_WN or MDX_PN of a member. */
@@ -419,6 +420,8 @@ int mdx_ensemble_set(mdx_ensemble_t* ens, int member, int field, const double* h
  * 32, <= 512), blocks per SM (0: as many as fit) and the register variant
  * (low_regs != 0: 64 registers per thread, twice the resident warps). */
 int mdx_ensemble_config(mdx_ensemble_t* ens, int threads, int blocks_per_sm, int low_regs);
+/* mdx_set_wait_limit of the on-chip sweeps (mixed precision, face form). */
+int mdx_ensemble_set_wait_limit(mdx_ensemble_t* ens, int polls);
 /* Time one step of each candidate launch shape from the same saved state and
  * keep the fastest; the choice is cached in the JSON file cache_path (may be
  * NULL) under a key of the member sizes, the mode and the device name

@@ -143,10 +143,11 @@ struct ens_args {
     int split;
     // on-chip FP32 face sweeps (res_* below); rbox null: not used
     struct ens_plan* rplan;          // per member: its blocks and their boxes
-    int* rstate;                     // {this round's plan holds, a block gave up a wait}
+    int* rstate;                     // {this round's plan holds, a block gave up a wait since the host looked}
     unsigned* rseq;                  // last sequence number used
     word* rbox;                      // inboxes, rstride words each
     int rstride, rsmem;              // rsmem: shared memory of a block for its box
+    int rpolls;                      // res_geom::polls
     const int* learn_ok;             // per member: the network wrote a correction
     int gate_period;                 // > 0: apply it per substage only while it takes fewer iterations
 };
@@ -577,7 +578,7 @@ __device__ void sweeps_resident(const ens_args& A, int iters) {
         const ens_member& M = A.mem[m];
         const float* p32 = A.st[m].p32;
         const ens_faces a{M.d, mixed_params{p32[0], p32[1], p32[2], p32[3]}, M.du, M.dv, M.dw, M.dp, M.r32, M.mu32, M.fac32};
-        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride, POLLS};
+        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride, A.rpolls};
         const res_box b = make_box<0>(M.d.ny, M.d.nz, p.nyb, p.nzb, R.tpr, p.first, at);
         if (!face_run_box<ens_faces, 0, RES_KZ>(a, b, R, iters, A.rbox, *(volatile unsigned*)A.rseq, ens_sm) && threadIdx.x == 0)
             A.rstate[1] = 1;
@@ -1241,6 +1242,7 @@ struct mdx_ensemble {
     size_t rbytes = 0;
     int rstride = 0, rsmem = 0;
     double rseq_bound = 0.0;
+    int rpolls = -1;                 // mdx_ensemble_set_wait_limit
 };
 
 namespace {
@@ -1346,6 +1348,7 @@ ens_args make_args(mdx_ensemble_t* E, int s, int momentum) {
     A.rplan = E->rplan;
     A.rstate = E->rstate;
     A.rseq = E->rseq;
+    A.rpolls = E->rpolls < 0 ? POLLS : E->rpolls;
     A.learn_ok = E->learn_ok;
     A.gate_period = E->gate_period;
     return A;
@@ -1385,8 +1388,23 @@ int res_prepare(mdx_ensemble_t* E, int variant, int threads, int grid, int subst
         ENS_CUDA(E, cudaMemsetAsync(E->rseq, 0, sizeof(unsigned), E->stream));
         E->rseq_bound = 2.0 * rounds * substages;
     }
-    ENS_CUDA(E, cudaMemsetAsync(E->rstate, 0, 2 * sizeof(int), E->stream));
     return MDX_OK;
+}
+
+// After a synchronisation: MDX_ERR_TIMEOUT when a block gave up a wait in any
+// launch since the last call, whatever later projections ended with.  The
+// flag stays up until then, so on-chip rounds behind it end at once.  The
+// half-swept corrections are cleared: the next projection starts from 0.
+int res_check(mdx_ensemble_t* E) {
+    if (!E->rstate) return MDX_OK;
+    int gave_up = 0;
+    ENS_CUDA(E, cudaMemcpy(&gave_up, E->rstate + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    if (!gave_up) return MDX_OK;
+    ENS_CUDA(E, cudaMemsetAsync(E->rstate, 0, 2 * sizeof(int), E->stream));
+    for (const auto& M : E->hm)
+        for (float* a : {M.du, M.dv, M.dw, M.dp})
+            ENS_CUDA(E, cudaMemsetAsync(a, 0, sizeof(float) * (size_t)split_elems(M.d), E->stream));
+    return efail(E, MDX_ERR_TIMEOUT, "on-chip sweeps: a block gave up waiting for its neighbour");
 }
 
 int launch_substage(mdx_ensemble_t* E, int s, int momentum, int variant, int threads, int grid, int split = 0) {
@@ -1807,6 +1825,7 @@ int mdx_ensemble_ic(mdx_ensemble_t* E) {
         ENS_CUDA(E, cudaMemsetAsync(E->hm[m].pn, 0, sizeof(double) * E->hm[m].d.npad, E->stream));
     std::vector<ens_state> after;
     MDX_TRY(read_stats(E, after));
+    MDX_TRY(res_check(E));
     for (int m = 0; m < E->n; ++m) {
         after[m].hist_valid = 0;
         after[m].flip = 0;
@@ -1913,6 +1932,13 @@ int mdx_ensemble_config(mdx_ensemble_t* E, int threads, int blocks_per_sm, int l
     return MDX_OK;
 }
 
+int mdx_ensemble_set_wait_limit(mdx_ensemble_t* E, int polls) {
+    if (!E) return MDX_ERR_ARG;
+    E->rpolls = polls;
+    free_graph(E);   // the limit is a kernel argument
+    return MDX_OK;
+}
+
 int mdx_ensemble_use_graph(mdx_ensemble_t* E, int on) {
     if (!E) return MDX_ERR_ARG;
     E->use_graph = on != 0;
@@ -1964,9 +1990,9 @@ int mdx_ensemble_step(mdx_ensemble_t* E, int nsteps, long long* total_iters) {
         if (after[m].status != MDX_OK && bad < 0) bad = m;
     }
     if (total_iters) *total_iters = it;
+    MDX_TRY(res_check(E));
     if (bad >= 0)
-        return efail(E, after[bad].status == MDX_ERR_NONFINITE ? MDX_ERR_NONFINITE
-                        : after[bad].status == MDX_ERR_TIMEOUT ? MDX_ERR_TIMEOUT : MDX_NOT_CONVERGED,
+        return efail(E, after[bad].status == MDX_ERR_NONFINITE ? MDX_ERR_NONFINITE : MDX_NOT_CONVERGED,
                      "member %d: last projection status %d", bad, after[bad].status);
     return MDX_OK;
 }
@@ -2047,6 +2073,10 @@ int mdx_ensemble_tune(mdx_ensemble_t* E, const char* cache_path, int* threads_ou
                 MDX_TRY(step_eager(E, v, cand_t[ti], grid));
                 ENS_CUDA(E, cudaEventRecord(E->ev[1], E->stream));
                 ENS_CUDA(E, cudaEventSynchronize(E->ev[1]));
+                if (const int rc = res_check(E)) {   // a step cut short is no candidate's time
+                    MDX_TRY(snapshot(E, true));
+                    return rc;
+                }
                 float ms = 0.f;
                 ENS_CUDA(E, cudaEventElapsedTime(&ms, E->ev[0], E->ev[1]));
                 if (ms < best) {
