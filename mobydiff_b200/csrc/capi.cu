@@ -345,6 +345,7 @@ int mdx_set_stream(mdx_ctx_t* ctx, void* stream) {
     cudaStreamSynchronize(ctx->stream);
     release_graph(ctx);
     ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
+    ctx->rs_refused = false;
     return MDX_OK;
 }
 

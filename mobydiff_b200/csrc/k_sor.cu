@@ -892,9 +892,14 @@ static int sor_iterate(mdx_ctx_t* ctx, const mdx_sor_params& p, int variant) {
     return sor_iteration(ctx, p);
 }
 
-static int sor_iterations(mdx_ctx_t* ctx, const mdx_sor_params& p, int variant, int n) {
-    if (variant == MDX_SORV_RESIDENT) return n > 0 ? mdx_res_face64_run(ctx, p, n) : MDX_OK;
-    for (int it = 0; it < n; ++it) MDX_TRY(sor_iterate(ctx, p, variant));
+// *variant: plain sweeps where the device refuses the on-chip run.
+static int sor_iterations(mdx_ctx_t* ctx, const mdx_sor_params& p, int* variant, int n) {
+    if (*variant == MDX_SORV_RESIDENT) {
+        const int rc = n > 0 ? mdx_res_face64_run(ctx, p, n) : MDX_OK;
+        if (rc != MDX_RES_REFUSED) return rc;
+        *variant = MDX_SORV_SWEEPS;
+    }
+    for (int it = 0; it < n; ++it) MDX_TRY(sor_iterate(ctx, p, *variant));
     return MDX_OK;
 }
 
@@ -1005,6 +1010,7 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
         return MDX_OK;
     };
     auto pick = [&]() -> int {
+        if (want == MDX_SORV_RESIDENT && ctx->rs_refused) want = MDX_SORV_SWEEPS;
         if (want != MDX_SORV_AUTO) return want;
         if (ctx->sor_tuned > 0) return ctx->sor_tuned;
         auto out = [&](int v) { return !pass_fits(ctx) && (v == MDX_SORV_FUSED8 || v == MDX_SORV_FUSED16); };
@@ -1019,7 +1025,7 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     mdx_solve_stats_t s{};
     s.guessed = guessed ? 1 : 0;
     if (o.tol <= 0.0) {
-        const int v = fixed_v;
+        int v = fixed_v;
         if (!copy_in_sweep) MDX_TRY(layout_for(v));
         if (copy_in_sweep && fixed_pass) MDX_TRY(pass_alloc(ctx));
         mdx_event_pair run{};
@@ -1038,7 +1044,7 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
             }
         } else {
             if (copy_in_sweep) MDX_TRY(sor_iteration(ctx, p, true));
-            MDX_TRY(sor_iterations(ctx, p, v, o.n_iter - (copy_in_sweep ? 1 : 0)));
+            MDX_TRY(sor_iterations(ctx, p, &v, o.n_iter - (copy_in_sweep ? 1 : 0)));
         }
         mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT || (copy_in_sweep && !fixed_pass) ? 2LL * o.n_iter
                                      : copy_in_sweep ? o.n_iter : -1);
@@ -1063,13 +1069,13 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
             int block = cs.every;
             while (it < o.max_iter) {
                 const int m = std::min(block, o.max_iter - it);
-                const int v = pick();
+                int v = pick();
                 MDX_TRY(layout_for(v));
                 const bool timing_block = want == MDX_SORV_AUTO && ctx->sor_tuned == 0;
                 if (timing_block) MDX_CUDA(ctx, cudaEventRecord(ctx->tune_ev[0], ctx->stream));
                 mdx_event_pair run{};
                 mdx_sweep_run_begin(ctx, &run);
-                MDX_TRY(sor_iterations(ctx, p, v, m));
+                MDX_TRY(sor_iterations(ctx, p, &v, m));
                 mdx_sweep_run_end(ctx, &run, v == MDX_SORV_RESIDENT ? 2LL * m : -1);
                 if (timing_block) MDX_CUDA(ctx, cudaEventRecord(ctx->tune_ev[1], ctx->stream));
                 it += m;

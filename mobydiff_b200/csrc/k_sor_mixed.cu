@@ -1418,8 +1418,8 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
             if (pot_shape_ok(ctx, c)) pcands[npc++] = c;
     // where the state fits the SMs the on-chip runs are taken without tuning:
     // they were the fastest on every such grid measured
-    const bool on_chip = pot ? (o.sor_variant < 1 || o.sor_variant > POT_SHAPES) && mdx_res_pot_ok(ctx)
-                             : (o.sor_variant < 1 || o.sor_variant > MDX_SORV_SPLITV) && mdx_res_face32_ok(ctx);
+    bool on_chip = pot ? (o.sor_variant < 1 || o.sor_variant > POT_SHAPES) && mdx_res_pot_ok(ctx)
+                       : (o.sor_variant < 1 || o.sor_variant > MDX_SORV_SPLITV) && mdx_res_face32_ok(ctx);
     if (pot && npc > 1 && !ctx->tune_ev[0]) {
         MDX_CUDA(ctx, cudaEventCreate(&ctx->tune_ev[0]));
         MDX_CUDA(ctx, cudaEventCreate(&ctx->tune_ev[1]));
@@ -1464,10 +1464,12 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
         if (on_chip) {
             mdx_event_pair run{};
             mdx_sweep_run_begin(ctx, &run);
-            MDX_TRY(pot ? mdx_res_pot_run(ctx, L, iters) : mdx_res_face32_run(ctx, P, iters));
-            mdx_sweep_run_end(ctx, &run, 2LL * iters);
+            const int rc = pot ? mdx_res_pot_run(ctx, L, iters) : mdx_res_face32_run(ctx, P, iters);
+            on_chip = rc != MDX_RES_REFUSED;
+            if (on_chip) MDX_TRY(rc);
+            mdx_sweep_run_end(ctx, &run, on_chip ? 2LL * iters : 0);
             used_kind = pot ? 7 : 1;
-            return MDX_OK;
+            if (on_chip) return MDX_OK;
         }
         if (pot) return pot_sweeps(iters);
         mdx_event_pair run{};

@@ -423,8 +423,15 @@ int res_launch(mdx_ctx_t* ctx, const char* what, F fn, const res_plan& P, int it
     void* av[] = {&args...};
     mdx_event_pair p{};
     mdx_timer_begin(ctx, MDX_T_SOR_SWEEP, &p);
-    MDX_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)fn, dim3(P.blocks), dim3(P.threads), av, P.smem, ctx->stream));
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel((const void*)fn, dim3(P.blocks), dim3(P.threads), av, P.smem, ctx->stream);
     mdx_timer_end(ctx, &p);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        cudaGetLastError();
+        ctx->rs_refused = true;
+        return MDX_RES_REFUSED;
+    }
+    MDX_CUDA(ctx, e);
     ctx->rs_seq += 2u * (unsigned)iters;
     return mdx_check_launch(ctx, what);
 }
@@ -479,15 +486,15 @@ int face32_run(mdx_ctx_t* ctx, const mixed_params& q, const res_plan& P, int ite
 
 bool mdx_res_pot_ok(mdx_ctx_t* ctx) {
     res_plan P;
-    return pot_plan(ctx, &P) && !capturing(ctx);
+    return !ctx->rs_refused && pot_plan(ctx, &P) && !capturing(ctx);
 }
 bool mdx_res_face32_ok(mdx_ctx_t* ctx) {
     res_plan P;
-    return face_plan<float>(ctx, face32_shapes, 12, &P) && !capturing(ctx);
+    return !ctx->rs_refused && face_plan<float>(ctx, face32_shapes, 12, &P) && !capturing(ctx);
 }
 bool mdx_res_face64_ok(mdx_ctx_t* ctx) {
     res_plan P;
-    return ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL &&
+    return !ctx->rs_refused && ctx->bc.is_periodic[0] && ctx->bc.is_periodic[2] && ctx->mu_mode != MU_FULL &&
            face_plan<double>(ctx, face64_shapes, 18, &P) && !capturing(ctx);
 }
 
@@ -522,4 +529,5 @@ void mdx_res_free(mdx_ctx_t* ctx) {
     ctx->rs_box = nullptr;
     ctx->rs_bytes = 0;
     ctx->rs_seq = 0;
+    ctx->rs_refused = false;
 }

@@ -12,7 +12,11 @@ bool mdx_res_pot_ok(mdx_ctx_t* ctx);
 bool mdx_res_face32_ok(mdx_ctx_t* ctx);
 bool mdx_res_face64_ok(mdx_ctx_t* ctx);
 // `iters` red-black iterations in one launch on, respectively, Phi, the FP32
-// corrections and the FP64 fields.
+// corrections and the FP64 fields.  MDX_RES_REFUSED: the device did not take
+// the cooperative launch (a stream that has part of the SMs only); nothing ran,
+// the caller sweeps with its other kernels, and the functions above say no from
+// then on, until the solver is set up again or the stream changes.
+enum { MDX_RES_REFUSED = -1 };
 int mdx_res_pot_run(mdx_ctx_t* ctx, const pot_geom& L, int iters);
 int mdx_res_face32_run(mdx_ctx_t* ctx, const mixed_params& P, int iters);
 struct mdx_sor_params;

@@ -1,0 +1,58 @@
+"""A device that refuses cooperative launches (cudaErrorCooperativeLaunchTooLarge,
+as a stream with part of the SMs gets it): the red-black solves run with their
+other kernels and give the same bits.  The refusal is made on the host, by a
+cudaLaunchCooperativeKernel of the test's own that a child process loads first."""
+import os
+import shutil
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+CHILD = """
+import sys
+import numpy as np
+import mobydiff_b200 as M
+from tests.helpers import channel_case, random_fields, to_device
+
+g, bc = channel_case(64, 32, 32)
+f = random_fields(g, 11, "zinv", scale=0.1)
+f.vs[:, 1, :] = f.vs[:, g.ny + 1, :] = 0.0
+out = {}
+for name, kw in (("fixed", dict(n_iter=5)), ("tol", dict(tol=1e-3)), ("pot", dict(tol=1e-3, precision=M.PREC_MIXED)),
+                 ("face", dict(tol=1e-3, precision=M.PREC_MIXED, inner_form=1))):
+    with to_device(M, g, bc, f) as s:
+        s.init_pressure_solver(M.make_solver_opts(M.SOLVER_REDBLACK, sor=1.7, adaptive_checks=False, **kw))
+        for p in range(2):
+            st = s.pressure_projection(1e-3)
+            out["%s%d" % (name, p)] = np.array([st.iterations, st.variant])
+        for n in ("un", "vn", "wn", "pn"):
+            out[name + n] = s.get(n)
+np.savez(sys.argv[1], **out)
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="needs gcc")
+def test_refused_cooperative_launch_falls_back(tmp_path):
+    src, shim = tmp_path / "refuse.c", tmp_path / "refuse.so"
+    src.write_text("int cudaLaunchCooperativeKernel(void) { return 720; }\n")   # cudaErrorCooperativeLaunchTooLarge
+    subprocess.check_call(["gcc", "-shared", "-fPIC", str(src), "-o", str(shim)])
+    out = []
+    for preload in ("", str(shim)):
+        env = dict(os.environ, PYTHONPATH=ROOT)
+        if preload:
+            env["LD_PRELOAD"] = preload
+        f = tmp_path / ("b.npz" if preload else "a.npz")
+        subprocess.run([sys.executable, "-c", CHILD, str(f)], cwd=ROOT, env=env, check=True, timeout=300)
+        out.append(dict(np.load(f)))
+    a, b = out
+    assert a["fixed0"][1] == 6 and b["fixed0"][1] == 1   # the shim is what ran
+    for k in a:
+        if k[-1] in "01":
+            assert a[k][0] == b[k][0], k
+        else:
+            assert np.array_equal(a[k], b[k]), k
