@@ -676,9 +676,13 @@ __device__ __forceinline__ void guess_cell(const ens_member& M, double dg, unsig
 // MINB 1: registers for the predictor (one block of 512 per SM); MINB 2:
 // 64 registers (spills in the predictor), twice the resident warps for
 // the latency-bound sweeps.  The autotuner picks one.
-template <int MINB>
+// RES: with the on-chip sweeps, in the full-register variant (the other has no
+// room for them) of batches that may run them.  Their registers cost the rest
+// of the kernel 360 bytes of spills: potential-form batches, which never run
+// them, took 17.9 ms a step without and 18.8 with them (241 and 259 ms for 24
+// members).
+template <int MINB, bool RES>
 __global__ void __launch_bounds__(MAX_THREADS, MINB) k_ens_substage(ens_args A) {
-    constexpr bool RES = MINB == 1;   // the 64-register variant has no room for the on-chip sweeps
     cg::grid_group grid = cg::this_grid();
     const int s = A.substage;
     const bool warm = A.momentum && A.guess_mode != MDX_GUESS_ZERO;
@@ -1278,10 +1282,6 @@ void free_graph(mdx_ensemble_t* E) {
     E->graph = nullptr;
 }
 
-const void* kernel_of(int variant) {
-    return variant ? (const void*)k_ens_substage<2> : (const void*)k_ens_substage<1>;
-}
-
 // Whether the on-chip sweeps may be used at all (FP32 faces, the
 // full-register variant), the shared memory they take per block and the words
 // of an inbox: the largest box a block of `threads` can hold of any member.
@@ -1303,12 +1303,18 @@ int res_smem(const mdx_ensemble_t* E, int variant, int threads) {
     return res_shape(E, variant, threads, &smem, &stride) ? smem : 0;
 }
 
+const void* kernel_of(const mdx_ensemble_t* E, int variant, int threads) {
+    if (variant) return (const void*)k_ens_substage<2, false>;
+    return res_smem(E, variant, threads) ? (const void*)k_ens_substage<1, true> : (const void*)k_ens_substage<1, false>;
+}
+
 int grid_for(mdx_ensemble_t* E, int variant, int threads, int bps, int* grid) {
     int occ = 0;
     const int smem = res_smem(E, variant, threads);
+    const void* fn = kernel_of(E, variant, threads);
     if (smem > 48 * 1024)
-        ENS_CUDA(E, cudaFuncSetAttribute(kernel_of(variant), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_of(variant), threads, smem));
+        ENS_CUDA(E, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem));
     int sms = 0;
     ENS_CUDA(E, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
     if (occ < 1) return efail(E, MDX_ERR_ARG, "ensemble kernel does not fit %d threads per block", threads);
@@ -1419,7 +1425,7 @@ int launch_substage(mdx_ensemble_t* E, int s, int momentum, int variant, int thr
         smem = res_smem(E, variant, threads);
     }
     void* args[] = {&A};
-    ENS_CUDA(E, cudaLaunchCooperativeKernel(kernel_of(variant), dim3(grid), dim3(threads), args, smem, E->stream));
+    ENS_CUDA(E, cudaLaunchCooperativeKernel(kernel_of(E, variant, threads), dim3(grid), dim3(threads), args, smem, E->stream));
     E->launches++;
     return MDX_OK;
 }
@@ -2062,7 +2068,7 @@ int mdx_ensemble_tune(mdx_ensemble_t* E, const char* cache_path, int* threads_ou
     for (int v = 0; v < 2; ++v)
         for (int ti = 0; ti < 3; ++ti) {
             int occ = 0;
-            ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_of(v), cand_t[ti], 0));
+            ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_of(E, v, cand_t[ti]), cand_t[ti], 0));
             for (int bi = 0; bi < 4; ++bi) {
                 if (cand_b[bi] > occ) continue;
                 int grid = 0;
