@@ -1282,10 +1282,19 @@ void free_graph(mdx_ensemble_t* E) {
     E->graph = nullptr;
 }
 
+// Iterations of a round that pay for taking the boxes on chip and back: ms a
+// step on chip / with grid barriers, six members of 49 k to 196 k cells (two
+// of 33 k and 49 k): check_every 2 45.5 / 42.6 (7.3 / 6.2), 3 32.4 / 33.8 (5.3
+// / 4.9), 4 26.3 / 29.6 (4.36 / 4.32), 6 19.7 / 25.4 (3.4 / 3.8), 15 12.0 /
+// 20.3 (2.1 / 2.9).
+constexpr int RES_ROUND = 4;
+
 // Whether the on-chip sweeps may be used at all (FP32 faces, the
-// full-register variant), the shared memory they take per block and the words
-// of an inbox: the largest box a block of `threads` can hold of any member.
+// full-register variant, rounds long enough), the shared memory they take per
+// block and the words of an inbox: the largest box a block of `threads` can
+// hold of any member.
 bool res_shape(const mdx_ensemble_t* E, int variant, int threads, int* smem, int* stride) {
+    if (E->opts.check_every < RES_ROUND) return false;
     if (variant != 0 || E->opts.precision != MDX_PREC_MIXED || !(E->opts.tol > 0.0) || E->opts.inner_form == 2) return false;
     *smem = *stride = 0;
     for (const auto& M : E->hm) {

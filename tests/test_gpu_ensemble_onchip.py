@@ -37,7 +37,7 @@ def _run(name, opts, threads, low_regs):
 
 
 @pytest.mark.parametrize("name", list(BATCHES))
-@pytest.mark.parametrize("form,check_every", [(1, 25), (1, 7), (1, 3), (2, 25)])
+@pytest.mark.parametrize("form,check_every", [(1, 25), (1, 7), (1, 4), (1, 3), (2, 25)])
 @pytest.mark.parametrize("threads", [256, 512])
 def test_on_chip_rounds_equal_grid_barriers(name, form, check_every, threads):
     a = _run(name, _opts(form, check_every), threads, False)
@@ -46,11 +46,12 @@ def test_on_chip_rounds_equal_grid_barriers(name, form, check_every, threads):
     assert all(np.array_equal(x, y) for x, y in zip(a[2], b[2]))
 
 
-@pytest.mark.parametrize("form,precision,low_regs,on_chip", [
-    (0, M.PREC_MIXED, False, True), (1, M.PREC_MIXED, False, True), (0, M.PREC_MIXED, True, False),
-    (2, M.PREC_MIXED, False, False), (0, M.PREC_FP64, False, False)])
-def test_which_batches_go_on_chip(form, precision, low_regs, on_chip):
-    with M.Ensemble(_members("uneven"), _opts(form, 25, precision)) as E:
+@pytest.mark.parametrize("form,precision,low_regs,check_every,on_chip", [
+    (0, M.PREC_MIXED, False, 25, True), (1, M.PREC_MIXED, False, 25, True), (0, M.PREC_MIXED, True, 25, False),
+    (2, M.PREC_MIXED, False, 25, False), (0, M.PREC_FP64, False, 25, False), (0, M.PREC_MIXED, False, 4, True),
+    (0, M.PREC_MIXED, False, 3, False)])
+def test_which_batches_go_on_chip(form, precision, low_regs, check_every, on_chip):
+    with M.Ensemble(_members("uneven"), _opts(form, check_every, precision)) as E:
         E.config(512, 0, low_regs=low_regs)
         E.ic()
         E.set_wait_limit(0)
