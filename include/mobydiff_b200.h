@@ -424,7 +424,8 @@ int mdx_ensemble_config(mdx_ensemble_t* ens, int threads, int blocks_per_sm, int
 int mdx_ensemble_set_wait_limit(mdx_ensemble_t* ens, int polls);
 /* Time one step of each candidate launch shape from the same saved state and
  * keep the fastest; the choice is cached in the JSON file cache_path (may be
- * NULL) under a key of the member sizes, the mode and the device name
+ * NULL) under a key of the member sizes, the mode, the precision and form of
+ * the sweeps and the device name
  * (*ms = -1 when it came from the cache). */
 int mdx_ensemble_tune(mdx_ensemble_t* ens, const char* cache_path, int* threads, int* blocks_per_sm, int* low_regs,
                       double* ms);

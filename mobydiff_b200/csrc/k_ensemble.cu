@@ -1317,13 +1317,19 @@ const void* kernel_of(const mdx_ensemble_t* E, int variant, int threads) {
     return res_smem(E, variant, threads) ? (const void*)k_ens_substage<1, true> : (const void*)k_ens_substage<1, false>;
 }
 
-int grid_for(mdx_ensemble_t* E, int variant, int threads, int bps, int* grid) {
-    int occ = 0;
+// Resident blocks per SM, with the shared memory the launch will ask for.
+int occupancy(mdx_ensemble_t* E, int variant, int threads, int* occ) {
     const int smem = res_smem(E, variant, threads);
     const void* fn = kernel_of(E, variant, threads);
     if (smem > 48 * 1024)
         ENS_CUDA(E, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem));
+    ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, fn, threads, smem));
+    return MDX_OK;
+}
+
+int grid_for(mdx_ensemble_t* E, int variant, int threads, int bps, int* grid) {
+    int occ = 0;
+    MDX_TRY(occupancy(E, variant, threads, &occ));
     int sms = 0;
     ENS_CUDA(E, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
     if (occ < 1) return efail(E, MDX_ERR_ARG, "ensemble kernel does not fit %d threads per block", threads);
@@ -1515,6 +1521,10 @@ std::string tune_key(const mdx_ensemble_t* E) {
     }
     mix((uint64_t)E->guess_mode);
     mix((uint64_t)(E->opts.tol > 0.0));
+    // what decides which kernel a variant is
+    mix((uint64_t)E->opts.precision);
+    mix((uint64_t)(E->opts.inner_form == 2));
+    mix((uint64_t)(E->opts.check_every >= RES_ROUND));
     cudaDeviceProp prop{};
     cudaGetDeviceProperties(&prop, E->device);
     char hex[17];
@@ -2077,7 +2087,7 @@ int mdx_ensemble_tune(mdx_ensemble_t* E, const char* cache_path, int* threads_ou
     for (int v = 0; v < 2; ++v)
         for (int ti = 0; ti < 3; ++ti) {
             int occ = 0;
-            ENS_CUDA(E, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_of(E, v, cand_t[ti]), cand_t[ti], 0));
+            MDX_TRY(occupancy(E, v, cand_t[ti], &occ));
             for (int bi = 0; bi < 4; ++bi) {
                 if (cand_b[bi] > occ) continue;
                 int grid = 0;

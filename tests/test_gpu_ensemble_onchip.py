@@ -61,3 +61,24 @@ def test_which_batches_go_on_chip(form, precision, low_regs, check_every, on_chi
             assert e.value.code == M.MDX_ERR_TIMEOUT
         else:
             E.step(1)
+
+
+def test_tuned_shapes_are_kept_per_kind_of_sweep(tmp_path):
+    """The same members in FP64, mixed face form, mixed with short rounds and
+    mixed potential form run different kernels: one cache entry each, and a
+    second ensemble of a kind takes its own."""
+    import json
+    cache = str(tmp_path / "tune.json")
+    kinds = [_opts(0, 25, M.PREC_FP64), _opts(0, 25), _opts(0, 3), _opts(2, 25)]
+    chosen = []
+    for n, opts in enumerate(kinds):
+        with M.Ensemble(_members("one"), opts) as E:
+            E.ic()
+            chosen.append(E.tune(cache))
+            assert chosen[-1][3] > 0.0           # timed, not another kind's entry
+            assert E.info()["grid"] % chosen[-1][1] == 0
+        assert len(json.load(open(cache))) == n + 1
+    for opts, c in zip(kinds, chosen):
+        with M.Ensemble(_members("one"), opts) as E:
+            E.ic()
+            assert E.tune(cache) == c[:3] + (-1.0,)
