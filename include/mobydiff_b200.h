@@ -93,7 +93,8 @@ typedef struct {
     int precision;     /* MDX_PREC_*                                          */
     int sor_variant;   /* red-black kernels (bit-identical results): 0 auto -- where the
                           whole state fits the SMs (about 1 M cells in FP64, 4 M in
-                          FP32), one launch per run of sweeps with the state on chip;
+                          FP32), one launch per run of sweeps with the state on chip
+                          (fixed counts from 3 iterations, 4 above 600 000 cells);
                           else the first projection times each variant on one residual-check
                           block of its own iterations and keeps the fastest; 1 one
                           launch per colour; 2 red+black pass, 60x5 tiles; 3 the same,

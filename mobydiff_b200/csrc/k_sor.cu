@@ -936,13 +936,22 @@ int mdx_k_projection_redblack(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t* st) 
     const bool fok = fused_ok(ctx);
     int want = ctx->opts.sor_variant;
     if (want < MDX_SORV_AUTO || want > MDX_SORV_RESIDENT) want = MDX_SORV_AUTO;
-    // where the state fits the SMs the on-chip run is taken without tuning:
-    // it was the fastest on every such grid measured
+    const bool warm = mdx_guess_supported(ctx) && (ctx->guess_mode != MDX_GUESS_ZERO || ctx->record_increments);
+    // Where the state fits the SMs the on-chip run is taken without tuning:
+    // to a tolerance it was the fastest on every grid and check_every measured
+    // (ms a step, on chip / colour sweeps: 116x70x62 3.48 / 3.80 checking every
+    // iteration, 1.57 / 2.80 every 50; 128x64x64 2.94 / 3.25 and 1.31 / 2.83).
+    // A short fixed count pays more for the copies of u* and for taking the
+    // boxes on chip and back than the sweeps that read u* (us a step, 1, 2, 3,
+    // 4 iterations: 32x24x32 112 130 136 149 / 99 124 149 173, 128x64x64 204
+    // 226 237 256 / 153 204 253 302, 128x96x80 320 351 379 408 / 210 284 356
+    // 431).
+    const int least = d.nint > 600000 ? 4 : 3;
+    const bool brief = want == MDX_SORV_AUTO && o.tol <= 0.0 && o.n_iter < least && !warm;
     if ((want == MDX_SORV_AUTO || want == MDX_SORV_RESIDENT))
-        want = mdx_res_face64_ok(ctx) ? MDX_SORV_RESIDENT : MDX_SORV_AUTO;
+        want = !brief && mdx_res_face64_ok(ctx) ? MDX_SORV_RESIDENT : MDX_SORV_AUTO;
     if (want != MDX_SORV_SWEEPS && !fok) want = MDX_SORV_SWEEPS;
     if ((want == MDX_SORV_FUSED8 || want == MDX_SORV_FUSED16) && !pass_fits(ctx)) want = MDX_SORV_SWEEPS;
-    const bool warm = mdx_guess_supported(ctx) && (ctx->guess_mode != MDX_GUESS_ZERO || ctx->record_increments);
     // :63-84 -- u <- u* over the whole padded arrays; a fixed number of plain
     // sweeps does it in its first sweep (three copies of 30 MB, 35 us, on
     // 180x150x140)

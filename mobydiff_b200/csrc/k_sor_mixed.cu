@@ -1416,8 +1416,12 @@ int mdx_k_projection_redblack_mixed(mdx_ctx_t* ctx, double dg, mdx_solve_stats_t
     else if (pot)
         for (int c = 0; c < POT_SHAPES; ++c)
             if (pot_shape_ok(ctx, c)) pcands[npc++] = c;
-    // where the state fits the SMs the on-chip runs are taken without tuning:
-    // they were the fastest on every such grid measured
+    // Where the state fits the SMs the on-chip runs are taken without tuning:
+    // they were the fastest on the grids measured (ms a step, on chip / the best
+    // of the others, checking every iteration and every 50: potential form
+    // 116x70x62 2.94 / 3.65 and 1.11 / 2.40, 256x128x128 28.3 / 29.7 and 15.0 /
+    // 20.4; faces 116x70x62 2.98 / 3.36 and 1.10 / 2.41), but for 128x64x64
+    // checking every iteration (2.81 / 2.53 and, faces, 2.94 / 2.88).
     bool on_chip = pot ? (o.sor_variant < 1 || o.sor_variant > POT_SHAPES) && mdx_res_pot_ok(ctx)
                        : (o.sor_variant < 1 || o.sor_variant > MDX_SORV_SPLITV) && mdx_res_face32_ok(ctx);
     if (pot && npc > 1 && !ctx->tune_ev[0]) {
