@@ -172,7 +172,7 @@ SOR_NAMES = {1: "one launch per colour sweep", 2: "red+black pass, 60x5 tiles", 
 SOR32_NAMES = {1: "k_sor_sweep32: one launch per colour, one cell per thread",
                3: "k_rb32_fused: one launch per red+black iteration",
                5: "k_sor_sweep32v: one launch per colour, 2 or 4 cells per thread",
-               7: "potential form: k_pot_resident (a block of iterations per cooperative launch, phi in registers) "
+               7: "potential form: k_pot_resident (a block of iterations per cooperative launch, phi in shared memory) "
                   "where the grid fits the SMs, as 256x128x128 does; else the autotuner's pick among k_pot_sweep, "
                   "k_pot_sweep_w, k_pot_sweep_a and k_pot_run_w"}
 SOR32_TRAFFIC = {1: "sor_sweep32", 3: "rb32_fused", 5: "sor_sweep32v", 7: "pot_resident"}
@@ -469,6 +469,16 @@ def _roofline(tim, kname, alg_per_cell, cells, ms, traffic_key=None):
             "share_of_step_time": kms / ms if ms > 0 else None}
 
 
+def _on_chip(roofline, kind):
+    """Sweeps whose state stays on the SMs for a whole run of iterations: the
+    bytes they count never reach HBM, so there is no fraction of it to state."""
+    roofline.update(bound="on chip", peak=None, frac=None,
+                    note="the state stays in registers and shared memory for a run of sweeps; HBM carries it once a "
+                         "run" + ("; on 256x128x128 issue slots 39 %, shared-memory pipe 35 %, FMA pipe 14 % busy "
+                                  "(profiles/on_chip_and_pass.md), the rest is the exchange between neighbouring SMs"
+                                  if kind == 7 else ""))
+
+
 def _sor_alg_per_launch(variant, fp32=False):
     """Algorithmic bytes per cell of one sweep launch: 4 arrays read and
     written for the cells of one colour (FP64 32 B, FP32 16 B per cell of
@@ -603,6 +613,8 @@ def run_plain(args, cfg):
         var = s.last_solve_stats().variant
         roofline = _roofline(tim, "sor_run", _sor_alg_per_launch(var), cells, ms,
                              traffic_key=_sor64_traffic_key(var))
+        if var == 6:
+            _on_chip(roofline, var)
         step_hbm = _step_hbm(cells, ms_all / args.steps, iters / args.steps, 64.0)
     else:
         roofline = _roofline(tim, "momentum", 112.0, cells, ms)   # 14 doubles per cell
@@ -1131,6 +1143,8 @@ def run_learned_mixed(args, cfg):
     roof64 = _roofline(p_tim, "sor_run", _sor_alg_per_launch(var64), cells, r_ms,
                        traffic_key=_sor64_traffic_key(var64))
     roof64["sor_kernel"] = SOR_NAMES.get(var64, "?")
+    if var64 == 6:
+        _on_chip(roof64, var64)
     plain_step_hbm = _step_hbm(cells, p_ms_all / K, p_iters / K, 64.0)
     plain_c1 = None
     if not args.quick:   # the plain FP64 step at the C1 tolerance 1e-10
@@ -1206,6 +1220,7 @@ def run_learned_mixed(args, cfg):
     # ---- the same steps with the sweep runs timed, for the roofline ------------
     s.warm_checkpoint(restore=True)
     s.update_device(*[h.numpy() for h in host])
+    l0 = s.launch_count()
     _, r_ms, _, _, tim = _timed_steps(s, stream, K, pg, timing=2)
     # 4 floats per cell per colour sweep; the FP32 sweep kernel the autotuner
     # kept is the hundreds digit of the solve's variant
@@ -1213,9 +1228,8 @@ def run_learned_mixed(args, cfg):
     roofline = _roofline(tim, "sor_run", SOR32_ALG.get(kind, 16.0), cells, r_ms,
                          traffic_key=SOR32_TRAFFIC.get(kind, "sor_sweep32"))
     roofline["sor_kernel"] = SOR32_NAMES.get(kind, "?")
-    if kind == 7:
-        roofline["note"] = ("phi and r~ stay in registers across the sweeps of a run, so the sweeps "
-                            "can pass the HBM copy rate")
+    if s.launch_count() - l0 < tim["sor_run"][1]:   # runs of sweeps in one launch each
+        _on_chip(roofline, kind)
     step_hbm = _step_hbm(cells, ms_all / K, iters / K, 16.0 if kind == 7 else 32.0)
 
     # ---- the same steps without the network: extrapolated increment only ----

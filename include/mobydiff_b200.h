@@ -92,8 +92,10 @@ typedef struct {
     int check_every;   /* red-black: iterations between residual checks       */
     int precision;     /* MDX_PREC_*                                          */
     int sor_variant;   /* red-black kernels (bit-identical results): 0 auto -- where the
-                          whole state fits the SMs (about 1 M cells in FP64, 4 M in
-                          FP32), one launch per run of sweeps with the state on chip
+                          whole state fits the SMs (up to about 1 M cells in FP64 and
+                          1.8 M in FP32 faces, nx <= 256; 4 M and nx <= 512 in
+                          FP32 potentials), one launch per run of sweeps with the
+                          state on chip
                           (fixed counts from 3 iterations, 4 above 600 000 cells);
                           else the first projection times each variant on one residual-check
                           block of its own iterations and keeps the fastest; 1 one

@@ -27,8 +27,8 @@
 // where they are used, 64 registers and no prefetch it ran at 3.9 TB/s
 // whatever the tile (32 x 4 to 128 x 2, 8 to 32 planes, 2 to 8 blocks per SM):
 // 895 us on 512x256x256, every warp waiting for DRAM four times a plane.  The
-// reads at the top 865, 80 registers (no spills) 795, the next plane's DRAM
-// reads prefetched into L2 580 us (6.0 TB/s).
+// reads at the top 865, 80 registers (4 bytes of spills, 68 with IBM factors)
+// 795, the next plane's DRAM reads prefetched into L2 580 us (6.0 TB/s).
 // GH: the ghost values of u*, v*, w* are set too (bc_fft_ghosts).
 template <bool IBM, bool DTD, int KZ, bool GH>
 __global__ void __launch_bounds__(256, 3)
@@ -117,7 +117,7 @@ int mdx_k_momentum(mdx_ctx_t* ctx, mdx_dscal da, mdx_dscal db, mdx_dscal dg, boo
     const mdx_dims& d = ctx->d;
     dim3 block(32, 8, 1);
     // planes per block: 8 (the values carried from plane to plane), fewer while
-    // the blocks would not give every SM four (its resident blocks)
+    // the blocks would not give every SM four (three are resident)
     dim3 grid((d.nx + 31) / 32, (d.ny + 7) / 8);
     int kz = 8;
     while (kz > 1 && (long long)grid.x * grid.y * ((d.nz + kz - 1) / kz) < 4 * 148) kz = kz == 8 ? 2 : 1;
