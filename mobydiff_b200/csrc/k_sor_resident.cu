@@ -406,7 +406,12 @@ int res_prepare(mdx_ctx_t* ctx, const res_plan& P, int iters) {
         cudaFree(ctx->rs_box);
         ctx->rs_box = nullptr;
         ctx->rs_bytes = 0;
-        MDX_CUDA(ctx, cudaMalloc(&ctx->rs_box, bytes));
+        if (cudaMalloc(&ctx->rs_box, bytes) != cudaSuccess) {   // no room: the sweeps need none
+            cudaGetLastError();
+            ctx->rs_box = nullptr;
+            ctx->rs_refused = true;
+            return MDX_RES_REFUSED;
+        }
         ctx->rs_bytes = bytes;
         ctx->rs_seq = 0;
     }

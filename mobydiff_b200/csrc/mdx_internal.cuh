@@ -164,7 +164,7 @@ struct mdx_ctx {
     void* rs_box = nullptr;
     size_t rs_bytes = 0;
     unsigned rs_seq = 0;
-    bool rs_refused = false;                 // the device refused a cooperative launch
+    bool rs_refused = false;                 // no cooperative launch or no room for the inboxes
     int rs_polls = -1;                       // mdx_set_wait_limit
     // warm starts: increments of the last projection of each RK substage
     int guess_mode = 0;                      // MDX_GUESS_*

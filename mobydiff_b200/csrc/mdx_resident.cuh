@@ -13,7 +13,8 @@ bool mdx_res_face32_ok(mdx_ctx_t* ctx);
 bool mdx_res_face64_ok(mdx_ctx_t* ctx);
 // `iters` red-black iterations in one launch on, respectively, Phi, the FP32
 // corrections and the FP64 fields.  MDX_RES_REFUSED: the device did not take
-// the cooperative launch (a stream that has part of the SMs only); nothing ran,
+// the cooperative launch (a stream that has part of the SMs only) or has no
+// memory left for the inboxes; nothing ran,
 // the caller sweeps with its other kernels, and the functions above say no from
 // then on, until the solver is set up again or the stream changes.
 enum { MDX_RES_REFUSED = -1 };

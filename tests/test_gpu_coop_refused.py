@@ -1,7 +1,8 @@
 """A device that refuses cooperative launches (cudaErrorCooperativeLaunchTooLarge,
-as a stream with part of the SMs gets it): the red-black solves run with their
-other kernels and give the same bits.  The refusal is made on the host, by a
-cudaLaunchCooperativeKernel of the test's own that a child process loads first."""
+as a stream with part of the SMs gets it), or has no memory left for the on-chip
+runs' inboxes: the red-black solves run with their other kernels and give the
+same bits.  The refusal is made on the host, by a cudaLaunchCooperativeKernel or
+a cudaMalloc of the test's own that a child process loads first."""
 import os
 import shutil
 import subprocess
@@ -56,3 +57,53 @@ def test_refused_cooperative_launch_falls_back(tmp_path):
             assert a[k][0] == b[k][0], k
         else:
             assert np.array_equal(a[k], b[k]), k
+
+
+NO_ROOM = """
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+int refuse = 0, refused = 0;
+int cudaMalloc(void** p, size_t n) {
+    static int (*real)(void**, size_t);
+    if (refuse) { ++refused; return 2; }   /* cudaErrorMemoryAllocation */
+    /* the library is not in the global scope: by name, already loaded */
+    if (!real) real = (int (*)(void**, size_t))dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), "cudaMalloc");
+    return real(p, n);
+}
+"""
+
+CHILD_NO_ROOM = """
+import ctypes as C
+import sys
+import numpy as np
+import mobydiff_b200 as M
+from oracle import oracle as O
+from tests.helpers import channel_case, random_fields, to_device
+
+shim = C.CDLL(sys.argv[1])
+refuse, refused = C.c_int.in_dll(shim, "refuse"), C.c_int.in_dll(shim, "refused")
+g, bc = channel_case(64, 32, 32)
+f = random_fields(g, 11, scale=0.1)
+with to_device(M, g, bc, f) as s:
+    s.init_pressure_solver(M.make_solver_opts(M.SOLVER_REDBLACK, sor=1.7, n_iter=5))
+    refuse.value = 1
+    st = s.pressure_projection(1e-3)
+    refuse.value = 0
+    assert refused.value > 0 and st.variant == 1, (refused.value, st.variant)
+    O.pressure_projection_redblack(g, bc, f, 1e-3, niter=5, sor=1.7, tol=0.0)
+    for n in ("un", "vn", "wn", "pn"):
+        assert np.array_equal(s.get(n), getattr(f, n)), n
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="needs gcc")
+def test_no_room_for_the_inboxes_falls_back(tmp_path):
+    src, shim = tmp_path / "full.c", tmp_path / "full.so"
+    src.write_text(NO_ROOM)
+    subprocess.check_call(["gcc", "-shared", "-fPIC", str(src), "-o", str(shim), "-ldl"])
+    env = dict(os.environ, PYTHONPATH=ROOT, LD_PRELOAD=str(shim))
+    r = subprocess.run([sys.executable, "-c", CHILD_NO_ROOM, str(shim)], cwd=ROOT, env=env, timeout=300,
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
