@@ -1239,7 +1239,7 @@ struct mdx_ensemble {
     // on-chip sweeps: per-member plans, {plan holds, gave up}, the last
     // sequence number (and a bound of it on the host), the inboxes of rgrid
     // blocks of rthreads threads
-    ens_plan* rplan = nullptr;
+    ens_plan* rplan = nullptr;       // (rseq is the last of the three)
     int* rstate = nullptr;
     unsigned* rseq = nullptr;
     void* rbox = nullptr;
@@ -1378,14 +1378,17 @@ ens_args make_args(mdx_ensemble_t* E, int s, int momentum) {
 size_t res_bytes(int grid, int stride) { return sizeof(word) * 2 * (size_t)grid * stride; }
 
 // Before launches (outside a capture) of `substages` substages of this shape:
-// the inboxes, and cleared ones before the sequence numbers run out.
+// the inboxes, and cleared ones before the sequence numbers run out.  Without
+// room for them the sweeps run from L2.
 int res_prepare(mdx_ensemble_t* E, int variant, int threads, int grid, int substages) {
     int smem = 0, stride = 0;
     if (!res_shape(E, variant, threads, &smem, &stride)) return MDX_OK;
-    if (!E->rplan) {
-        MDX_TRY(ealloc(E, &E->rplan, E->n));
-        MDX_TRY(ealloc(E, &E->rstate, 2));
-        MDX_TRY(ealloc(E, &E->rseq, 1));
+    if (!E->rseq) {
+        if ((!E->rplan && ealloc(E, &E->rplan, E->n) != MDX_OK) || (!E->rstate && ealloc(E, &E->rstate, 2) != MDX_OK) ||
+            ealloc(E, &E->rseq, 1) != MDX_OK) {
+            cudaGetLastError();
+            return MDX_OK;
+        }
         free_graph(E);
     }
     const size_t bytes = res_bytes(grid, stride);
@@ -1393,15 +1396,16 @@ int res_prepare(mdx_ensemble_t* E, int variant, int threads, int grid, int subst
     E->rseq_bound += 2.0 * rounds * substages;
     bool clear = E->rseq_bound > 4.0e9;
     if (E->rbytes < bytes) {
+        free_graph(E);   // its kernels hold the old ones
         cudaFree(E->rbox);
         E->rbox = nullptr;
         E->rbytes = 0;
-        if (cudaMalloc(&E->rbox, bytes) != cudaSuccess) {   // without them the sweeps run from L2
+        if (cudaMalloc(&E->rbox, bytes) != cudaSuccess) {
             cudaGetLastError();
+            E->rbox = nullptr;
             return MDX_OK;
         }
         E->rbytes = bytes;
-        free_graph(E);
         clear = true;
     }
     if (clear) {

@@ -97,13 +97,40 @@ with to_device(M, g, bc, f) as s:
 """
 
 
+CHILD_NO_ROOM_ENSEMBLE = """
+import ctypes as C
+import sys
+import numpy as np
+import mobydiff_b200 as M
+
+shim = C.CDLL(sys.argv[1])
+refuse, refused = C.c_int.in_dll(shim, "refuse"), C.c_int.in_dll(shim, "refused")
+opts = M.make_solver_opts(M.SOLVER_REDBLACK, sor=1.7, tol=1e-4, check_every=25, precision=M.PREC_MIXED)
+out = []
+for no_room in (0, 1):
+    with M.Ensemble([M.make_member(64, 32, 32, seed=5), M.make_member(32, 32, 48, seed=6)], opts) as E:
+        E.config(256, 1)
+        E.ic()
+        E.step(1)
+        E.config(512, 1)     # larger inboxes
+        refuse.value = no_room
+        E.step(1)
+        refuse.value = 0
+        E.step(1)            # and room again
+        out.append([E.get(k, n) for k in range(2) for n in ("un", "vn", "wn", "pn")])
+assert refused.value > 0
+assert all(np.array_equal(a, b) for a, b in zip(*out))
+"""
+
+
 @pytest.mark.gpu
 @pytest.mark.skipif(shutil.which("gcc") is None, reason="needs gcc")
-def test_no_room_for_the_inboxes_falls_back(tmp_path):
+@pytest.mark.parametrize("child", [CHILD_NO_ROOM, CHILD_NO_ROOM_ENSEMBLE], ids=["channel", "ensemble"])
+def test_no_room_for_the_inboxes_falls_back(tmp_path, child):
     src, shim = tmp_path / "full.c", tmp_path / "full.so"
     src.write_text(NO_ROOM)
     subprocess.check_call(["gcc", "-shared", "-fPIC", str(src), "-o", str(shim), "-ldl"])
     env = dict(os.environ, PYTHONPATH=ROOT, LD_PRELOAD=str(shim))
-    r = subprocess.run([sys.executable, "-c", CHILD_NO_ROOM, str(shim)], cwd=ROOT, env=env, timeout=300,
+    r = subprocess.run([sys.executable, "-c", child, str(shim)], cwd=ROOT, env=env, timeout=300,
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
