@@ -423,8 +423,9 @@ int mdx_ensemble_set(mdx_ensemble_t* ens, int member, int field, const double* h
  * 32, <= 512), blocks per SM (0: as many as fit) and the register variant
  * (low_regs != 0: 64 registers per thread, twice the resident warps). */
 int mdx_ensemble_config(mdx_ensemble_t* ens, int threads, int blocks_per_sm, int low_regs);
-/* mdx_set_wait_limit of the on-chip sweeps (mixed precision, face form). */
-int mdx_ensemble_set_wait_limit(mdx_ensemble_t* ens, int polls);
+/* on != 0: on-chip rounds (mixed precision, face form) end as if a block had
+ * given up a wait, for tests of what follows. */
+int mdx_ensemble_fail_waits(mdx_ensemble_t* ens, int on);
 /* Time one step of each candidate launch shape from the same saved state and
  * keep the fastest; the choice is cached in the JSON file cache_path (may be
  * NULL) under a key of the member sizes, the mode, the precision and form of
@@ -583,7 +584,7 @@ int mdx_divergence_norms(mdx_ctx_t* ctx, double* l2, double* linf);
 
 /* How often a block of an on-chip red-black run reads a neighbour's word that
  * has not come before the run gives up (< 0: the default, about a second;
- * 0: at the first miss).  The fields are half swept then: MDX_ERR_TIMEOUT,
+ * 0: at the first miss; up to 32, rounded down to a power of two).  The fields are half swept then: MDX_ERR_TIMEOUT,
  * from the tolerance solve itself or, for a fixed count of iterations, from
  * the next call that waits for the stream and returns fields or numbers made
  * of them, or starts another run. */

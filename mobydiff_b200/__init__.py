@@ -211,7 +211,7 @@ def lib():
         "mdx_ensemble_get": (i, [vp, i, i, vp]),
         "mdx_ensemble_set": (i, [vp, i, i, vp]),
         "mdx_ensemble_config": (i, [vp, i, i, i]),
-        "mdx_ensemble_set_wait_limit": (i, [vp, i]),
+        "mdx_ensemble_fail_waits": (i, [vp, i]),
         "mdx_ensemble_tune": (i, [vp, C.c_char_p, P(i), P(i), P(i), P(d)]),
         "mdx_ensemble_use_graph": (i, [vp, i]),
         "mdx_ensemble_info": (i, [vp, P(i), P(i), P(i), P(i), P(d), P(C.c_longlong)]),
@@ -765,9 +765,9 @@ class Ensemble:
     def config(self, threads: int, blocks_per_sm: int = 0, low_regs: bool = False) -> None:
         self._c(lib().mdx_ensemble_config(self.h, int(threads), int(blocks_per_sm), 1 if low_regs else 0))
 
-    def set_wait_limit(self, polls: int) -> None:
-        """Solver.set_wait_limit of the on-chip sweeps."""
-        self._c(lib().mdx_ensemble_set_wait_limit(self.h, int(polls)))
+    def fail_waits(self, on: bool) -> None:
+        """On-chip rounds end as if a block had given up a wait."""
+        self._c(lib().mdx_ensemble_fail_waits(self.h, 1 if on else 0))
 
     def tune(self, cache_path=None):
         """(threads, blocks per SM, low-register variant, ms of the chosen

@@ -143,11 +143,11 @@ struct ens_args {
     int split;
     // on-chip FP32 face sweeps (res_* below); rbox null: not used
     struct ens_plan* rplan;          // per member: its blocks and their boxes
-    int* rstate;                     // {this round's plan holds, a block gave up a wait since the host looked}
+    int* rstate;                     // {this round's plan holds, a block gave up a wait since the host
+                                     // looked, rounds are to end as if one had}
     unsigned* rseq;                  // last sequence number used
     word* rbox;                      // inboxes, rstride words each
     int rstride, rsmem;              // rsmem: shared memory of a block for its box
-    int rpolls;                      // res_geom::polls
     const int* learn_ok;             // per member: the network wrote a correction
     int gate_period;                 // > 0: apply it per substage only while it takes fewer iterations
 };
@@ -499,6 +499,7 @@ struct ens_plan { int first, nyb, nzb, by, bz; };
 struct ens_faces {                   // a member as face_run_box wants it
     typedef float T;
     static constexpr bool HAS_R = true;
+    static constexpr int WAIT = WAIT_POLLS;
     mdx_dims d;
     mixed_params P;
     float *u, *v, *w, *q;
@@ -578,10 +579,10 @@ __device__ void sweeps_resident(const ens_args& A, int iters) {
         const ens_member& M = A.mem[m];
         const float* p32 = A.st[m].p32;
         const ens_faces a{M.d, mixed_params{p32[0], p32[1], p32[2], p32[3]}, M.du, M.dv, M.dw, M.dp, M.r32, M.mu32, M.fac32};
-        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride, A.rpolls};
+        const res_geom R{p.nyb, p.by, p.bz, M.d.nx / 2, A.rstride};
         const res_box b = make_box<0>(M.d.ny, M.d.nz, p.nyb, p.nzb, R.tpr, p.first, at);
-        if (!face_run_box<ens_faces, 0, RES_KZ>(a, b, R, iters, A.rbox, *(volatile unsigned*)A.rseq, ens_sm) && threadIdx.x == 0)
-            A.rstate[1] = 1;
+        const bool came = face_run_box<ens_faces, 0, RES_KZ>(a, b, R, iters, A.rbox, *(volatile unsigned*)A.rseq, ens_sm);
+        if (threadIdx.x == 0 && (!came || A.rstate[2])) A.rstate[1] = 1;
         break;
     }
 }
@@ -1246,7 +1247,7 @@ struct mdx_ensemble {
     size_t rbytes = 0;
     int rstride = 0, rsmem = 0;
     double rseq_bound = 0.0;
-    int rpolls = -1;                 // mdx_ensemble_set_wait_limit
+    int rfail = 0;                   // mdx_ensemble_fail_waits
 };
 
 namespace {
@@ -1369,7 +1370,6 @@ ens_args make_args(mdx_ensemble_t* E, int s, int momentum) {
     A.rplan = E->rplan;
     A.rstate = E->rstate;
     A.rseq = E->rseq;
-    A.rpolls = E->rpolls < 0 ? POLLS : E->rpolls;
     A.learn_ok = E->learn_ok;
     A.gate_period = E->gate_period;
     return A;
@@ -1384,12 +1384,13 @@ int res_prepare(mdx_ensemble_t* E, int variant, int threads, int grid, int subst
     int smem = 0, stride = 0;
     if (!res_shape(E, variant, threads, &smem, &stride)) return MDX_OK;
     if (!E->rseq) {
-        if ((!E->rplan && ealloc(E, &E->rplan, E->n) != MDX_OK) || (!E->rstate && ealloc(E, &E->rstate, 2) != MDX_OK) ||
+        if ((!E->rplan && ealloc(E, &E->rplan, E->n) != MDX_OK) || (!E->rstate && ealloc(E, &E->rstate, 3) != MDX_OK) ||
             ealloc(E, &E->rseq, 1) != MDX_OK) {
             cudaGetLastError();
             return MDX_OK;
         }
         free_graph(E);
+        if (E->rfail) ENS_CUDA(E, cudaMemcpyAsync(E->rstate + 2, &E->rfail, sizeof(int), cudaMemcpyHostToDevice, E->stream));
     }
     const size_t bytes = res_bytes(grid, stride);
     const double rounds = (double)E->opts.max_iter + 64.0 * std::max(E->opts.check_every, 1);
@@ -1416,14 +1417,11 @@ int res_prepare(mdx_ensemble_t* E, int variant, int threads, int grid, int subst
     return MDX_OK;
 }
 
-// After a synchronisation: MDX_ERR_TIMEOUT when a block gave up a wait in any
-// launch since the last call, whatever later projections ended with.  The
-// flag stays up until then, so on-chip rounds behind it end at once.  The
-// half-swept corrections are cleared: the next projection starts from 0.
-int res_check(mdx_ensemble_t* E) {
-    if (!E->rstate) return MDX_OK;
-    int gave_up = 0;
-    ENS_CUDA(E, cudaMemcpy(&gave_up, E->rstate + 1, sizeof(int), cudaMemcpyDeviceToHost));
+// MDX_ERR_TIMEOUT when a block gave up a wait in any launch since the flag was
+// last read (gave_up), whatever later projections ended with.  The flag stays up
+// until then, so on-chip rounds behind it end at once.  The half-swept
+// corrections are cleared: the next projection starts from 0.
+int res_check(mdx_ensemble_t* E, int gave_up) {
     if (!gave_up) return MDX_OK;
     ENS_CUDA(E, cudaMemsetAsync(E->rstate, 0, 2 * sizeof(int), E->stream));
     for (const auto& M : E->hm)
@@ -1488,8 +1486,12 @@ int ensure_grid(mdx_ensemble_t* E) {
     return grid_for(E, E->variant, E->threads, E->blocks_per_sm, &E->grid);
 }
 
-int read_stats(mdx_ensemble_t* E, std::vector<ens_state>& h) {
+// gave_up: the flag of the on-chip sweeps (res_check).
+int read_stats(mdx_ensemble_t* E, std::vector<ens_state>& h, int* gave_up = nullptr) {
     h.resize(E->n);
+    if (gave_up) *gave_up = 0;
+    if (gave_up && E->rstate)
+        ENS_CUDA(E, cudaMemcpyAsync(gave_up, E->rstate + 1, sizeof(int), cudaMemcpyDeviceToHost, E->stream));
     ENS_CUDA(E, cudaMemcpyAsync(h.data(), E->dst, sizeof(ens_state) * E->n, cudaMemcpyDeviceToHost, E->stream));
     ENS_CUDA(E, cudaStreamSynchronize(E->stream));
     return MDX_OK;
@@ -1853,8 +1855,9 @@ int mdx_ensemble_ic(mdx_ensemble_t* E) {
     for (int m = 0; m < E->n; ++m)
         ENS_CUDA(E, cudaMemsetAsync(E->hm[m].pn, 0, sizeof(double) * E->hm[m].d.npad, E->stream));
     std::vector<ens_state> after;
-    MDX_TRY(read_stats(E, after));
-    MDX_TRY(res_check(E));
+    int gave_up = 0;
+    MDX_TRY(read_stats(E, after, &gave_up));
+    MDX_TRY(res_check(E, gave_up));
     for (int m = 0; m < E->n; ++m) {
         after[m].hist_valid = 0;
         after[m].flip = 0;
@@ -1961,10 +1964,10 @@ int mdx_ensemble_config(mdx_ensemble_t* E, int threads, int blocks_per_sm, int l
     return MDX_OK;
 }
 
-int mdx_ensemble_set_wait_limit(mdx_ensemble_t* E, int polls) {
+int mdx_ensemble_fail_waits(mdx_ensemble_t* E, int on) {
     if (!E) return MDX_ERR_ARG;
-    E->rpolls = polls;
-    free_graph(E);   // the limit is a kernel argument
+    E->rfail = on ? 1 : 0;
+    if (E->rstate) ENS_CUDA(E, cudaMemcpyAsync(E->rstate + 2, &E->rfail, sizeof(int), cudaMemcpyHostToDevice, E->stream));
     return MDX_OK;
 }
 
@@ -2009,7 +2012,8 @@ int mdx_ensemble_step(mdx_ensemble_t* E, int nsteps, long long* total_iters) {
     }
     ENS_CUDA(E, cudaEventRecord(E->ev[1], E->stream));
     std::vector<ens_state> after;
-    MDX_TRY(read_stats(E, after));
+    int gave_up = 0;
+    MDX_TRY(read_stats(E, after, &gave_up));
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, E->ev[0], E->ev[1]) == cudaSuccess) E->last_step_ms = nsteps ? ms / nsteps : 0.0;
     long long it = 0;
@@ -2019,7 +2023,7 @@ int mdx_ensemble_step(mdx_ensemble_t* E, int nsteps, long long* total_iters) {
         if (after[m].status != MDX_OK && bad < 0) bad = m;
     }
     if (total_iters) *total_iters = it;
-    MDX_TRY(res_check(E));
+    MDX_TRY(res_check(E, gave_up));
     if (bad >= 0)
         return efail(E, after[bad].status == MDX_ERR_NONFINITE ? MDX_ERR_NONFINITE : MDX_NOT_CONVERGED,
                      "member %d: last projection status %d", bad, after[bad].status);
@@ -2102,7 +2106,10 @@ int mdx_ensemble_tune(mdx_ensemble_t* E, const char* cache_path, int* threads_ou
                 MDX_TRY(step_eager(E, v, cand_t[ti], grid));
                 ENS_CUDA(E, cudaEventRecord(E->ev[1], E->stream));
                 ENS_CUDA(E, cudaEventSynchronize(E->ev[1]));
-                if (const int rc = res_check(E)) {   // a step cut short is no candidate's time
+                std::vector<ens_state> h;
+                int gave_up = 0;
+                MDX_TRY(read_stats(E, h, &gave_up));
+                if (const int rc = res_check(E, gave_up)) {   // a step cut short is no candidate's time
                     MDX_TRY(snapshot(E, true));
                     return rc;
                 }

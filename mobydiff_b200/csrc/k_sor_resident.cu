@@ -228,7 +228,7 @@ k_pot_resident(pot_geom L, res_geom R, int iters, float* __restrict__ phi, const
 #pragma unroll
             for (int u = 0; u < NB; ++u)
                 if (t + u * T < nw) {
-                    ok = wait_word(in + t + u * T, sq, v[u], R.polls) && ok;
+                    ok = wait_word<WAIT_LIMIT_BEHIND>(in + t + u * T, sq, v[u]) && ok;
                     st2s(W + DT[t + u * T], (f2)v[u].a | (f2)v[u].b << 32);
                 }
         }
@@ -267,6 +267,7 @@ template <int PY, int MU>
 struct faces64 {
     typedef double T;
     static constexpr bool HAS_R = false;
+    static constexpr int WAIT = WAIT_LIMIT_BEHIND;
     mdx_dims d;
     mdx_bc_dev bc;
     mdx_sor_params p;
@@ -306,6 +307,7 @@ template <int PY>
 struct faces32 {
     typedef float T;
     static constexpr bool HAS_R = true;
+    static constexpr int WAIT = WAIT_LIMIT_AHEAD;
     mdx_dims d;
     mixed_params P;
     float *u, *v, *w, *q;
@@ -376,7 +378,7 @@ bool make_plan(const mdx_ctx_t* ctx, int tpr, const res_shape* shapes, int nshap
             const double cost = (double)bz * std::max(issue * warps, 100) + (double)(by + bz) * tpr + 0.01 * s;
             if (out->shape >= 0 && cost >= best) continue;
             best = cost;
-            out->R = res_geom{nyb, by, bz, tpr, 2 * (by + bz) * tpr, ctx->rs_polls < 0 ? POLLS : ctx->rs_polls};
+            out->R = res_geom{nyb, by, bz, tpr, 2 * (by + bz) * tpr};
             out->blocks = nyb * nzb;
             out->threads = (by * tpr + 31) & ~31;
             out->shape = s;
@@ -415,11 +417,20 @@ int res_prepare(mdx_ctx_t* ctx, const res_plan& P, int iters) {
         ctx->rs_bytes = bytes;
         ctx->rs_seq = 0;
     }
-    if (ctx->rs_seq == 0 || ctx->rs_seq > 0xffffffffu - 2u * (unsigned)iters - 2u) {
+    const unsigned limit = res_limit(ctx->rs_polls);
+    if (ctx->rs_seq == 0 || ctx->rs_seq < limit || ctx->rs_seq - limit >= SEQ_END - 2u * (unsigned)iters - 2u) {
         MDX_CUDA(ctx, cudaMemsetAsync(ctx->rs_box, 0, ctx->rs_bytes, ctx->stream));
-        ctx->rs_seq = 2;
+        ctx->rs_seq = limit + 2;
     }
     return MDX_OK;
+}
+
+// A run of any length in launches whose numbers fit.
+template <class F>
+int res_pieces(int iters, F&& run) {
+    constexpr int MOST = 1 << 27;
+    for (; iters > MOST; iters -= MOST) MDX_TRY(run(MOST));
+    return run(iters);
 }
 
 template <class F, class... Args>
@@ -504,21 +515,23 @@ bool mdx_res_face64_ok(mdx_ctx_t* ctx) {
 }
 
 int mdx_res_pot_run(mdx_ctx_t* ctx, const pot_geom& L, int iters) {
-    return ctx->bc.is_periodic[1] ? pot_run<1>(ctx, L, iters) : pot_run<0>(ctx, L, iters);
+    return res_pieces(iters, [&](int n) { return ctx->bc.is_periodic[1] ? pot_run<1>(ctx, L, n) : pot_run<0>(ctx, L, n); });
 }
 int mdx_res_face32_run(mdx_ctx_t* ctx, const mixed_params& q, int iters) {
     res_plan P;
     if (!face_plan<float>(ctx, face32_shapes, 12, &P))
         return mdx_fail(ctx, MDX_ERR_ARG, "resident sweeps: the grid does not fit the SMs");
-    return ctx->bc.is_periodic[1] ? face32_run<1>(ctx, q, P, iters) : face32_run<0>(ctx, q, P, iters);
+    return res_pieces(iters, [&](int n) { return ctx->bc.is_periodic[1] ? face32_run<1>(ctx, q, P, n) : face32_run<0>(ctx, q, P, n); });
 }
 int mdx_res_face64_run(mdx_ctx_t* ctx, const mdx_sor_params& p, int iters) {
     res_plan P;
     if (!face_plan<double>(ctx, face64_shapes, 18, &P))
         return mdx_fail(ctx, MDX_ERR_ARG, "resident sweeps: the grid does not fit the SMs");
-    if (ctx->mu_mode == MU_ONE)
-        return ctx->bc.is_periodic[1] ? face64_run<1, MU_NONE>(ctx, p, P, iters) : face64_run<0, MU_NONE>(ctx, p, P, iters);
-    return ctx->bc.is_periodic[1] ? face64_run<1, MU_PLANES>(ctx, p, P, iters) : face64_run<0, MU_PLANES>(ctx, p, P, iters);
+    const bool py = ctx->bc.is_periodic[1] != 0;
+    return res_pieces(iters, [&](int n) {
+        if (ctx->mu_mode == MU_ONE) return py ? face64_run<1, MU_NONE>(ctx, p, P, n) : face64_run<0, MU_NONE>(ctx, p, P, n);
+        return py ? face64_run<1, MU_PLANES>(ctx, p, P, n) : face64_run<0, MU_PLANES>(ctx, p, P, n);
+    });
 }
 
 int mdx_res_check(mdx_ctx_t* ctx) {

@@ -68,12 +68,44 @@ __device__ __forceinline__ word ld_word(const word* p) {
                  : "memory");
     return w;
 }
-// False when the word did not come within `polls` more reads of it.
-constexpr int POLLS = 1 << 20;   // about a second, the default
-__device__ __forceinline__ bool wait_word(const word* p, unsigned seq, word& w, int polls) {
-    for (int n = 0; w.sa != seq || w.sb != seq; ++n) {
-        if (n >= polls) return false;
-        w = ld_word(p);
+// Sequence numbers are 29 bits; the three above say how often a word that has
+// not come is read before the block gives up (res_limit; 0: POLLS times, about a
+// second).  So the limit needs no register in the sweeps: as a kernel argument
+// it cost the FP64 runs 1 to 5 %.  WAIT_POLLS: always POLLS (the ensemble, whose
+// numbers are 32 bits).  Where the limit is looked up decides a few registers:
+// behind a first look at the word FP64 and potentials gain 1 to 3 % over POLLS
+// and FP32 faces lose 1.7, in the loop's head FP64 loses 2 and FP32 faces 0 to
+// 1.6.
+constexpr int POLLS = 1 << 20;
+constexpr unsigned SEQ_END = 1u << 29;
+enum { WAIT_POLLS, WAIT_LIMIT_BEHIND, WAIT_LIMIT_AHEAD };
+// Limits of 0, 1, 2, 4 .. 32 reads (polls < 0: the usual one).
+inline unsigned res_limit(int polls) {
+    unsigned c = 0;
+    if (polls >= 0)
+        for (c = 1; c < 7 && ((1 << c) >> 1) <= polls; ++c) {}
+    return c * SEQ_END;
+}
+__device__ __forceinline__ int first_poll(unsigned seq) {   // the loop below counts up to POLLS
+    const unsigned c = seq / SEQ_END;
+    return c ? POLLS - ((1 << c) >> 2) : 0;
+}
+// False when the word did not come.
+template <int MODE>
+__device__ __forceinline__ bool wait_word(const word* p, unsigned seq, word& w) {
+    if constexpr (MODE == WAIT_LIMIT_BEHIND) {
+        if (w.sa == seq && w.sb == seq) return true;
+        int n = first_poll(seq);
+        do {
+            if (n == POLLS) return false;
+            ++n;
+            w = ld_word(p);
+        } while (w.sa != seq || w.sb != seq);
+    } else {
+        for (int n = MODE == WAIT_POLLS ? 0 : first_poll(seq); w.sa != seq || w.sb != seq; ++n) {
+            if (n == POLLS) return false;
+            w = ld_word(p);
+        }
     }
     return true;
 }
@@ -86,7 +118,6 @@ struct res_geom {
     int nyb, by, bz;   // blocks along y; rows and planes of the largest box
     int tpr;           // words per row
     int stride;        // words of one inbox, at least 2 (by + bz) tpr
-    int polls;         // reads of a word that has not come before a block gives up
 };
 __device__ __forceinline__ word* inbox(word* box, const res_geom& R, int block, int parity) {
     return box + ((long long)block * 2 + parity) * R.stride;
@@ -241,15 +272,15 @@ __device__ __forceinline__ bool face_run_box(const A& a, const res_box& b, const
 #pragma unroll
             for (int e = 0; e < 2; ++e)
                 if (t + e * NTH < nw) {
-                    ok = wait_word(in + 2 * nzw + t + e * NTH, sq, w[e], R.polls) && ok;
+                    ok = wait_word<A::WAIT>(in + 2 * nzw + t + e * NTH, sq, w[e]) && ok;
                     const int dst = DT[t + e * NTH];
                     value(w[e], V[(dst >> 1) + ((dst ^ PAR) & 1 ? tpr : 0)]);
                 }
         }
         // the z faces: those of the columns this block did not sweep there
         if (act) {
-            ok = wait_word(in + at, sq, zl, R.polls) && ok;
-            ok = wait_word(in + nzw + at, sq, zh, R.polls) && ok;
+            ok = wait_word<A::WAIT>(in + at, sq, zl) && ok;
+            ok = wait_word<A::WAIT>(in + nzw + at, sq, zh) && ok;
             value(zl, wY[0]);
             T v;
             value(zh, v);

@@ -2,7 +2,7 @@
 64-register variant never goes on chip): the same bits and iterations, members
 converging at different rounds, rows and planes that do not divide evenly, and
 a batch that fits the blocks only once its smaller members are done.  Which
-batches go on chip is seen by a limit of no waits, which only they run into."""
+batches go on chip is seen by rounds made to fail, which only they have."""
 import numpy as np
 import pytest
 
@@ -54,7 +54,7 @@ def test_which_batches_go_on_chip(form, precision, low_regs, check_every, on_chi
     with M.Ensemble(_members("uneven"), _opts(form, check_every, precision)) as E:
         E.config(512, 0, low_regs=low_regs)
         E.ic()
-        E.set_wait_limit(0)
+        E.fail_waits(True)
         if on_chip:
             with pytest.raises(M.MdxError) as e:
                 E.step(1)

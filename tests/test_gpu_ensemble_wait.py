@@ -30,20 +30,20 @@ def test_step_reports_and_recovers(graph):
         with M.Ensemble(_members(amp=0.04), _opts(tol=1e-6)) as E:
             E.use_graph(graph)
             if give_up:
-                E.set_wait_limit(0)
+                E.fail_waits(True)
                 with pytest.raises(M.MdxError) as e:   # the t=0 projection
                     E.ic()
                 assert e.value.code == M.MDX_ERR_TIMEOUT
-                E.set_wait_limit(-1)
+                E.fail_waits(False)
                 E.ic()
-                E.set_wait_limit(0)
+                E.fail_waits(True)
                 with pytest.raises(M.MdxError) as e:
                     E.step(2)
                 assert e.value.code == M.MDX_ERR_TIMEOUT
                 with pytest.raises(M.MdxError) as e:
                     E.tune()
                 assert e.value.code == M.MDX_ERR_TIMEOUT
-                E.set_wait_limit(-1)
+                E.fail_waits(False)
             E.ic()
             its = E.step(2)
             out.append((its, _fields(E)))
@@ -68,7 +68,7 @@ def test_timeout_of_an_early_step_is_not_lost():
         for k, a in enumerate(noise):
             for n, x in zip(("un", "vn", "wn"), a):
                 E.set(k, n, x)
-        E.set_wait_limit(0)
+        E.fail_waits(True)
         return E
 
     last = []   # per member, ||div u*|| of each step's last projection
